@@ -148,7 +148,7 @@ static int bse_kernels(qk_ctx* ctx, int TDA_W, int TDA, double eta, double lam, 
   QK_TRY(qk_wst(ctx, W_SLAB, N2 * nS, &slab));
   QK_TRY(qk_wst(ctx, W_RHO, N2 * nS, &rho));
   QK_TRY(qk_launch_slab_gather(ctx, N, nC, nO, nR, ERI, slab));
-  QK_TRY(qk_dgemm(ctx, 'N', 'T', (int)N2, nS, nS, 1.0, slab, (long long)N2, 0, XpY, nS, 0, 0.0,
+  QK_TRY(qk_gemm_tc(ctx, 'N', 'T', (int)N2, nS, nS, 1.0, slab, (long long)N2, 0, XpY, nS, 0, 0.0,
                   rho, (long long)N2, 0, 1));
   // ---- static kernels (RGW_phBSE_static_kernel_A/B.f90:32-52) ----
   k_bse_weights<<<grid_1d(ctx, nS), 256, 0, ctx->stream>>>(nS, eta, lam * lam, OmRPA, f);
@@ -169,7 +169,7 @@ static int bse_kernels(qk_ctx* ctx, int TDA_W, int TDA, double eta, double lam, 
   k_rho_block<<<grid_1d(ctx, (long long)v2 * nS), 256, 0, ctx->stream>>>(N, nS, nO, nv, nO, nv,
                                                                           rho, nullptr, Rvv);
   QK_LAUNCHED();
-  QK_TRY(qk_dgemm(ctx, 'N', 'T', (int)o2, (int)v2, nS, 1.0, Roo, (long long)o2, 0, Rvv,
+  QK_TRY(qk_gemm_tc(ctx, 'N', 'T', (int)o2, (int)v2, nS, 1.0, Roo, (long long)o2, 0, Rvv,
                   (long long)v2, 0, 0.0, G1, (long long)o2, 0, 1));
   if (!TDA) {
     k_rho_block<<<grid_1d(ctx, (long long)S2), 256, 0, ctx->stream>>>(N, nS, nC, no, nO, nv, rho,
@@ -178,7 +178,7 @@ static int bse_kernels(qk_ctx* ctx, int TDA_W, int TDA, double eta, double lam, 
     k_rho_block<<<grid_1d(ctx, (long long)S2), 256, 0, ctx->stream>>>(N, nS, nO, nv, nC, no, rho,
                                                                        nullptr, Rvo);
     QK_LAUNCHED();
-    QK_TRY(qk_dgemm(ctx, 'N', 'T', nS, nS, nS, 1.0, Rov, nS, 0, Rvo, nS, 0, 0.0, G2, nS, 0, 1));
+    QK_TRY(qk_gemm_tc(ctx, 'N', 'T', nS, nS, nS, 1.0, Rov, nS, 0, Rvo, nS, 0, 0.0, G2, nS, 0, 1));
   }
   *G1_out = G1;
   *G2_out = G2;
@@ -289,9 +289,9 @@ int qk_bse_acfdt_dev(qk_ctx* ctx, int exchange_kernel, int doXBS, int TDA_W, int
       QK_TRY(phrlr_dev(ctx, TDA, nS, dA, dB, Om, &XpY, &XmY, sm + 8, 1));
       k_acfdt_xy<<<grid_1d(ctx, (long long)S2), 256, 0, ctx->stream>>>(nS, XpY, XmY, Z);
       QK_LAUNCHED();
-      QK_TRY(qk_dgemm(ctx, 'N', 'T', 2 * nS, nS, nS, 1.0, Z, 2 * nS, 0, Bp, nS, 0, 0.0, ZB,
+      QK_TRY(qk_gemm_tc(ctx, 'N', 'T', 2 * nS, nS, nS, 1.0, Z, 2 * nS, 0, Bp, nS, 0, 0.0, ZB,
                       2 * nS, 0, 1));
-      QK_TRY(qk_dgemm(ctx, 'N', 'T', 2 * nS, nS, nS, 1.0, Z, 2 * nS, 0, Ap, nS, 0, 0.0, ZA,
+      QK_TRY(qk_gemm_tc(ctx, 'N', 'T', 2 * nS, nS, nS, 1.0, Z, 2 * nS, 0, Ap, nS, 0, 0.0, ZA,
                       2 * nS, 0, 1));
       k_acfdt_dots<<<1, 1024, 0, ctx->stream>>>(nS, Z, ZB, ZA, sm + 1);
       QK_LAUNCHED();

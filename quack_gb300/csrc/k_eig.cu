@@ -1613,7 +1613,7 @@ int bt_big_gemm(qk_ctx* ctx, bool mixed, char ta, char tb, int m, int n, int k, 
                 double* C, long long ldc) {
   if (mixed)
     return qk_gemm_f32p(ctx, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1);
-  return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1);
+  return qk_gemm_tc(ctx, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1);
 }
 
 // T factors of all reflector blocks of the last tridiagonalisation on this context:
@@ -1630,15 +1630,19 @@ int eig_tfactors(qk_ctx* ctx, int n, const double* V, const double* tau, const d
   double* T = buf + B2 * nblk;
   const int full = nref / BT_NB;
   const long long bstride = (long long)n * BT_NB;
-  auto gemm = fp32 ? qk_gemm_f32p : qk_dgemm;
+  auto gemm = [&](char ta, char tb, int m, int nn, int k, double alpha, const double* A, long long lda,
+                  long long sA, const double* B, long long ldb, long long sB, double beta, double* C,
+                  long long ldc, long long sC, int batch) {
+    return fp32 ? qk_gemm_f32p(ctx, ta, tb, m, nn, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch)
+                : qk_gemm_tc(ctx, ta, tb, m, nn, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+  };
   if (full > 0)
-    QK_TRY(gemm(ctx, 'T', 'N', BT_NB, BT_NB, n, 1.0, V, n, bstride, V, n, bstride, 0.0, G, BT_NB,
+    QK_TRY(gemm('T', 'N', BT_NB, BT_NB, n, 1.0, V, n, bstride, V, n, bstride, 0.0, G, BT_NB,
                 (long long)B2, full));
   if (full < nblk) {
     const int kb = full * BT_NB, nb = nref - kb;
     const double* Vb = V + (size_t)n * kb;
-    QK_TRY(gemm(ctx, 'T', 'N', nb, nb, n, 1.0, Vb, n, 0, Vb, n, 0, 0.0, G + B2 * full, BT_NB, 0,
-                1));
+    QK_TRY(gemm('T', 'N', nb, nb, n, 1.0, Vb, n, 0, Vb, n, 0, 0.0, G + B2 * full, BT_NB, 0, 1));
   }
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
@@ -1989,7 +1993,6 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
   // ---- 4. back-transformation Zt <- Zt * Q^T, blocks from last to first ----
   // (backtransform == 2, the mixed tier: the block products and the T factors with compensated
   // FP32 products; Zt stays FP64)
-  auto gemm = backtransform == 2 ? qk_gemm_f32p : qk_dgemm;
   if (tm) qk_tic(ctx, T_BACKTRANS);
   const int nref = n - 2;  // reflectors 0..n-3 can be non-trivial
   if (nref > 0) {
@@ -2009,7 +2012,8 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
       double* Es = Zt + N * (kb + 1);
       QK_TRY(bt_big_gemm(ctx, backtransform == 2, 'N', 'N', n, nb, m, 1.0, Es, n, Vb, n, 0.0, W1,
                          n));
-      QK_TRY(gemm(ctx, 'N', 'T', n, nb, nb, 1.0, W1, n, 0, Tb, BT_NB, 0, 0.0, W2, n, 0, 1));
+      QK_TRY(bt_big_gemm(ctx, backtransform == 2, 'N', 'T', n, nb, nb, 1.0, W1, n, Tb, BT_NB, 0.0, W2,
+                         n));
       QK_TRY(bt_big_gemm(ctx, backtransform == 2, 'N', 'T', n, m, nb, -1.0, W2, n, Vb, n, 1.0, Es,
                          n));
     }
@@ -2035,7 +2039,6 @@ int qk_eig_apply_qt(qk_ctx* ctx, int n, double* X, long long ldx, int ncols, int
   double* W1 = bt;
   double* W2 = bt + (size_t)ncols * BT_NB;
   const int nblk = (nref + BT_NB - 1) / BT_NB;
-  auto gemm = fp32 ? qk_gemm_f32p : qk_dgemm;
   for (int b = 0; b < nblk; ++b) {
     const int kb = b * BT_NB;
     const int nb = (nref - kb) < BT_NB ? (nref - kb) : BT_NB;
@@ -2045,7 +2048,7 @@ int qk_eig_apply_qt(qk_ctx* ctx, int n, double* X, long long ldx, int ncols, int
     double* Xs = X + (kb + 1);
     // W1 = V^T X (nb x ncols), W2 = T^T W1, X -= V W2
     QK_TRY(bt_big_gemm(ctx, fp32 != 0, 'T', 'N', nb, ncols, m, 1.0, Vb, n, Xs, ldx, 0.0, W1, nb));
-    QK_TRY(gemm(ctx, 'T', 'N', nb, ncols, nb, 1.0, Tb, BT_NB, 0, W1, nb, 0, 0.0, W2, nb, 0, 1));
+    QK_TRY(bt_big_gemm(ctx, fp32 != 0, 'T', 'N', nb, ncols, nb, 1.0, Tb, BT_NB, W1, nb, 0.0, W2, nb));
     QK_TRY(bt_big_gemm(ctx, fp32 != 0, 'N', 'N', m, ncols, nb, -1.0, Vb, n, W2, nb, 1.0, Xs, ldx));
   }
   return QK_OK;

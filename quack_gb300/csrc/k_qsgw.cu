@@ -286,15 +286,20 @@ int qk_qs_mo_slab(qk_ctx* ctx, int nBas, int N, int nC, int nO, int nR, const do
   const long long N1 = N, B = nBas;
   const double* cocc = c + B * nC;
   const double* cvir = c + B * nO;
-  auto gemm = df ? qk_gemm_df : qk_dgemm;
+  auto gemm = [&](char ta, char tb, int m, int n, int k, double alpha, const double* A, long long lda,
+                  long long sA, const double* Bm, long long ldb, long long sB, double beta, double* C,
+                  long long ldc, long long sC, int batch) {
+    return df ? qk_gemm_df(ctx, ta, tb, m, n, k, alpha, A, lda, sA, Bm, ldb, sB, beta, C, ldc, sC, batch)
+              : qk_gemm_tc(ctx, ta, tb, m, n, k, alpha, A, lda, sA, Bm, ldb, sB, beta, C, ldc, sC, batch);
+  };
   // <mu la|nu si> -> (la,nu,si,j) -> (nu,si,j,p) -> (si,j,p,b) -> (j,p,b,q); c is nBas x nOrb
-  QK_TRY(gemm(ctx, 'T', 'N', (int)(B * B * B), no, nBas, 1.0, ERI, B, 0, cocc, B, 0, 0.0, W1,
+  QK_TRY(gemm('T', 'N', (int)(B * B * B), no, nBas, 1.0, ERI, B, 0, cocc, B, 0, 0.0, W1,
               B * B * B, 0, 1));
-  QK_TRY(gemm(ctx, 'T', 'N', (int)(B * B * no), N, nBas, 1.0, W1, B, 0, c, B, 0, 0.0, W2,
+  QK_TRY(gemm('T', 'N', (int)(B * B * no), N, nBas, 1.0, W1, B, 0, c, B, 0, 0.0, W2,
               B * B * no, 0, 1));
-  QK_TRY(gemm(ctx, 'T', 'N', (int)(B * no * N1), nv, nBas, 1.0, W2, B, 0, cvir, B, 0, 0.0, W1,
+  QK_TRY(gemm('T', 'N', (int)(B * no * N1), nv, nBas, 1.0, W2, B, 0, cvir, B, 0, 0.0, W1,
               B * no * N1, 0, 1));
-  QK_TRY(gemm(ctx, 'T', 'N', (int)((long long)no * N1 * nv), N, nBas, 1.0, W1, B, 0, c, B, 0, 0.0,
+  QK_TRY(gemm('T', 'N', (int)((long long)no * N1 * nv), N, nBas, 1.0, W1, B, 0, c, B, 0, 0.0,
               W2, (long long)no * N1 * nv, 0, 1));
   const long long nS = (long long)no * nv;
   k_qs_slab<<<grid_1d(ctx, N1 * N1 * nS), 256, 0, ctx->stream>>>(N, no, nv, W2, slab);
@@ -312,9 +317,11 @@ int qk_qs_sigma(qk_ctx* ctx, int doSRG, double eta, double flow, int N, int nC, 
     k_qs_weight<<<grid_1d(ctx, N2 * nS), 256, 0, ctx->stream>>>(N, nC, nO, nR, nS, eta, e, Om,
                                                                   rho, W);
     QK_LAUNCHED();
-    auto gemm = df ? qk_gemm_df : qk_dgemm;
-    return gemm(ctx, 'N', 'T', N, N, (int)(N1 * nS), 1.0, W, N1, 0, rho, N1, 0, 0.0, Sig, N1, 0,
-                1);
+    if (df)
+      return qk_gemm_df(ctx, 'N', 'T', N, N, (int)(N1 * nS), 1.0, W, N1, 0, rho, N1, 0, 0.0, Sig, N1,
+                        0, 1);
+    return qk_gemm_tc(ctx, 'N', 'T', N, N, (int)(N1 * nS), 1.0, W, N1, 0, rho, N1, 0, 0.0, Sig, N1, 0,
+                      1);
   }
   const int tiles = (N + SRG_T - 1) / SRG_T;
   const long long K = (long long)(N - nC - nR) * nS;

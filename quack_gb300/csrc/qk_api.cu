@@ -194,7 +194,7 @@ int rho_gemm(qk_ctx* ctx, int prec, int N, int nS, const double* S, const double
   const long long N2 = (long long)N * N;
   if (prec == QK_PREC_BF16X3)
     return qk_gemm_bf16x3_nt(ctx, (int)N2, nS, nS, S, N2, XpY, nS, rho, N2);
-  return qk_dgemm(ctx, 'N', 'T', (int)N2, nS, nS, 1.0, S, N2, 0, XpY, nS, 0, 0.0, rho, N2, 0, 1);
+  return qk_gemm_tc(ctx, 'N', 'T', (int)N2, nS, nS, 1.0, S, N2, 0, XpY, nS, 0, 0.0, rho, N2, 0, 1);
 }
 
 // contractions of the factorised integrals:
@@ -207,7 +207,7 @@ int factor_prep(qk_ctx* ctx, const Dims& d, int naux, const double* L, double** 
   QK_TRY(qk_wst(ctx, W_KMAT, (size_t)nS * nS, &K));
   qk_tic(ctx, T_SLAB);
   QK_TRY(qk_launch_gather_ov(ctx, N, d.nC, d.nO, d.nR, naux, L, Lov));
-  QK_TRY(qk_dgemm(ctx, 'N', 'T', nS, nS, naux, 1.0, Lov, nS, 0, Lov, nS, 0, 0.0, K, nS, 0, 1));
+  QK_TRY(qk_gemm_tc(ctx, 'N', 'T', nS, nS, naux, 1.0, Lov, nS, 0, Lov, nS, 0, 0.0, K, nS, 0, 1));
   qk_toc(ctx, T_SLAB);
   *K_out = K;
   *Lov_out = Lov;
@@ -247,8 +247,8 @@ int casida_factored(qk_ctx* ctx, int prec, const Dims& d, const double* e, const
     QK_CK(cudaMemcpyAsync(X, Lov, (size_t)nS * naux * sizeof(double), cudaMemcpyDeviceToDevice,
                           ctx->stream));
     QK_TRY(qk_eig_apply_qt(ctx, nS, X, nS, naux, f32));
-    QK_TRY((f32 ? qk_gemm_f32p : qk_dgemm)(ctx, 'N', 'N', nS, naux, nS, 1.0, Zt, nS, 0, X, nS, 0,
-                                           0.0, T, nS, 0, 1));
+    QK_TRY(f32 ? qk_gemm_f32p(ctx, 'N', 'N', nS, naux, nS, 1.0, Zt, nS, 0, X, nS, 0, 0.0, T, nS, 0, 1)
+               : qk_gemm_tc(ctx, 'N', 'N', nS, naux, nS, 1.0, Zt, nS, 0, X, nS, 0, 0.0, T, nS, 0, 1));
     qk_toc(ctx, T_BACKTRANS);
     k_vsum_om<<<1, 1024, 0, ctx->stream>>>(nS, w, Om, scal + 1);
     QK_LAUNCHED();
@@ -264,8 +264,8 @@ int casida_factored(qk_ctx* ctx, int prec, const Dims& d, const double* e, const
   qk_tic(ctx, T_BACKTRANS);
   QK_TRY(qk_launch_rowscale(ctx, nS, naux, sq, 0, Lov, nS, X, nS));           // D_s Lov
   QK_TRY(qk_eig_apply_qt(ctx, nS, X, nS, naux, f32));                        // Q^T (.)
-  QK_TRY((f32 ? qk_gemm_f32p : qk_dgemm)(ctx, 'N', 'N', nS, naux, nS, 1.0, Zt, nS, 0, X, nS, 0,
-                                         0.0, T, nS, 0, 1));
+  QK_TRY(f32 ? qk_gemm_f32p(ctx, 'N', 'N', nS, naux, nS, 1.0, Zt, nS, 0, X, nS, 0, 0.0, T, nS, 0, 1)
+             : qk_gemm_tc(ctx, 'N', 'N', nS, naux, nS, 1.0, Zt, nS, 0, X, nS, 0, 0.0, T, nS, 0, 1));
   QK_TRY(qk_launch_rowscale(ctx, nS, naux, w, 1, T, nS, T, nS));             // D_Om^-1/2
   qk_toc(ctx, T_BACKTRANS);
   QK_TRY(qk_launch_sum_sqrt(ctx, nS, w, scal + 1));
@@ -281,7 +281,7 @@ int rho_from_T(qk_ctx* ctx, int prec, const Dims& d, int naux, const double* L, 
   const long long N2 = (long long)N * N;
   if (prec == QK_PREC_BF16X3)
     return qk_gemm_bf16x3_nt(ctx, (int)N2, nS, naux, L, N2, T, nS, rho, N2);
-  return qk_dgemm(ctx, 'N', 'T', (int)N2, nS, naux, 1.0, L, N2, 0, T, nS, 0, 0.0, rho, N2, 0, 1);
+  return qk_gemm_tc(ctx, 'N', 'T', (int)N2, nS, naux, 1.0, L, N2, 0, T, nS, 0, 0.0, rho, N2, 0, 1);
 }
 
 // Casida with eigenvectors for the dRPA singlet screening at energies e.
@@ -846,21 +846,21 @@ int phrlr_dev(qk_ctx* ctx, int TDA, int nS, double* dA, double* dB, double* dOm,
     // AmBSq = U diag(sqrt l) U^T = Ut^T (D Ut)
     k_rowscale<<<grid_for(ctx, (long long)S2), 256, 0, ctx->stream>>>(nS, lam, 0, ut, tmp);
     QK_LAUNCHED();
-    QK_TRY(qk_dgemm(ctx, 'T', 'N', nS, nS, nS, 1.0, ut, nS, 0, tmp, nS, 0, 0.0, sqm, nS, 0, 1));
+    QK_TRY(qk_gemm_tc(ctx, 'T', 'N', nS, nS, nS, 1.0, ut, nS, 0, tmp, nS, 0, 0.0, sqm, nS, 0, 1));
     if (want_vectors) {
       k_rowscale<<<grid_for(ctx, (long long)S2), 256, 0, ctx->stream>>>(nS, lam, 1, ut, tmp);
       QK_LAUNCHED();
-      QK_TRY(qk_dgemm(ctx, 'T', 'N', nS, nS, nS, 1.0, ut, nS, 0, tmp, nS, 0, 0.0, ivm, nS, 0, 1));
+      QK_TRY(qk_gemm_tc(ctx, 'T', 'N', nS, nS, nS, 1.0, ut, nS, 0, tmp, nS, 0, 0.0, ivm, nS, 0, 1));
     }
     // ApB into amb, tmp = ApB.AmBSq, M = AmBSq.tmp
     k_axpby<<<grid_for(ctx, (long long)S2), 256, 0, ctx->stream>>>((long long)S2, 1.0, dA, 1.0, dB, amb);
     QK_LAUNCHED();
-    QK_TRY(qk_dgemm(ctx, 'N', 'N', nS, nS, nS, 1.0, amb, nS, 0, sqm, nS, 0, 0.0, tmp, nS, 0, 1));
-    QK_TRY(qk_dgemm(ctx, 'N', 'N', nS, nS, nS, 1.0, sqm, nS, 0, tmp, nS, 0, 0.0, dM, nS, 0, 1));
+    QK_TRY(qk_gemm_tc(ctx, 'N', 'N', nS, nS, nS, 1.0, amb, nS, 0, sqm, nS, 0, 0.0, tmp, nS, 0, 1));
+    QK_TRY(qk_gemm_tc(ctx, 'N', 'N', nS, nS, nS, 1.0, sqm, nS, 0, tmp, nS, 0, 0.0, dM, nS, 0, 1));
     QK_TRY(qk_eig_sym(ctx, nS, dM, nS, w, dZt, want_vectors));  // dZt = Z^T
     if (want_vectors) {
-      QK_TRY(qk_dgemm(ctx, 'N', 'N', nS, nS, nS, 1.0, dZt, nS, 0, sqm, nS, 0, 0.0, dX, nS, 0, 1));
-      QK_TRY(qk_dgemm(ctx, 'N', 'N', nS, nS, nS, 1.0, dZt, nS, 0, ivm, nS, 0, 0.0, dY, nS, 0, 1));
+      QK_TRY(qk_gemm_tc(ctx, 'N', 'N', nS, nS, nS, 1.0, dZt, nS, 0, sqm, nS, 0, 0.0, dX, nS, 0, 1));
+      QK_TRY(qk_gemm_tc(ctx, 'N', 'N', nS, nS, nS, 1.0, dZt, nS, 0, ivm, nS, 0, 0.0, dY, nS, 0, 1));
       k_xpy_general<<<grid_for(ctx, (long long)S2), 256, 0, ctx->stream>>>(nS, w, dOm, dX, dY, ctx->d_status);
       QK_LAUNCHED();
     } else {
@@ -1167,7 +1167,7 @@ int aotomo_dev(qk_ctx* ctx, int nBas, int nOrb, const double* dc, double* X, dou
       QK_TRY(qk_gemm_df(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, 0, dc, nBas, 0, 0.0,
                         dst, R[s], 0, 1));
     else
-      QK_TRY(qk_dgemm(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, 0, dc, nBas, 0, 0.0,
+      QK_TRY(qk_gemm_tc(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, 0, dc, nBas, 0, 0.0,
                       dst, R[s], 0, 1));
     double* t = src;
     src = dst;
@@ -1249,7 +1249,7 @@ int qsgw_dev(qk_ctx* ctx, const qk_gw_params* prm, int nBas, const Dims& d, cons
     QK_CK(cudaMemcpyAsync(out.P, in.PHF, B2 * 8, cudaMemcpyDeviceToDevice, ctx->stream));
   auto gemm = [&](char ta, char tb, int m, int n, int k, double alpha, const double* A, int lda,
                   const double* Bm, int ldb, double beta, double* C, int ldc) {
-    return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, 0, Bm, ldb, 0, beta, C, ldc, 0, 1);
+    return qk_gemm_tc(ctx, ta, tb, m, n, k, alpha, A, lda, 0, Bm, ldb, 0, beta, C, ldc, 0, 1);
   };
   int nSCF = -1, n_diis = 0;
   double Conv = 1.0, hs[32] = {0.0};
@@ -1456,8 +1456,11 @@ int qk_dgemm_dev(qk_ctx* ctx, char transa, char transb, int m, int n, int k, dou
                  const double* d_A, int lda, const double* d_B, int ldb, double beta, double* d_C,
                  int ldc) {
   QK_TRY(begin(ctx));
-  const int st = qk_dgemm(ctx, transa, transb, m, n, k, alpha, d_A, lda, 0, d_B, ldb, 0, beta, d_C,
-                          ldc, 0, 1);
+  const int st = qk_tune_get(ctx, TUNE_DGEMM_PATH, (long long)m * n, 1) == 3
+                     ? qk_gemm_tc(ctx, transa, transb, m, n, k, alpha, d_A, lda, 0, d_B, ldb, 0,
+                                  beta, d_C, ldc, 0, 1, true)
+                     : qk_dgemm(ctx, transa, transb, m, n, k, alpha, d_A, lda, 0, d_B, ldb, 0,
+                                beta, d_C, ldc, 0, 1);
   return end(ctx, st);
 }
 
