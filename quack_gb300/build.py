@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libqkgw.so")
 
-SOURCES = ["qk_ctx.cu", "k_gemm64.cu", "k_gemm_tc.cu", "k_eig.cu", "k_casida.cu", "k_sigma.cu", "k_bf16x3.cu",
+SOURCES = ["qk_ctx.cu", "k_gemm64.cu", "k_gemm_tc.cu", "k_tri_fx.cu", "k_eig.cu", "k_casida.cu", "k_sigma.cu", "k_bf16x3.cu",
            "k_mlp.cu", "k_probe.cu", "k_noalloc.cu", "k_tune.cu", "k_rpa_quad.cu", "k_bse.cu",
            "k_eri_io.cu", "k_qsgw.cu", "qk_api.cu", "qk_batch.cu"]
 

@@ -101,7 +101,7 @@ struct TriArgs {
   double* tau;
   double* V;
   long long ldv;
-  int df;        // 1: double-float arithmetic on the FP32 pipe (sytrd_df_body)
+  int df;        // arithmetic: TRI_FP64, TRI_DF (sytrd_df_body) or TRI_FX (qk_tri_fx)
   double* vscal;   // df: n slots for the reflectors' scale factors (consumed by k_tri_df_finish)
   double* dfscale; // df: one slot, the power of two that undoes the matrix scaling
   double* pbuf;  // 6*n: three rotating p vectors, each as two exact accumulators (n + n)
@@ -1665,6 +1665,7 @@ int eig_tfactors(qk_ctx* ctx, int n, const double* V, const double* tau, const d
 struct qk_tri_service {
   struct Req {
     TriArgs ta;
+    qk_tri_fx_args fx;   // (ta.df == TRI_FX)
     cudaStream_t stream;
     cudaEvent_t ready;
   };
@@ -1727,10 +1728,19 @@ void tri_split(const std::vector<qk_tri_service::Req>& rq, int sms, int* cta0) {
   for (int r = 0; r < R; ++r) cta0[r + 1] = cta0[r] + g[r];
 }
 
-// one cooperative launch for the pending requests of one arithmetic (FP64 or double-float)
-int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& rq, bool df) {
+// one launch for the pending requests of one arithmetic (FP64 and double-float cooperative)
+int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& rq, int mode) {
   const int R = (int)rq.size();
   if (R == 0) return QK_OK;
+  if (mode == TRI_FX) {
+    qk_tri_fx_args fx[TRI_GROUP_MAX];
+    for (int r = 0; r < R; ++r) fx[r] = rq[r].fx;
+    QK_TRY(qk_tri_fx(sv->parent, sv->stream, R, fx));
+    sv->launches++;
+    sv->matrices += R;
+    return QK_OK;
+  }
+  const bool df = mode == TRI_DF;
   TriGroup g;
   g.nreq = R;
   size_t smem = 0;
@@ -1758,17 +1768,17 @@ int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& 
   return QK_OK;
 }
 
-// cooperative launches for all pending requests (called with the lock held): one per arithmetic
-// present, one after the other on the service stream, each over all SMs
+// launches for all pending requests (called with the lock held): one per arithmetic present, one
+// after the other on the service stream, each over all SMs
 void tri_launch_locked(qk_tri_service* sv) {
   int st = QK_OK;
   const int R = (int)sv->pending.size();
-  std::vector<qk_tri_service::Req> part[2];
+  std::vector<qk_tri_service::Req> part[3];
   for (int r = 0; r < R; ++r) {
-    part[sv->pending[r].ta.df ? 1 : 0].push_back(sv->pending[r]);
+    part[sv->pending[r].ta.df].push_back(sv->pending[r]);
     if (cudaStreamWaitEvent(sv->stream, sv->pending[r].ready, 0) != cudaSuccess) st = QK_ERR_CUDA;
   }
-  for (int k = 0; k < 2 && st == QK_OK; ++k) st = tri_launch_part(sv, part[k], k == 1);
+  for (int k = 0; k < 3 && st == QK_OK; ++k) st = tri_launch_part(sv, part[k], k);
   if (cudaEventRecord(sv->done, sv->stream) != cudaSuccess) st = QK_ERR_CUDA;
   // every requester's stream continues after the group (enqueued before they wake up)
   for (int r = 0; r < R; ++r)
@@ -1779,11 +1789,11 @@ void tri_launch_locked(qk_tri_service* sv) {
   sv->cv.notify_all();
 }
 
-int tri_submit(qk_tri_service* sv, qk_ctx* ctx, const TriArgs& ta) {
+int tri_submit(qk_tri_service* sv, qk_ctx* ctx, const TriArgs& ta, const qk_tri_fx_args& fx = {}) {
   if (!ctx->ev_tri) QK_CK(cudaEventCreateWithFlags(&ctx->ev_tri, cudaEventDisableTiming));
   QK_CK(cudaEventRecord(ctx->ev_tri, ctx->stream));
   std::unique_lock<std::mutex> lk(sv->mu);
-  sv->pending.push_back({ta, ctx->stream, ctx->ev_tri});
+  sv->pending.push_back({ta, fx, ctx->stream, ctx->ev_tri});
   const unsigned long long my = sv->gen;
   if ((int)sv->pending.size() >= sv->n_active || (int)sv->pending.size() >= TRI_GROUP_MAX)
     tri_launch_locked(sv);
@@ -1838,8 +1848,9 @@ void qk_tri_service_free(qk_tri_service* sv) {
 
 // ------------------------------------------------------------------------------------------
 int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, int want_vectors,
-               int backtransform, int tri_df) {
+               int backtransform, int mode) {
   if (n <= 0) return QK_OK;
+  const bool tri_df = mode == TRI_DF;
   const size_t N = (size_t)n;
   // workspace: V (n*n), small vectors (d, e, tau, e2, pbuf(6n), prep(64), per-CTA slots)
   double *V = nullptr, *tri = nullptr;
@@ -1860,7 +1871,17 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
   // ---- 1. tridiagonalisation ----
   const bool tm = ctx->time_eig;
   if (tm) qk_tic(ctx, T_TRIDIAG);
-  {
+  if (mode == TRI_FX && qk_tri_fx_cluster(n)) {
+    const qk_tri_fx_args fa{A, lda, n, d, e, tau, V, n};
+    if (ctx->tri_service && !ctx->capturing) {
+      TriArgs ta = {};
+      ta.df = TRI_FX;
+      ta.n = n;
+      QK_TRY(tri_submit(ctx->tri_service, ctx, ta, fa));
+    } else {
+      QK_TRY(qk_tri_fx(ctx, ctx->stream, 1, &fa));
+    }
+  } else {
     // threads per CTA: the FP64 kernel 1024, the double-float kernel 512 (its registers)
     const int nt = tri_df ? DF_THREADS : TRI_THREADS;
     const size_t tile_bytes = (size_t)(nt / 32) * TRI_TC * TRI_TLD * 8;
@@ -1907,7 +1928,7 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
     ta.tau = tau;
     ta.V = V;
     ta.ldv = n;
-    ta.df = tri_df != 0;
+    ta.df = tri_df ? TRI_DF : TRI_FP64;
     ta.vscal = e2;           // free until k_tri_prep fills e^2
     ta.dfscale = prep + 8;   // k_tri_prep writes prep[0..4]
     ta.pbuf = pbuf;
@@ -2060,6 +2081,7 @@ extern "C" int qk_dsyev_dev(qk_ctx* ctx, int n, double* d_A, int lda, double* d_
   cudaSetDevice(ctx->device);
   QK_TRY(qk_order_after_default(ctx));
   QK_TRY(qk_status_reset(ctx));
-  QK_TRY(qk_eig_sym(ctx, n, d_A, lda, d_w, d_Zt, want_vectors, 1, ctx->dsyev_df));
+  QK_TRY(qk_eig_sym(ctx, n, d_A, lda, d_w, d_Zt, want_vectors, 1,
+                    ctx->dsyev_df == 0 ? TRI_FP64 : ctx->dsyev_df == 1 ? TRI_DF : TRI_FX));
   return qk_status_check(ctx, QKD_BARRIER_TIMEOUT | QKD_BAD_INDEX);
 }

@@ -1,0 +1,521 @@
+// k_tri_fx.cu -- Householder tridiagonalisation in 64-bit fixed point on the integer pipe, the whole
+// matrix resident in the shared memory of one thread-block cluster.
+//
+// The FP64 tier's reduction of a Casida matrix (dsyev's dsytrd step) for the sizes that fit.  The
+// grid-wide FP64 kernel (k_sytrd) pays ~10 us per column whatever the size -- a grid barrier, L2 round
+// trips and FP64 block sums at 64 cycles per warp instruction.  Here
+//   - A is full (not only its lower triangle) and row-cyclic over the cluster's CTAs, so row r's
+//     part of p = A v is one warp's dot product and nothing is summed across CTAs;
+//   - p_r and the next column's element A_(r,j+1) go to every CTA by one distributed-shared-memory
+//     store instruction per row, and one cluster barrier (~0.25 us) ends the column;
+//   - the arithmetic is fixed point: orthogonal similarity keeps |A_ij| <= ||A||_2, so with the matrix
+//     scaled by the power of two S that makes min(||A||_inf, ||A||_F) / S < 1/2 an element is an int64 multiple of
+//     2^-62, and a product of two such numbers is three 32 x 32 -> 64 multiply-adds (2 cycles per
+//     warp each, against 64 for an FP64 FMA).  An element costs ~45 issue slots per column.
+// Accuracy: every update rounds to 2^-62 S without bias; FP64 rounds to
+// 2^-53 of the element.  The reflectors are normalised to unit length to ~2^-60, so the transformation
+// is orthogonal to working precision, and the factorisation is backward stable with a smaller
+// constant than in FP64 (the test measures both).  Elements below 2^-62 S are lost, which is why
+// qk_dsyev_dev, which takes any matrix, stays with the FP64 kernel.  Integer sums make the result
+// independent of the number of CTAs and of the order of summation.
+//
+// Column j (u = the previous reflector, |u| = 1, H = I - 2 u u^T):
+//   K = u^T p;  w = p - K u;  x = column j of A - 2 (u w^T + w u^T);  d_j = x_j;
+//   u' = unit vector of x_(j+1..) + sign(alpha) |x| e_1, e_j = -sign(alpha) |x|   (dlarfg's choice)
+//   rows r > j: A_r -= 2 (u_r w + w_r u), p'_r = A_r u', broadcast p'_r and A_(r,j+1).
+// Measured (one GB300), eigenvalues alone (this kernel plus the bisection), before -> now: n = 48
+// 0.77 -> 0.42 ms, 128 1.84 -> 0.87, 256 3.55 -> 1.60, 400 5.55 -> 2.61, 600 8.43 -> 4.63.  A column
+// takes ~7.6k cycles at n = 400: the vector work ~3.1k (block sums, the reflector's scalars), the
+// rows ~2.9k, the cluster barrier with its wait ~1.7k.
+#include <cooperative_groups.h>
+#include <mutex>
+#include "qk_internal.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int WORKERS = 512;             // worker threads; one more warp writes d, e, tau and V
+constexpr int VT = 256, VW = VT / 32;    // of them the O(n) vector work of a column
+constexpr int THREADS = WORKERS + 32;
+constexpr int NWARPS = WORKERS / 32;
+constexpr int MAX_CL = 16;
+constexpr int SMEM_MAX = 226 * 1024;
+
+struct FxGroup {
+  qk_tri_fx_args req[QK_TRI_FX_GROUP];
+};
+
+// x = h 2^32 + l' with l' signed; l = l' >> 3 (29 bits): in Q62, x = h 2^-30 + l 2^-59
+struct Fx {
+  int h, l;
+};
+__device__ __forceinline__ Fx fx_split(long long x) {
+  const int lo = (int)(unsigned)x;
+  return Fx{(int)(x >> 32) + (int)((unsigned)lo >> 31), lo >> 3};
+}
+__device__ __forceinline__ long long wide(int a, int b) { return (long long)a * b; }
+constexpr long long CR_HALF = 1ll << 26;
+// round(x y 2^62): the l l term (zero mean, below 2^-62) is dropped
+__device__ __forceinline__ long long fx_mul(Fx x, Fx y) {
+  const long long hh = wide(x.h, y.h);
+  const long long cr = CR_HALF + wide(x.h, y.l) + wide(x.l, y.h);
+  return (hh << 2) + (cr >> 27);
+}
+// 2 (a b + c d)
+__device__ __forceinline__ long long fx_mul2(Fx a, Fx b, Fx c, Fx d) {
+  const long long hh = wide(a.h, b.h) + wide(c.h, d.h);
+  const long long cr =
+      (CR_HALF >> 1) + wide(a.h, b.l) + wide(a.l, b.h) + wide(c.h, d.l) + wide(c.l, d.h);
+  return (hh << 3) + (cr >> 26);
+}
+constexpr long long FX_ONE = 1ll << 62;
+
+// 1 / sqrt(4 m4) for m4 in [1/4, 1]: the hardware's FP32 value r0 (an integer of Q30, relative error
+// below 2^-21) and one third-order step r = r0 (1 + h + 3 h^2 / 2), h = (1 - 4 m4 r0^2) / 2
+__device__ __forceinline__ long long fx_rsqrt4(long long m4) {
+  const float m = (float)(int)(m4 >> 32) * 0x1p-28f;     // 4 m4 in [1, 4]
+  const int r0 = (int)fminf(rsqrtf(m) * 0x1p30f, 0x1p30f);
+  const long long u = fx_mul(fx_split(m4), fx_split(wide(r0, r0) << 2));  // m4 r0^2, near 1/4
+  const long long h = ((FX_ONE >> 2) - u) << 1;                             // |h| < 2^42 (Q62)
+  const int hq = (int)(h >> 20);                                           // Q42
+  const long long c = h + ((3 * wide(hq, hq)) >> 23);                      // h + 3 h^2 / 2
+  // r0 c: c in two parts of 25 + 18 bits
+  const int ch = (int)(c >> 18), clow = (int)(c & 0x3FFFF);
+  return ((long long)r0 << 32) + ((wide(r0, ch) + (wide(r0, clow) >> 18)) >> 12);
+}
+
+// double -> Q62 of the scaled matrix (x 2^(62 - E - 1)), 2^E above the norm bound
+__device__ __forceinline__ long long fx_from_double(double x, int E) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)((b >> 52) & 0x7FF);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (ex ? 1ull << 52 : 0ull);
+  const int sh = max(ex, 1) - 1075 + 61 - E;
+  long long q;
+  if (sh >= 0) q = (long long)(m << min(sh, 63));
+  else if (sh > -63) q = (long long)((m + (1ull << (-sh - 1))) >> -sh);
+  else q = 0;
+  return (long long)b < 0 ? -q : q;
+}
+__device__ __forceinline__ double pow2(int k) {  // |k| <= 1022
+  return __longlong_as_double((long long)(k + 1023) << 52);
+}
+// x 2^k rounded to a double, on the integer pipe where the result is a normal number
+__device__ __forceinline__ double fx_to_double(long long x, int k) {
+  if (x == 0) return 0.0;
+  unsigned long long m = (unsigned long long)(x < 0 ? -x : x);
+  const int z = __clzll((long long)m);
+  m <<= z;                                            // leading bit at 63
+  const unsigned rem = (unsigned)m & 0x7FFu;
+  m >>= 11;
+  m += rem + (unsigned)(m & 1ull) > 0x400u ? 1ull : 0ull;
+  const int ex = 63 - z + k + 1023;
+  const unsigned long long sign = x < 0 ? 1ull << 63 : 0ull;
+  if (ex > 0 && ex < 2046)
+    return __longlong_as_double((long long)((((unsigned long long)(ex - 1) << 52) + m) | sign));
+  const int q = max(-2200, min(2200, ex - 1023)), q1 = q / 3;
+  return __longlong_as_double((long long)(((1022ull << 52) + m) | sign)) * pow2(q1) * pow2(q1) *
+         pow2(q - 2 * q1);
+}
+
+// sum of one int64 per lane over the warp, in every lane (REDUX is 32 bits wide and issues slowly:
+// three of them took 330 cycles with all warps at it, this butterfly ~150)
+__device__ __forceinline__ long long warp_sum64(long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ void vec_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ long long sum_parts(const long long* p) {
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < VW; ++w) t += p[w];
+  return t;
+}
+
+struct Scal {             // one column's scalars, written by one thread
+  long long f;            // u'_i = (x_i << sh) f
+  long long u1;           // u'_(j+1), signed
+  long long nx;           // |x| 2^(sh - xs)
+  int sh;
+  long long g;            // 1 / (2 |u1|)
+  int neg, zero;          // alpha < 0; no reflector (x = 0, or the last column)
+  long long dj, alpha;
+};
+
+__device__ __forceinline__ void reflector(long long s0, long long s1, int xs, bool last, long long xj,
+                                          long long alpha, int lane, Scal& out) {
+  Scal t;
+  t.dj = xj;
+  t.alpha = alpha;
+  t.neg = alpha < 0;
+  t.zero = xs < 0 || last;
+  t.sh = 0;
+  t.f = t.u1 = t.nx = t.g = 0;
+  if (!t.zero) {
+    // |x|^2 = T 2^-89: m4 = T 2^-89 4^(sh - xs) in [1/4, 1)
+    unsigned long long hi = (unsigned long long)(s0 >> 35), lo = (unsigned long long)s0 << 29;
+    const unsigned long long lo2 = lo + (unsigned long long)s1;
+    hi += (unsigned long long)(s1 >> 63) + (lo2 < lo ? 1ull : 0ull);
+    lo = lo2;
+    const int lead = 128 - __clzll((long long)hi);        // bits of T (hi > 0)
+    const int q = (89 - lead) >> 1;                       // T 4^q has 88 or 89 bits
+    const int down = 89 - 62 - 2 * q;                     // m4 (Q62) = T >> down, 0 < down < 64
+    const long long m4 = (long long)((hi << (64 - down)) | (lo >> down));
+    const long long r = fx_rsqrt4(m4);                    // 1 / (2 |x'|), |x'| = |x| 2^(q + xs)
+    const Fx rs = fx_split(r);
+    t.nx = fx_mul(fx_split(m4), rs) << 1;                 // |x'| in [1/2, 1)
+    t.sh = q + xs;
+    const long long ax = (alpha < 0 ? -alpha : alpha) << t.sh;
+    // a = |alpha| / |x| in [0, 1]; b = (1 + a) / 2; u1 = sqrt(b); u_i = x_i / (2 |x| u1)
+    long long b = (FX_ONE >> 1) + fx_mul(fx_split(ax), rs);
+    b = b > FX_ONE ? FX_ONE : b;
+    t.g = fx_rsqrt4(b);                                   // 1 / (2 sqrt(b))
+    const Fx gs = fx_split(t.g);
+    const long long u1 = fx_mul(fx_split(b), gs) << 1;
+    t.u1 = alpha < 0 ? -u1 : u1;
+    t.f = fx_mul(rs, gs) << 1;                            // 1 / (2 |x'| u1)
+  }
+  if (lane == 0) out = t;
+}
+
+// R own rows (lr, lr + NWARPS): the rank-2 update, the dot product with u' and the broadcast of p'
+// and of the next column's element.  The loads of two column groups are issued together.
+template <int R>
+__device__ __forceinline__ void row_pass(long long* As, int lr, int n, int j, int CL, int rank, int par,
+                                         int lane, const Fx* U, const Fx* Wb, const Fx* Un,
+                                         long long* Pb, long long* Xb, cg::cluster_group& cl) {
+  long long* Ar[R];
+  Fx ur[R], wr[R];
+  long long hh[R], cr[R], xn[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int r = (lr + q * NWARPS) * CL + rank;
+    Ar[q] = As + (size_t)(lr + q * NWARPS) * n;
+    ur[q] = U[r];
+    wr[q] = Wb[r];
+    hh[q] = cr[q] = xn[q] = 0;
+  }
+  constexpr int B = 2;                     // column groups in flight
+  for (int c0 = j + 1; c0 < n; c0 += 32 * B) {
+    Fx u[B], w[B], v[B];
+    long long y[R][B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const int c = c0 + 32 * b + lane, cc = c < n ? c : n - 1;
+      u[b] = U[cc];
+      w[b] = Wb[cc];
+      v[b] = Un[cc];
+      if (c >= n) v[b] = Fx{0, 0};
+#pragma unroll
+      for (int q = 0; q < R; ++q) y[q][b] = Ar[q][cc];
+    }
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const int c = c0 + 32 * b + lane;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        y[q][b] -= fx_mul2(ur[q], w[b], wr[q], u[b]);
+        if (c < n) Ar[q][c] = y[q][b];
+        const Fx ys = fx_split(y[q][b]);
+        hh[q] += wide(ys.h, v[b].h);
+        cr[q] += wide(ys.h, v[b].l) + wide(ys.l, v[b].h);
+      }
+    }
+    if (c0 == j + 1) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) xn[q] = y[q][0];
+    }
+  }
+  long long p[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) p[q] = (hh[q] << 2) + ((cr[q] + CR_HALF) >> 27);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < R; ++q) p[q] += __shfl_xor_sync(0xffffffffu, p[q], o);
+  // lanes 0..15: p' to CTA lane, lanes 16..31: the next column's element to CTA lane - 16
+  const int dst = lane & 15;
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const long long x = __shfl_sync(0xffffffffu, xn[q], 0);
+    if (dst < CL) {
+      long long* base = (lane < 16 ? Pb : Xb) + (par ^ 1) * n + (lr + q * NWARPS) * CL + rank;
+      *cl.map_shared_rank(base, dst) = lane < 16 ? p[q] : x;
+    }
+  }
+}
+
+// cluster b of the grid reduces matrix b
+__global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ FxGroup grp) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const qk_tri_fx_args& a = grp.req[blockIdx.x / CL];
+  const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rows = (n - rank + CL - 1) / CL;      // rows rank, rank + CL, ..
+  const int max_rows = (n + CL - 1) / CL;
+  extern __shared__ long long sm[];
+  long long* As = sm;                                // rows x n
+  long long* Pb = As + (size_t)max_rows * n;         // [2][n] p of the next column, by all CTAs
+  long long* Xb = Pb + 2 * n;                        // [2][n] the next column
+  long long* Xc = Xb + 2 * n;                        // [n] the updated column
+  Fx* Ub = (Fx*)(Xc + n);                            // [2][n] reflectors u, u'
+  Fx* Wb = Ub + 2 * n;                               // [n]
+  __shared__ long long redk[VW], red[2][NWARPS];
+  __shared__ int s_small;
+  __shared__ unsigned redm[VW];
+  __shared__ double cmax[MAX_CL], cfro[MAX_CL];
+  __shared__ Scal sc;
+
+  // ---- ||A||_inf and ||A||_F^2: a warp per own row, lanes along the row (the lower triangle is
+  // referenced) ----
+  if (warp < NWARPS) {
+    double m = 0.0, f = 0.0;
+    for (int lr = warp; lr < rows; lr += NWARPS) {
+      const int r = lr * CL + rank;
+      double s = 0.0;
+#pragma unroll 4
+      for (int c = lane; c < n; c += 32) {
+        const double x = c <= r ? a.A[r + a.lda * c] : a.A[c + a.lda * r];
+        s += fabs(x);
+        f = fma(x, x, f);
+      }
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      m = s > m || s != s ? s : m;                   // (a NaN stays: comparisons with it fail)
+    }
+    for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+    if (lane == 0) {
+      ((double*)red[0])[warp] = m;
+      ((double*)red[1])[warp] = f;
+    }
+  }
+  __syncthreads();
+  if (tid < CL) {
+    double m = 0.0, f = 0.0;
+    for (int w = 0; w < NWARPS; ++w) {
+      const double s = ((double*)red[0])[w];
+      m = s > m || s != s ? s : m;
+      f += ((double*)red[1])[w];
+    }
+    *cl.map_shared_rank(&cmax[rank], tid) = m;
+    *cl.map_shared_rank(&cfro[rank], tid) = f;
+  }
+  cl.sync();
+  double nrm = 0.0, fro = 0.0;
+  for (int b = 0; b < CL; ++b) {
+    nrm = cmax[b] > nrm || cmax[b] != cmax[b] ? cmax[b] : nrm;
+    fro += cfro[b];
+  }
+  if (!(nrm <= 1.7976931348623157e308)) {            // NaN or infinity: everything NaN
+    const double qnan = __longlong_as_double(0x7FF8000000000000ll);
+    for (int i = tid; i < n; i += THREADS) {
+      if (rank == 0) {
+        a.d[i] = qnan;
+        a.e[i] = qnan;
+        a.tau[i] = qnan;
+      }
+    }
+    for (int j = rank; j < n - 1; j += CL)
+      for (int i = j + 1 + tid; i < n; i += THREADS) a.V[i + a.ldv * j] = qnan;
+    return;
+  }
+  // the sum of squares may over- or underflow: it counts only where it is a comfortable number
+  if (fro > 1e-200 && fro < 1e300) nrm = fmin(nrm, 1.000001 * sqrt(fro));
+  const int E = nrm > 0.0 ? ilogb(nrm) + 1 : 0;      // nrm < 2^E
+  // ---- own rows and the first column into fixed point ----
+  for (int lr = 0; lr < rows; ++lr) {
+    const int r = lr * CL + rank;
+    for (int c = tid; c < n; c += THREADS)
+      As[(size_t)lr * n + c] = fx_from_double(c <= r ? a.A[r + a.lda * c] : a.A[c + a.lda * r], E);
+  }
+  for (int i = tid; i < n; i += THREADS) {
+    Xb[i] = fx_from_double(a.A[i], E);
+    Pb[i] = 0;
+    Ub[i] = Fx{0, 0};
+    Wb[i] = Fx{0, 0};
+  }
+  cl.sync();
+
+  int lr0 = rank == 0 ? 1 : 0;                       // own rows beyond column j start here
+  for (int j = 0; j < n; ++j) {
+    const int par = j & 1;
+    const long long* P = Pb + par * n;
+    const long long* X = Xb + par * n;
+    const Fx* U = Ub + par * n;
+    Fx* Un = Ub + (par ^ 1) * n;
+    if (tid < VT) {
+      // ---- K = u^T p ----
+      long long Ksum = 0;
+      if (j > 0) {
+        for (int i = j + tid; i < n; i += VT) Ksum += fx_mul(fx_split(P[i]), U[i]);
+        Ksum = warp_sum64(Ksum);
+        if (lane == 0) redk[warp] = Ksum;
+        vec_bar();
+        Ksum = sum_parts(redk);
+      }
+      const Fx K = fx_split(Ksum);
+      // ---- w and the updated column x; sums of h^2 and of h l' / 4 + l'^2 / 2^35 ----
+      const Fx uj = U[j];
+      const Fx wj = fx_split(P[j] - fx_mul(K, uj) + 4);
+      long long s0 = 0, s1 = 0;
+      for (int i = j + tid; i < n; i += VT) {
+        const Fx u = U[i];
+        const Fx w = fx_split(P[i] - fx_mul(K, u) + 4);
+        const long long x = X[i] - fx_mul2(u, wj, w, uj);
+        Wb[i] = w;
+        Xc[i] = x;
+        if (i > j) {
+          const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
+          s0 += wide(h, h);
+          s1 += wide(h, lo >> 2) + (wide(lo, lo) >> 35);
+        }
+      }
+      s0 = warp_sum64(s0);
+      s1 = warp_sum64(s1);
+      if (lane == 0) {
+        red[0][warp] = s0;
+        red[1][warp] = s1;
+      }
+      vec_bar();
+      int xs = 0;
+      for (;;) {
+        if (warp == 0) {
+          // ---- the reflector's scalars (one warp; all lanes the same values) ----
+          s0 = sum_parts(red[0]);
+          s1 = sum_parts(red[1]);
+          // |x|^2 = s0 2^-60 + s1 2^-89; below 2^-25 the sums have too few bits: x << xs instead
+          const bool small = xs == 0 && s0 + (s1 >> 29) < (1ll << 35);
+          if (!small) reflector(s0, s1, xs, j >= n - 2, Xc[j], j + 1 < n ? Xc[j + 1] : 0, lane, sc);
+          if (lane == 0) s_small = small;
+        }
+        vec_bar();
+        if (!s_small) break;
+        unsigned long long mx = 0;            // leading bits of max |x|
+        for (int i = j + 1 + tid; i < n; i += VT) {
+          const long long x = Xc[i];
+          const unsigned long long ax = (unsigned long long)(x < 0 ? -x : x);
+          mx = mx > ax ? mx : ax;
+        }
+        unsigned m = mx ? 64u - (unsigned)__clzll((long long)mx) : 0u;
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) redm[warp] = m;
+        vec_bar();
+        m = __reduce_max_sync(0xffffffffu, lane < VW ? redm[lane] : 0u);
+        xs = m ? 55 - (int)m : -1;            // max |x| << xs in [2^54, 2^55); -1: x = 0
+        s0 = s1 = 0;
+        if (xs > 0)
+          for (int i = j + 1 + tid; i < n; i += VT) {
+            const long long x = Xc[i] << xs;
+            const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
+            s0 += wide(h, h);
+            s1 += wide(h, lo >> 2) + (wide(lo, lo) >> 35);
+          }
+        s0 = warp_sum64(s0);
+        s1 = warp_sum64(s1);
+        if (lane == 0) {
+          red[0][warp] = s0;
+          red[1][warp] = s1;
+        }
+        vec_bar();
+      }
+      // ---- u' ----
+      {
+        const Fx f = fx_split(sc.f);
+        const int sh = sc.sh;
+        const bool zero = sc.zero != 0;
+        for (int i = j + 1 + tid; i < n; i += VT) {
+          long long u = 0;
+          if (!zero) u = i == j + 1 ? sc.u1 : fx_mul(fx_split(Xc[i] << sh), f);
+          Un[i] = fx_split(u + 4);                  // (the split keeps 59 bits: to nearest)
+        }
+      }
+    }
+    __syncthreads();
+    if (warp < NWARPS) {
+      // ---- big pass over the own rows r > j, two rows of a warp at a time ----
+      int lr = warp + lr0;
+      for (; lr + NWARPS < rows; lr += 2 * NWARPS)
+        row_pass<2>(As, lr, n, j, CL, rank, par, lane, U, Wb, Un, Pb, Xb, cl);
+      if (lr < rows) row_pass<1>(As, lr, n, j, CL, rank, par, lane, U, Wb, Un, Pb, Xb, cl);
+      // (the first own row beyond column j + 1)
+      if (lr0 * CL + rank <= j + 1) ++lr0;
+    } else {
+      // ---- output warp ----
+      const Scal t = sc;
+      if (rank == 0 && lane == 0) {
+        a.d[j] = fx_to_double(t.dj, E + 1 - 62);
+        if (j < n - 1) {
+          a.e[j] = t.zero ? fx_to_double(t.alpha, E + 1 - 62)
+                          : fx_to_double(t.neg ? t.nx : -t.nx, E + 1 - 62 - t.sh);
+          const Fx u1 = fx_split(t.u1);
+          a.tau[j] = fx_to_double(fx_mul(u1, u1), 1 - 62);
+        }
+      }
+      if (j < n - 1) {
+        // v = u / u1 (unit first entry): u 2 g, with the sign of u1
+        const Fx g = fx_split(t.u1 < 0 ? -t.g : t.g);
+        for (int i = j + 1 + 32 * rank + lane; i < n; i += 32 * CL)
+          a.V[i + a.ldv * j] = i == j + 1 ? 1.0 : fx_to_double(fx_mul(Un[i], g), 1 - 62);
+      }
+    }
+    cl.sync();
+  }
+}
+
+size_t fx_smem(int n, int cl) {
+  const size_t rows = (n + cl - 1) / cl;
+  return rows * n * 8 + (size_t)n * 8 * (2 + 2 + 1 + 2 + 1);
+}
+
+}  // namespace
+
+// CTAs of the cluster for a matrix of order n (0: does not fit; 615 is the largest that does).  More
+// CTAs shorten the row pass and lengthen the broadcast; a single CTA needs no remote stores.
+int qk_tri_fx_cluster(int n) {
+  if (n < 2) return 0;
+  int cl = n <= 64 ? 1 : n <= 128 ? 4 : n <= 256 ? 8 : 16;
+  while (cl < MAX_CL && fx_smem(n, cl) > (size_t)SMEM_MAX) cl *= 2;
+  return fx_smem(n, cl) <= (size_t)SMEM_MAX ? cl : 0;
+}
+
+// One launch over R matrices, a cluster each (all of the size the largest needs; the result does not
+// depend on it).
+int qk_tri_fx(qk_ctx* ctx, cudaStream_t stream, int R, const qk_tri_fx_args* req) {
+  if (R < 1 || R > QK_TRI_FX_GROUP) return qk_fail(ctx, QK_ERR_ARG, "qk_tri_fx: %d matrices", R);
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(k_tri_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(k_tri_fx, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  QK_CK(attr_err);
+  FxGroup g;
+  int cl = 1;
+  for (int r = 0; r < R; ++r) {
+    const int c = qk_tri_fx_cluster(req[r].n);
+    if (!c) return qk_fail(ctx, QK_ERR_ARG, "qk_tri_fx: n=%d does not fit", req[r].n);
+    cl = c > cl ? c : cl;
+    g.req[r] = req[r];
+  }
+  size_t smem = 0;
+  for (int r = 0; r < R; ++r) {
+    const size_t s = fx_smem(req[r].n, cl);
+    smem = s > smem ? s : smem;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cl * R);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cl;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  QK_CK(cudaLaunchKernelEx(&cfg, k_tri_fx, g));
+  ctx->launches++;
+  return QK_OK;
+}

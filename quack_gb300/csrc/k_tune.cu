@@ -103,7 +103,7 @@ int qk_tune_set(qk_ctx* ctx, const char* name, long long size, int value) {
     return QK_OK;
   }
   if (!strcmp(name, "dsyev_df")) {
-    if (value < 0 || value > 1) return QK_ERR_ARG;
+    if (value < 0 || value > 2) return QK_ERR_ARG;
     ctx->dsyev_df = value;
     return QK_OK;
   }

@@ -55,7 +55,7 @@ struct qk_ctx {
   int newton_maxit = 64;   // Newton steps of the graphical QP solve (RGW_QP_graph.f90:38)
   int guess_gate = 0;      // learned-guess start rule (k_guess: 0 Halley agreement, 1, 2)
   int fail_alloc_in = 0;   // > 0: the n-th next growing workspace allocation fails (test hook)
-  int dsyev_df = 0;        // qk_dsyev_dev tridiagonalises in double-float (the mixed tier's way)
+  int dsyev_df = 0;        // qk_dsyev_dev: 0 FP64 kernel, 1 double-float, 2 as the FP64-tier drivers
   qk_tri_service* tri_service = nullptr;  // batch worker: tridiagonalise through the group launch
   cudaEvent_t ev_tri = nullptr;           // end of this context's work before a group launch
   long long tri_groups = 0;               // grouped tridiagonalisation launches of the last batch
@@ -230,8 +230,21 @@ int qk_bse_dev(qk_ctx* ctx, int TDA_W, int TDA, int singlet, int triplet, int ex
 qk_tri_service* qk_tri_service_new(qk_ctx* parent, int n_workers);
 void qk_tri_service_worker_done(qk_tri_service* svc);
 void qk_tri_service_free(qk_tri_service* svc);
+// tri: TRI_FX (the drivers' FP64 tier) takes the fixed-point cluster kernel (k_tri_fx.cu) where
+// the matrix fits it and else the FP64 kernel; TRI_FP64 always the FP64 kernel; TRI_DF double-float.
+enum { TRI_FX = 0, TRI_DF = 1, TRI_FP64 = 2 };
 int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, int want_vectors,
-               int backtransform = 1, int tri_df = 0);
+               int backtransform = 1, int tri = TRI_FX);
+int qk_tri_fx_cluster(int n);
+struct qk_tri_fx_args {
+  const double* A;
+  long long lda;
+  int n;
+  double *d, *e, *tau, *V;
+  long long ldv;
+};
+constexpr int QK_TRI_FX_GROUP = 32;
+int qk_tri_fx(qk_ctx* ctx, cudaStream_t stream, int R, const qk_tri_fx_args* req);
 int qk_eig_apply_qt(qk_ctx* ctx, int n, double* X, long long ldx, int ncols, int fp32 = 0);
 
 // Casida pieces (k_casida.cu)
