@@ -9,6 +9,8 @@
 //      recomputes the O(n) vector work redundantly (bitwise identical in all CTAs), leaving
 //      one bounded grid barrier per column.  The mat-vec's partial sums from different CTAs
 //      meet in exact (order-independent) accumulators, so the result is the same in every run.
+//      The FP64 tier's drivers take the fixed-point kernels of k_tri_fx.cu instead wherever the
+//      matrix fits them; k_sytrd serves qk_dsyev_dev and matrices above order ~8000.
 //   2. k_stebz: Sturm-count k-section (K lanes per eigenvalue), full FP64 precision.
 //   3. k_stein: inverse iteration on T - lambda I (tridiagonal GEPP), one thread per cluster of
 //      close eigenvalues, modified Gram-Schmidt inside clusters; eigenvectors written as rows.
@@ -1665,7 +1667,8 @@ int eig_tfactors(qk_ctx* ctx, int n, const double* V, const double* tau, const d
 struct qk_tri_service {
   struct Req {
     TriArgs ta;
-    qk_tri_fx_args fx;   // (ta.df == TRI_FX)
+    qk_tri_fx_args fx;        // (ta.df == TRI_FX)
+    qk_tri_fx_grid_args fxg;  // (ta.df == TRI_FX_GRID)
     cudaStream_t stream;
     cudaEvent_t ready;
   };
@@ -1740,6 +1743,16 @@ int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& 
     sv->matrices += R;
     return QK_OK;
   }
+  if (mode == TRI_FX_GRID) {
+    qk_tri_fx_grid_group g;
+    g.nreq = R;
+    for (int r = 0; r < R; ++r) g.req[r] = rq[r].fxg;
+    tri_split(rq, sv->parent->num_sms, g.cta0);
+    QK_TRY(qk_tri_fx_grid_launch_group(sv->parent, sv->stream, g));
+    sv->launches++;
+    sv->matrices += R;
+    return QK_OK;
+  }
   const bool df = mode == TRI_DF;
   TriGroup g;
   g.nreq = R;
@@ -1773,12 +1786,12 @@ int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& 
 void tri_launch_locked(qk_tri_service* sv) {
   int st = QK_OK;
   const int R = (int)sv->pending.size();
-  std::vector<qk_tri_service::Req> part[3];
+  std::vector<qk_tri_service::Req> part[4];
   for (int r = 0; r < R; ++r) {
     part[sv->pending[r].ta.df].push_back(sv->pending[r]);
     if (cudaStreamWaitEvent(sv->stream, sv->pending[r].ready, 0) != cudaSuccess) st = QK_ERR_CUDA;
   }
-  for (int k = 0; k < 3 && st == QK_OK; ++k) st = tri_launch_part(sv, part[k], k);
+  for (int k = 0; k < 4 && st == QK_OK; ++k) st = tri_launch_part(sv, part[k], k);
   if (cudaEventRecord(sv->done, sv->stream) != cudaSuccess) st = QK_ERR_CUDA;
   // every requester's stream continues after the group (enqueued before they wake up)
   for (int r = 0; r < R; ++r)
@@ -1789,11 +1802,12 @@ void tri_launch_locked(qk_tri_service* sv) {
   sv->cv.notify_all();
 }
 
-int tri_submit(qk_tri_service* sv, qk_ctx* ctx, const TriArgs& ta, const qk_tri_fx_args& fx = {}) {
+int tri_submit(qk_tri_service* sv, qk_ctx* ctx, const TriArgs& ta, const qk_tri_fx_args& fx = {},
+               const qk_tri_fx_grid_args& fxg = {}) {
   if (!ctx->ev_tri) QK_CK(cudaEventCreateWithFlags(&ctx->ev_tri, cudaEventDisableTiming));
   QK_CK(cudaEventRecord(ctx->ev_tri, ctx->stream));
   std::unique_lock<std::mutex> lk(sv->mu);
-  sv->pending.push_back({ta, fx, ctx->stream, ctx->ev_tri});
+  sv->pending.push_back({ta, fx, fxg, ctx->stream, ctx->ev_tri});
   const unsigned long long my = sv->gen;
   if ((int)sv->pending.size() >= sv->n_active || (int)sv->pending.size() >= TRI_GROUP_MAX)
     tri_launch_locked(sv);
@@ -1880,6 +1894,31 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
       QK_TRY(tri_submit(ctx->tri_service, ctx, ta, fa));
     } else {
       QK_TRY(qk_tri_fx(ctx, ctx->stream, 1, &fa));
+    }
+  } else if (mode == TRI_FX && qk_tri_fx_grid_fits(n)) {
+    qk_tri_fx_grid_args ga = {};
+    ga.A = A;
+    ga.lda = lda;
+    ga.n = n;
+    ga.d = d;
+    ga.e = e;
+    ga.tau = tau;
+    ga.V = V;
+    ga.ldv = n;
+    ga.work = pbuf;
+    ga.bar = ctx->d_bar;
+    ga.status = ctx->d_status;
+    if (ctx->tri_service && !ctx->capturing) {
+      TriArgs ta = {};
+      ta.df = TRI_FX_GRID;
+      ta.n = n;
+      QK_TRY(tri_submit(ctx->tri_service, ctx, ta, {}, ga));
+    } else {
+      int grid = ctx->num_sms * qk_tune_get(ctx, TUNE_SYTRD_GRID, n, 4) / 4;
+      const int want = (int)((N * N) / (32 * 128)) + 1;
+      if (grid > want) grid = want;
+      if (ctx->sytrd_max_ctas > 0 && grid > ctx->sytrd_max_ctas) grid = ctx->sytrd_max_ctas;
+      QK_TRY(qk_tri_fx_grid(ctx, grid < 1 ? 1 : grid, ga));
     }
   } else {
     // threads per CTA: the FP64 kernel 1024, the double-float kernel 512 (its registers)

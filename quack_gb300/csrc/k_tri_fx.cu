@@ -1,5 +1,6 @@
-// k_tri_fx.cu -- Householder tridiagonalisation in 64-bit fixed point on the integer pipe, the whole
-// matrix resident in the shared memory of one thread-block cluster.
+// k_tri_fx.cu -- Householder tridiagonalisation in 64-bit fixed point on the integer pipe: matrices up
+// to order 615 resident in the shared memory of one thread-block cluster (k_tri_fx), larger ones by
+// the whole grid (k_tri_fx_grid, further down).
 //
 // The FP64 tier's reduction of a Casida matrix (dsyev's dsytrd step) for the sizes that fit.  The
 // grid-wide FP64 kernel (k_sytrd) pays ~10 us per column whatever the size -- a grid barrier, L2 round
@@ -46,28 +47,37 @@ struct FxGroup {
   qk_tri_fx_args req[QK_TRI_FX_GROUP];
 };
 
-// x = h 2^32 + l' with l' signed; l = l' >> 3 (29 bits): in Q62, x = h 2^-30 + l 2^-59
+// x = h 2^32 + l' with l' signed; l = l' >> 1 (31 bits): in Q62, x = h 2^-30 + l 2^-61
 struct Fx {
   int h, l;
 };
 __device__ __forceinline__ Fx fx_split(long long x) {
   const int lo = (int)(unsigned)x;
-  return Fx{(int)(x >> 32) + (int)((unsigned)lo >> 31), lo >> 3};
+  return Fx{(int)(x >> 32) + (int)((unsigned)lo >> 31), lo >> 1};
 }
 __device__ __forceinline__ long long wide(int a, int b) { return (long long)a * b; }
-constexpr long long CR_HALF = 1ll << 26;
+constexpr long long CR_HALF = 1ll << 28;
 // round(x y 2^62): the l l term (zero mean, below 2^-62) is dropped
 __device__ __forceinline__ long long fx_mul(Fx x, Fx y) {
   const long long hh = wide(x.h, y.h);
   const long long cr = CR_HALF + wide(x.h, y.l) + wide(x.l, y.h);
-  return (hh << 2) + (cr >> 27);
+  return (hh << 2) + (cr >> 29);
 }
 // 2 (a b + c d)
 __device__ __forceinline__ long long fx_mul2(Fx a, Fx b, Fx c, Fx d) {
   const long long hh = wide(a.h, b.h) + wide(c.h, d.h);
   const long long cr =
       (CR_HALF >> 1) + wide(a.h, b.l) + wide(a.l, b.h) + wide(c.h, d.l) + wide(c.l, d.h);
-  return (hh << 3) + (cr >> 26);
+  return (hh << 3) + (cr >> 28);
+}
+// the same with the l l term (its upper 29 bits): without it every product errs by 0.3 x 2^-62, which
+// over the thousands of products of a long row outweighs the rounding
+__device__ __forceinline__ long long ll_term(int a, int b) { return wide(a >> 16, b >> 15); }
+__device__ __forceinline__ long long fx_mul2x(Fx a, Fx b, Fx c, Fx d) {
+  const long long hh = wide(a.h, b.h) + wide(c.h, d.h);
+  const long long cr = (CR_HALF >> 1) + wide(a.h, b.l) + wide(a.l, b.h) + wide(c.h, d.l) +
+                       wide(c.l, d.h) + ll_term(a.l, b.l) + ll_term(c.l, d.l);
+  return (hh << 3) + (cr >> 28);
 }
 constexpr long long FX_ONE = 1ll << 62;
 
@@ -143,8 +153,9 @@ struct Scal {             // one column's scalars, written by one thread
   long long dj, alpha;
 };
 
-__device__ __forceinline__ void reflector(long long s0, long long s1, int xs, bool last, long long xj,
-                                          long long alpha, int lane, Scal& out) {
+// from the sums s0 of h^2 and s1 of h l' 2^-sq + l'^2 2^-(33 + sq): |x|^2 = s0 2^-60 + s1 2^(sq - 91)
+__device__ __forceinline__ void reflector(long long s0, long long s1, int sq, int xs, bool last,
+                                          long long xj, long long alpha, int lane, Scal& out) {
   Scal t;
   t.dj = xj;
   t.alpha = alpha;
@@ -153,14 +164,15 @@ __device__ __forceinline__ void reflector(long long s0, long long s1, int xs, bo
   t.sh = 0;
   t.f = t.u1 = t.nx = t.g = 0;
   if (!t.zero) {
-    // |x|^2 = T 2^-89: m4 = T 2^-89 4^(sh - xs) in [1/4, 1)
-    unsigned long long hi = (unsigned long long)(s0 >> 35), lo = (unsigned long long)s0 << 29;
+    // |x|^2 = T 2^(sq - 91): m4 = |x|^2 4^(sh - xs) in [1/4, 1)
+    const int fb = 91 - sq;
+    unsigned long long hi = (unsigned long long)(s0 >> (124 - fb)), lo = (unsigned long long)s0 << (fb - 60);
     const unsigned long long lo2 = lo + (unsigned long long)s1;
     hi += (unsigned long long)(s1 >> 63) + (lo2 < lo ? 1ull : 0ull);
     lo = lo2;
     const int lead = 128 - __clzll((long long)hi);        // bits of T (hi > 0)
-    const int q = (89 - lead) >> 1;                       // T 4^q has 88 or 89 bits
-    const int down = 89 - 62 - 2 * q;                     // m4 (Q62) = T >> down, 0 < down < 64
+    const int q = (fb - lead) >> 1;                       // T 4^q has fb - 1 or fb bits
+    const int down = fb - 62 - 2 * q;                     // m4 (Q62) = T >> down, 0 < down < 64
     const long long m4 = (long long)((hi << (64 - down)) | (lo >> down));
     const long long r = fx_rsqrt4(m4);                    // 1 / (2 |x'|), |x'| = |x| 2^(q + xs)
     const Fx rs = fx_split(r);
@@ -229,7 +241,7 @@ __device__ __forceinline__ void row_pass(long long* As, int lr, int n, int j, in
   }
   long long p[R];
 #pragma unroll
-  for (int q = 0; q < R; ++q) p[q] = (hh[q] << 2) + ((cr[q] + CR_HALF) >> 27);
+  for (int q = 0; q < R; ++q) p[q] = (hh[q] << 2) + ((cr[q] + CR_HALF) >> 29);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -356,11 +368,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
       const Fx K = fx_split(Ksum);
       // ---- w and the updated column x; sums of h^2 and of h l' / 4 + l'^2 / 2^35 ----
       const Fx uj = U[j];
-      const Fx wj = fx_split(P[j] - fx_mul(K, uj) + 4);
+      const Fx wj = fx_split(P[j] - fx_mul(K, uj) + 1);
       long long s0 = 0, s1 = 0;
       for (int i = j + tid; i < n; i += VT) {
         const Fx u = U[i];
-        const Fx w = fx_split(P[i] - fx_mul(K, u) + 4);
+        const Fx w = fx_split(P[i] - fx_mul(K, u) + 1);
         const long long x = X[i] - fx_mul2(u, wj, w, uj);
         Wb[i] = w;
         Xc[i] = x;
@@ -383,9 +395,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
           // ---- the reflector's scalars (one warp; all lanes the same values) ----
           s0 = sum_parts(red[0]);
           s1 = sum_parts(red[1]);
-          // |x|^2 = s0 2^-60 + s1 2^-89; below 2^-25 the sums have too few bits: x << xs instead
-          const bool small = xs == 0 && s0 + (s1 >> 29) < (1ll << 35);
-          if (!small) reflector(s0, s1, xs, j >= n - 2, Xc[j], j + 1 < n ? Xc[j + 1] : 0, lane, sc);
+          // |x|^2 = s0 2^-60 + s1 2^-89; below 2^-22 the sums have too few bits: x << xs instead
+          const bool small = xs == 0 && s0 + (s1 >> 29) < (1ll << 38);
+          if (!small) reflector(s0, s1, 2, xs, j >= n - 2, Xc[j], j + 1 < n ? Xc[j + 1] : 0, lane, sc);
           if (lane == 0) s_small = small;
         }
         vec_bar();
@@ -426,7 +438,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
         for (int i = j + 1 + tid; i < n; i += VT) {
           long long u = 0;
           if (!zero) u = i == j + 1 ? sc.u1 : fx_mul(fx_split(Xc[i] << sh), f);
-          Un[i] = fx_split(u + 4);                  // (the split keeps 59 bits: to nearest)
+          Un[i] = fx_split(u + 1);                  // (the split keeps 61 bits: to nearest)
         }
       }
     }
@@ -461,6 +473,389 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
     cl.sync();
   }
 }
+
+// ---------------------------------------------------------------------------------------------
+// The same reduction for larger matrices: the whole grid (or a group of CTAs per matrix) works on
+// the lower triangle in global memory (L2), converted in place, with one grid barrier per column.
+//
+// The trailing triangle is cut into tiles of 32 rows x 8 columns; a warp takes a contiguous run of
+// tiles, lane = row.  It updates A(i, c), adds y u'_c to its row's sum, parks y in shared memory,
+// and the lanes then sum the tile's columns (4 lanes per column, 8 rows each) against u'_i.  Every
+// tile's sums are rounded to 64 bits on their own and added to p by integer atomics, so p does not
+// depend on the number of CTAs, the runs or the order.  An element costs ~50 issue slots (12 wide
+// multiply-adds at 2 each), half of what the row-wise form of the cluster kernel takes per
+// symmetric pair, and half its L2 traffic, which is why the triangle is kept here.  The O(n) vector
+// work is repeated by every CTA (the same bits), as in k_sytrd.
+// Measured, eigenvalues alone, k_sytrd -> this kernel: n = 700 9.9 -> 6.1 ms, 1575 25.7 -> 15.5, 3600
+// 109.7 -> 64.7 (tridiagonalisation 97.8 -> 53).  A column takes 12.4k cycles at 700 and 30.6k at 3600: the
+// vector work 5.3k / 8.9k (L2 latency, block sums, the reflector), the triangle 2.2k / 16k, the grid
+// barrier 4.6k / 5.1k.  Tried and not kept: the tiles through a ring of asynchronous copies instead of
+// one tile ahead in registers (the triangle 16k -> 19k cycles).
+// ---------------------------------------------------------------------------------------------
+constexpr int GT = 512, GW = GT / 32;     // threads, warps
+constexpr int TC = 8, TLD = 33;           // tile columns, padded rows of a warp's shared tile
+constexpr int G_SMEM_MAX = 226 * 1024;
+
+__device__ __forceinline__ void grid_parts_sum(long long v, long long* red, long long& out) {
+  v = warp_sum64(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < GW; ++w) t += red[w];
+  out = t;
+}
+
+// 8 columns of one tile: update, row sums, transposed sums.  EDGE: the tile meets the diagonal or
+// the last row.
+template <bool EDGE>
+__device__ __forceinline__ void fx_tile(const long long (&x)[TC], long long* col, long long lda, int i, int c0, int n, bool rowok,
+                                        bool upd, Fx ui, Fx wi, const Fx* __restrict__ U,
+                                        const Fx* __restrict__ W, const Fx* __restrict__ Un,
+                                        long long* tile, int lane, int row0, long long& racc,
+                                        long long* pnext) {
+  long long hh = 0, cr = 0;
+#pragma unroll
+  for (int q = 0; q < TC; ++q) {
+    const int c = c0 + q;
+    const bool ok = !EDGE || (rowok && c <= i);
+    long long y = x[q];
+    const Fx v = Un[EDGE ? min(c, n - 1) : c];
+    if (upd) {
+      const Fx u = U[EDGE ? min(c, n - 1) : c], w = W[EDGE ? min(c, n - 1) : c];
+      y -= fx_mul2x(ui, w, wi, u);
+      if (ok) __stcg(col + lda * c, y);
+    }
+    if (EDGE && !ok) y = 0;
+    const Fx ys = fx_split(y);
+    hh += wide(ys.h, v.h);
+    cr += wide(ys.h, v.l) + wide(ys.l, v.h) + ll_term(ys.l, v.l);
+    tile[q * TLD + lane] = EDGE && c >= i ? 0 : y;      // strictly lower
+  }
+  racc += (hh << 2) + ((cr + CR_HALF) >> 29);
+  __syncwarp();
+  // column q of the tile: lanes q, q + 8, q + 16, q + 24 sum 8 rows each
+  const int q = lane & (TC - 1), r8 = (lane >> 3) * 8;
+  const long long* tp = tile + q * TLD + r8;
+  hh = cr = 0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const Fx v = Un[EDGE ? min(row0 + r8 + r, n - 1) : row0 + r8 + r];
+    const Fx ys = fx_split(tp[r]);
+    hh += wide(ys.h, v.h);
+    cr += wide(ys.h, v.l) + wide(ys.l, v.h) + ll_term(ys.l, v.l);
+  }
+  long long t = (hh << 2) + ((cr + CR_HALF) >> 29);
+  t += __shfl_xor_sync(0xffffffffu, t, 8);
+  t += __shfl_xor_sync(0xffffffffu, t, 16);
+  if (lane < TC && (!EDGE || c0 + q < n))
+    atomicAdd((unsigned long long*)(pnext + c0 + q), (unsigned long long)t);
+  __syncwarp();
+}
+
+struct GridWhole {
+  __device__ __forceinline__ int size() const { return (int)gridDim.x; }
+  __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
+};
+struct GridSlice {
+  const int* s;
+  __device__ __forceinline__ int size() const { return *(const volatile int*)s; }
+  __device__ __forceinline__ int rank() const { return *(const volatile int*)(s + 1); }
+};
+
+template <class Grp>
+__device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, const Grp grp) {
+  extern __shared__ long long sm[];
+  __shared__ long long redk[GW], red0[GW], red1[GW];
+  __shared__ unsigned redm[GW];
+  __shared__ int s_small;
+  __shared__ double s_dred[GW];
+  __shared__ Scal sc;
+  const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = grp.size(), rank = grp.rank();
+  const int gthread = rank * GT + tid, totthreads = G * GT;
+  unsigned epoch = 0;
+  Fx* Ub = (Fx*)sm;                      // [2][n]
+  Fx* Wv = Ub + 2 * n;                   // [n]
+  long long* tile = (long long*)(Wv + n) + (size_t)warp * (TC * TLD);
+  long long* Ai = (long long*)a.A;
+  double* rs = a.work + 3 * (size_t)n;   // row sums of |A| and A^2 (before the loop only)
+  double* fs = rs + n;
+  long long* pb = (long long*)a.work;    // [3][n] rotating p
+
+  // ---- norms: a warp per row (fixed order within a row; then every CTA adds the rows alike) ----
+  for (int r = rank * GW + warp; r < n; r += G * GW) {
+    double s = 0.0, f = 0.0;
+#pragma unroll 4
+    for (int c = lane; c < n; c += 32) {
+      const double x = __ldcg(c <= r ? a.A + r + a.lda * c : a.A + c + a.lda * r);
+      s += fabs(x);
+      f = fma(x, x, f);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      f += __shfl_xor_sync(0xffffffffu, f, o);
+    }
+    if (lane == 0) {
+      __stcg(rs + r, s);
+      __stcg(fs + r, f);
+    }
+  }
+  if (!qk_grid_barrier(a.bar, G, epoch, a.status)) return;
+  double m = 0.0, f = 0.0;
+  for (int r = tid; r < n; r += GT) {
+    const double s = __ldcg(rs + r);
+    m = s > m || s != s ? s : m;
+    f += __ldcg(fs + r);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double s = __shfl_xor_sync(0xffffffffu, m, o);
+    m = s > m || s != s ? s : m;
+    f += __shfl_xor_sync(0xffffffffu, f, o);
+  }
+  if (lane == 0) {
+    s_dred[warp] = m;
+    ((double*)red0)[warp] = f;
+  }
+  __syncthreads();
+  m = f = 0.0;
+  for (int w = 0; w < GW; ++w) {
+    const double s = s_dred[w];
+    m = s > m || s != s ? s : m;
+    f += ((double*)red0)[w];
+  }
+  if (!(m <= 1.7976931348623157e308)) {              // NaN or infinity: everything NaN
+    const double qnan = __longlong_as_double(0x7FF8000000000000ll);
+    for (int i = gthread; i < n; i += totthreads) a.d[i] = a.e[i] = a.tau[i] = qnan;
+    for (int j = rank; j < n - 1; j += G)
+      for (int i = j + 1 + tid; i < n; i += GT) a.V[i + a.ldv * j] = qnan;
+    return;
+  }
+  if (f > 1e-200 && f < 1e300) m = fmin(m, 1.000001 * sqrt(f));
+  const int E = m > 0.0 ? ilogb(m) + 1 : 0;
+  // ---- the lower triangle into fixed point, in place; p of the first columns zero ----
+  for (int c = rank; c < n; c += G)
+    for (int i = c + tid; i < n; i += GT)
+      __stcg(Ai + i + a.lda * c, fx_from_double(__ldcg(a.A + i + a.lda * c), E));
+  for (int i = gthread; i < 3 * n; i += totthreads) __stcg(pb + i, 0ll);
+  if (!qk_grid_barrier(a.bar, G, epoch, a.status)) return;
+
+  for (int j = 0; j < n; ++j) {
+    // p of this column in pb[j % 3]; the big pass adds into (j + 1) % 3; (j + 2) % 3 is zeroed
+    const long long* p = pb + (size_t)(j % 3) * n;
+    long long* pnext = pb + (size_t)((j + 1) % 3) * n;
+    long long* pz = pb + (size_t)((j + 2) % 3) * n;
+    const Fx* U = Ub + (j & 1) * n;
+    Fx* Un = Ub + ((j & 1) ^ 1) * n;
+    long long* Xc = (long long*)Un;      // x, until u' takes its place element by element
+    for (int i = gthread; i < n; i += totthreads) __stcg(pz + i, 0ll);
+    // ---- vector work (every CTA) ----
+    const int cnt = n - j;
+    long long Ks = 0;
+    for (int t0 = tid; t0 < cnt; t0 += 4 * GT) {
+      long long pv[4], xv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = j + t0 + q * GT;
+        pv[q] = i < n && j > 0 ? __ldcg(p + i) : 0;
+        xv[q] = i < n ? __ldcg(Ai + i + a.lda * j) : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = j + t0 + q * GT;
+        if (i < n) {
+          Xc[i] = xv[q];
+          ((long long*)Wv)[i] = pv[q];
+          if (j > 0) Ks += fx_mul(fx_split(pv[q]), U[i]);
+        }
+      }
+    }
+    if (j > 0) grid_parts_sum(Ks, redk, Ks);
+    const Fx K = fx_split(Ks);
+    const Fx uj = j > 0 ? U[j] : Fx{0, 0};
+    const long long pj = j > 0 ? __ldcg(p + j) : 0;
+    const Fx wj = fx_split(pj - fx_mul(K, uj) + 1);
+    long long s0 = 0, s1 = 0;
+    for (int i = j + tid; i < n; i += GT) {
+      long long x = Xc[i];
+      if (j > 0) {
+        const Fx u = U[i];
+        const Fx w = fx_split(((long long*)Wv)[i] - fx_mul(K, u) + 1);
+        Wv[i] = w;
+        x -= fx_mul2(u, wj, w, uj);
+        Xc[i] = x;
+      }
+      if (i > j) {
+        const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
+        s0 += wide(h, h);
+        s1 += wide(h, lo >> a.sq) + (wide(lo, lo) >> (33 + a.sq));
+      }
+    }
+    s0 = warp_sum64(s0);
+    s1 = warp_sum64(s1);
+    if (lane == 0) {
+      red0[warp] = s0;
+      red1[warp] = s1;
+    }
+    __syncthreads();
+    int xs = 0;
+    for (;;) {
+      if (warp == 0) {
+        s0 = s1 = 0;
+#pragma unroll
+        for (int w = 0; w < GW; ++w) {
+          s0 += red0[w];
+          s1 += red1[w];
+        }
+        // |x|^2 = s0 2^-60 + s1 2^(sq - 91); below 2^-18 the sums have too few bits: x << xs
+        const bool small = xs == 0 && s0 + (s1 >> (31 - a.sq)) < (1ll << 42);
+        if (!small) reflector(s0, s1, a.sq, xs, j >= n - 2, Xc[j], j + 1 < n ? Xc[j + 1] : 0, lane, sc);
+        if (lane == 0) s_small = small;
+      }
+      __syncthreads();
+      if (!s_small) break;
+      unsigned long long mx = 0;
+      for (int i = j + 1 + tid; i < n; i += GT) {
+        const long long x = Xc[i];
+        const unsigned long long ax = (unsigned long long)(x < 0 ? -x : x);
+        mx = mx > ax ? mx : ax;
+      }
+      unsigned mb = mx ? 64u - (unsigned)__clzll((long long)mx) : 0u;
+      mb = __reduce_max_sync(0xffffffffu, mb);
+      if (lane == 0) redm[warp] = mb;
+      __syncthreads();
+      mb = __reduce_max_sync(0xffffffffu, lane < GW ? redm[lane] : 0u);
+      xs = mb ? a.xbits - (int)mb : -1;     // max |x| << xs below 2^xbits
+      s0 = s1 = 0;
+      if (xs > 0)
+        for (int i = j + 1 + tid; i < n; i += GT) {
+          const long long x = Xc[i] << xs;
+          const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
+          s0 += wide(h, h);
+          s1 += wide(h, lo >> a.sq) + (wide(lo, lo) >> (33 + a.sq));
+        }
+      s0 = warp_sum64(s0);
+      s1 = warp_sum64(s1);
+      if (lane == 0) {
+        red0[warp] = s0;
+        red1[warp] = s1;
+      }
+      __syncthreads();
+    }
+    const Scal t = sc;
+    {
+      const Fx fx = fx_split(t.f);
+      for (int i = j + 1 + tid; i < n; i += GT) {
+        long long u = 0;
+        if (!t.zero) u = i == j + 1 ? t.u1 : fx_mul(fx_split(Xc[i] << t.sh), fx);
+        Un[i] = fx_split(u + 1);
+      }
+    }
+    __syncthreads();
+    // ---- outputs: d, e, tau by one thread, a slice of the V column by every CTA ----
+    if (rank == 0 && tid == 0) {
+      a.d[j] = fx_to_double(t.dj, E + 1 - 62);
+      if (j < n - 1) {
+        a.e[j] = t.zero ? fx_to_double(t.alpha, E + 1 - 62)
+                        : fx_to_double(t.neg ? t.nx : -t.nx, E + 1 - 62 - t.sh);
+        const Fx u1 = fx_split(t.u1);
+        a.tau[j] = fx_to_double(fx_mul(u1, u1), 1 - 62);
+      }
+    }
+    if (j < n - 1) {
+      const Fx g = fx_split(t.u1 < 0 ? -t.g : t.g);
+      for (int i = j + 1 + gthread; i < n; i += totthreads)
+        a.V[i + a.ldv * j] = i == j + 1 ? 1.0 : fx_to_double(fx_mul(Un[i], g), 1 - 62);
+    }
+    // ---- big pass: rows and columns beyond j ----
+    const int r0 = j + 1, mm = n - r0;
+    if (mm > 0) {
+      const bool upd = j > 0;
+      const int nb = (mm + 31) >> 5;
+      const int items = 2 * nb * (nb + 1);             // row block b holds tiles 0 .. 4 b + 3
+      const int totwarps = G * GW;
+      const int per = (items + totwarps - 1) / totwarps;
+      const int it0 = (warp * G + rank) * per, it1 = min(it0 + per, items);
+      if (it0 < it1) {
+        int bi = (int)((sqrtf(2.0f * (float)it0 + 1.0f) - 1.0f) * 0.5f);
+        while (bi > 0 && 2 * bi * (bi + 1) > it0) --bi;
+        while (2 * (bi + 1) * (bi + 2) <= it0) ++bi;
+        int off = 2 * bi * (bi + 1);
+        int i = r0 + 32 * bi + lane;
+        bool rowok = i < n;
+        Fx ui = U[min(i, n - 1)], wi = Wv[min(i, n - 1)];
+        long long racc = 0;
+        long long x[TC], xn[TC];
+        auto edge_of = [&](int b, int c) { return c + TC > r0 + 32 * b || r0 + 32 * b + 32 > n; };
+        auto load = [&](long long (&dst)[TC], int row, bool rok, int b, int c0) {
+          const long long* col = Ai + row;
+          if (!edge_of(b, c0)) {
+#pragma unroll
+            for (int q = 0; q < TC; ++q) dst[q] = __ldcg(col + a.lda * (c0 + q));
+          } else {
+#pragma unroll
+            for (int q = 0; q < TC; ++q)
+              dst[q] = rok && c0 + q <= row ? __ldcg(col + a.lda * (c0 + q)) : 0;
+          }
+        };
+        load(x, i, rowok, bi, r0 + TC * (it0 - off));
+        for (int it = it0; it < it1; ++it) {
+          const int c0 = r0 + TC * (it - off);
+          // the next tile's loads are in flight while this one is worked on
+          int nbi = bi, noff = off;
+          if (it + 1 >= off + 4 * bi + 4) {
+            noff += 4 * bi + 4;
+            ++nbi;
+          }
+          if (it + 1 < it1) {
+            const int ni = r0 + 32 * nbi + lane;
+            load(xn, ni, ni < n, nbi, r0 + TC * (it + 1 - noff));
+          }
+          if (edge_of(bi, c0))
+            fx_tile<true>(x, Ai + i, a.lda, i, c0, n, rowok, upd, ui, wi, U, Wv, Un, tile, lane,
+                          r0 + 32 * bi, racc, pnext);
+          else
+            fx_tile<false>(x, Ai + i, a.lda, i, c0, n, rowok, upd, ui, wi, U, Wv, Un, tile, lane,
+                           r0 + 32 * bi, racc, pnext);
+          if (nbi != bi || it + 1 == it1) {
+            if (rowok) atomicAdd((unsigned long long*)(pnext + i), (unsigned long long)racc);
+            racc = 0;
+            bi = nbi;
+            off = noff;
+            i = r0 + 32 * bi + lane;
+            rowok = i < n;
+            ui = U[min(i, n - 1)];
+            wi = Wv[min(i, n - 1)];
+          }
+#pragma unroll
+          for (int q = 0; q < TC; ++q) x[q] = xn[q];
+        }
+      }
+    }
+    if (!qk_grid_barrier(a.bar, G, epoch, a.status)) return;
+  }
+}
+
+__global__ void __launch_bounds__(GT, 1) k_tri_fx_grid(qk_tri_fx_grid_args a) {
+  tri_fx_grid_body(a, GridWhole{});
+}
+
+// request r on its own CTA group (cta0[r] .. cta0[r + 1] - 1)
+__global__ void __launch_bounds__(GT, 1)
+    k_tri_fx_grid_grouped(const __grid_constant__ qk_tri_fx_grid_group g) {
+  __shared__ int s_grp[2];
+  int r = 0;
+  while (r + 1 < g.nreq && (int)blockIdx.x >= g.cta0[r + 1]) ++r;
+  if ((int)blockIdx.x >= g.cta0[g.nreq]) return;
+  if (threadIdx.x == 0) {
+    s_grp[0] = g.cta0[r + 1] - g.cta0[r];
+    s_grp[1] = (int)blockIdx.x - g.cta0[r];
+  }
+  __syncthreads();
+  tri_fx_grid_body(g.req[r], GridSlice{s_grp});
+}
+
+size_t fx_grid_smem(int n) { return (size_t)n * 24 + (size_t)GW * TC * TLD * 8; }
 
 size_t fx_smem(int n, int cl) {
   const size_t rows = (n + cl - 1) / cl;
@@ -516,6 +911,78 @@ int qk_tri_fx(qk_ctx* ctx, cudaStream_t stream, int R, const qk_tri_fx_args* req
   cfg.attrs = at;
   cfg.numAttrs = 1;
   QK_CK(cudaLaunchKernelEx(&cfg, k_tri_fx, g));
+  ctx->launches++;
+  return QK_OK;
+}
+
+int qk_tri_fx_grid_fits(int n) { return n >= 2 && fx_grid_smem(n) <= (size_t)G_SMEM_MAX; }
+
+namespace {
+int fx_grid_attr() {
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(k_tri_fx_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM_MAX);
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(k_tri_fx_grid_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      G_SMEM_MAX);
+  });
+  return (int)attr_err;
+}
+// the sums of h l' / 2^sq stay below 2^63 (|x| < 1/2): sqrt(n) 2^29 2^(31 - sq) < 2^63
+int fx_sq(int n) {
+  int sq = 2;
+  while ((1ll << (2 * (sq + 3))) < (long long)n * 4 + 4) ++sq;
+  return sq;
+}
+// 2^xbits sqrt(n) <= 2^61: a vector of elements below 2^xbits has a norm below 1/2
+int fx_xbits(int n) {
+  int b = 61;
+  for (long long s = 1; s < n; s *= 4) --b;
+  return b;
+}
+}  // namespace
+
+// cooperative launch over `grid` CTAs (one per SM)
+int qk_tri_fx_grid(qk_ctx* ctx, int grid, qk_tri_fx_grid_args a) {
+  QK_CK((cudaError_t)fx_grid_attr());
+  a.sq = fx_sq(a.n);
+  a.xbits = fx_xbits(a.n);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(GT);
+  cfg.dynamicSmemBytes = fx_grid_smem(a.n);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  QK_CK(cudaLaunchKernelEx(&cfg, k_tri_fx_grid, a));
+  ctx->launches++;
+  return QK_OK;
+}
+
+int qk_tri_fx_grid_launch_group(qk_ctx* ctx, cudaStream_t stream, qk_tri_fx_grid_group& g) {
+  QK_CK((cudaError_t)fx_grid_attr());
+  size_t smem = 0;
+  for (int r = 0; r < g.nreq; ++r) {
+    g.req[r].sq = fx_sq(g.req[r].n);
+    g.req[r].xbits = fx_xbits(g.req[r].n);
+    const size_t s = fx_grid_smem(g.req[r].n);
+    smem = s > smem ? s : smem;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.cta0[g.nreq]);
+  cfg.blockDim = dim3(GT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  QK_CK(cudaLaunchKernelEx(&cfg, k_tri_fx_grid_grouped, g));
   ctx->launches++;
   return QK_OK;
 }

@@ -230,9 +230,9 @@ int qk_bse_dev(qk_ctx* ctx, int TDA_W, int TDA, int singlet, int triplet, int ex
 qk_tri_service* qk_tri_service_new(qk_ctx* parent, int n_workers);
 void qk_tri_service_worker_done(qk_tri_service* svc);
 void qk_tri_service_free(qk_tri_service* svc);
-// tri: TRI_FX (the drivers' FP64 tier) takes the fixed-point cluster kernel (k_tri_fx.cu) where
-// the matrix fits it and else the FP64 kernel; TRI_FP64 always the FP64 kernel; TRI_DF double-float.
-enum { TRI_FX = 0, TRI_DF = 1, TRI_FP64 = 2 };
+// tri: TRI_FX (the drivers' FP64 tier) takes the fixed-point kernels (k_tri_fx.cu) where the matrix
+// fits them and else the FP64 kernel; TRI_FP64 always the FP64 kernel; TRI_DF double-float.
+enum { TRI_FX = 0, TRI_DF = 1, TRI_FP64 = 2, TRI_FX_GRID = 3 /* requests of the service only */ };
 int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, int want_vectors,
                int backtransform = 1, int tri = TRI_FX);
 int qk_tri_fx_cluster(int n);
@@ -245,6 +245,25 @@ struct qk_tri_fx_args {
 };
 constexpr int QK_TRI_FX_GROUP = 32;
 int qk_tri_fx(qk_ctx* ctx, cudaStream_t stream, int R, const qk_tri_fx_args* req);
+// the grid-wide form for larger matrices: A's lower triangle is overwritten, work holds 5 n doubles
+struct qk_tri_fx_grid_args {
+  double* A;
+  long long lda;
+  int n, sq, xbits;   // (the last two are the launcher's)
+  double *d, *e, *tau, *V;
+  long long ldv;
+  double* work;
+  unsigned* bar;
+  int* status;
+};
+struct qk_tri_fx_grid_group {
+  int nreq;
+  int cta0[QK_TRI_FX_GROUP + 1];
+  qk_tri_fx_grid_args req[QK_TRI_FX_GROUP];
+};
+int qk_tri_fx_grid_fits(int n);
+int qk_tri_fx_grid(qk_ctx* ctx, int grid, qk_tri_fx_grid_args a);
+int qk_tri_fx_grid_launch_group(qk_ctx* ctx, cudaStream_t stream, qk_tri_fx_grid_group& g);
 int qk_eig_apply_qt(qk_ctx* ctx, int n, double* X, long long ldx, int ncols, int fp32 = 0);
 
 // Casida pieces (k_casida.cu)

@@ -1,10 +1,11 @@
-"""The fixed-point cluster tridiagonalisation of the FP64 tier's drivers, through qk_dsyev_dev with
-the context setting dsyev_df = 2.
+"""The fixed-point tridiagonalisation of the FP64 tier's drivers, through qk_dsyev_dev with the
+context setting dsyev_df = 2.
 
 An element update rounds to 2^-62 S with S < 4 ||A||_F, so over n columns the backward error of an
 eigenvalue is far below n 2^-53 ||A||_F, the bound used here; the eigenvectors' residuals carry the
 inverse iteration and the back-transformation as well (8 times that).  Sizes: every cluster size,
-their edges, the largest matrix that fits (615) and one that does not (the FP64 kernel takes it).
+their edges, the largest matrix of the cluster form (615) and sizes of the grid form, where the
+number of CTAs must not change a bit.
 """
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ import pytest
 from quack_gb300 import api
 
 pytestmark = pytest.mark.gpu
-SIZES = [2, 3, 31, 33, 64, 65, 128, 129, 200, 256, 257, 401, 615, 616]
+SIZES = [2, 3, 31, 33, 64, 65, 128, 129, 257, 615, 616, 801]
 
 
 def _eig(c, A, lower_only=False):
@@ -61,7 +62,7 @@ def test_casida_and_dense(fx, n):
     _check(fx, A + A.T)
 
 
-@pytest.mark.parametrize("n", [33, 300])
+@pytest.mark.parametrize("n", [33, 300, 640])
 def test_degenerate_columns(fx, n):
     """Columns already reduced, columns of tiny norm, rank deficiency, extreme magnitudes."""
     rng = np.random.default_rng(n)
@@ -78,7 +79,18 @@ def test_degenerate_columns(fx, n):
         assert np.array_equal(w, _eig(fx, C)[0] * scale)
 
 
-def test_nan_gives_nan(fx):
-    A = _casida(50, np.random.default_rng(1))
+@pytest.mark.parametrize("n", [50, 650])
+def test_nan_gives_nan(fx, n):
+    A = _casida(n, np.random.default_rng(1))
     A[20, 7] = A[7, 20] = np.nan
     assert np.isnan(_eig(fx, A)[0]).all()
+
+
+def test_grid_form_independent_of_the_cta_count(fx):
+    A = _casida(700, np.random.default_rng(3))
+    outs = []
+    for quarters in (4, 1, 3):
+        fx.tune_set("sytrd_grid", 700, quarters)
+        outs.append(_eig(fx, A))
+    for w, Z in outs[1:]:
+        assert np.array_equal(w, outs[0][0]) and np.array_equal(Z, outs[0][1])
