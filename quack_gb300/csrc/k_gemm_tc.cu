@@ -69,7 +69,9 @@ struct Operand {           // op(A) as rows x K, or op(B)^T as rows x K
   const double* X;         // X(r, k) = X[r + ld k] (trans = 0) or X[k + ld r]
   long long ld, stride;    // stride between batch entries (0: one shared operand)
   int rows, rb, trans;     // rb: rows per plane block (TM for A, TN for B)
-  int row_blocks, batch;
+  int row_blocks, batch;   // batch: plane sets (1: shared by all batch entries)
+  const double* kscale;    // optional factors of the k index: X(r, k) kscale[k + sk b]
+  long long sk;
   uint8_t* P;              // digit planes: [batch][row block][k block][digit][rb rows][64 B]
   unsigned* info;          // per row: high word of max |x| (exponent; Inf and NaN codes)
   unsigned* part;          // partial maxima [batch][k slab][row] (slabs > 0)
@@ -85,6 +87,9 @@ struct TcGemm {
 };
 
 // ---- operand preparation -----------------------------------------------------------------------
+__device__ __forceinline__ double at_k(const Operand& o, const double* ks, double x, int k) {
+  return ks ? x * ks[k] : x;
+}
 __device__ __forceinline__ unsigned abs_hi(double x) {
   const unsigned hi = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
   return (hi >= HI_INF && (hi > HI_INF || __double2loint(x) != 0)) ? HI_NAN : hi;
@@ -106,6 +111,7 @@ __global__ void __launch_bounds__(256) k_tc_rowmax(Operand a, Operand b, int K, 
   bid /= o.slabs;
   const int strip = bid % strips, bt = bid / strips;
   const double* __restrict__ X = o.X + (long long)bt * o.stride;
+  const double* sc = o.kscale ? o.kscale + (long long)bt * o.sk : nullptr;
   unsigned* out = o.part + ((size_t)bt * o.slabs + ks) * o.row_blocks * o.rb;
   unsigned m = 0;
   if (o.trans) {
@@ -113,7 +119,7 @@ __global__ void __launch_bounds__(256) k_tc_rowmax(Operand a, Operand b, int K, 
     if (r < o.rows) {
       const int k1 = min(K, ks * 1024 + 1024);
 #pragma unroll 8
-      for (int k = ks * 1024 + tx; k < k1; k += 32) m = max(m, abs_hi(X[k + o.ld * r]));
+      for (int k = ks * 1024 + tx; k < k1; k += 32) m = max(m, abs_hi(at_k(o, sc, X[k + o.ld * r], k)));
     }
     m = __reduce_max_sync(0xffffffffu, m);
     if (tx == 0 && r < o.rows) out[r] = m;
@@ -122,7 +128,7 @@ __global__ void __launch_bounds__(256) k_tc_rowmax(Operand a, Operand b, int K, 
     if (r < o.rows) {
       const int k1 = min(K, ks * 256 + 256);
 #pragma unroll 8
-      for (int k = ks * 256 + ty; k < k1; k += 8) m = max(m, abs_hi(X[r + o.ld * k]));
+      for (int k = ks * 256 + ty; k < k1; k += 8) m = max(m, abs_hi(at_k(o, sc, X[r + o.ld * k], k)));
     }
     red[ty][tx] = m;
     __syncthreads();
@@ -167,6 +173,7 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
   const int kb = bid % kblks, bt = bid / kblks;
   const int r0 = strip * 32, k0 = kb * KB;
   const double* __restrict__ X = o.X + (long long)bt * o.stride;
+  const double* sc = o.kscale ? o.kscale + (long long)bt * o.sk : nullptr;
   const size_t rows_pad = (size_t)o.row_blocks * o.rb;
   double v[8];
   if (o.trans) {
@@ -174,7 +181,7 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int r = r0 + ty + 4 * i;
-      v[i] = (r < o.rows && k < K) ? X[k + o.ld * r] : 0.0;
+      v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[k + o.ld * r], k) : 0.0;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) t[ty + 4 * i][tx] = v[i];
@@ -183,7 +190,7 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = k0 + ty + 4 * i;
-      v[i] = (r < o.rows && k < K) ? X[r + o.ld * k] : 0.0;
+      v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[r + o.ld * k], k) : 0.0;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) t[tx][ty + 4 * i] = v[i];
@@ -197,7 +204,7 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
           m = max(m, o.part[((size_t)bt * o.slabs + i) * rows_pad + r0 + tx]);
       } else {
 #pragma unroll 8
-        for (int k = ty; k < K; k += 4) m = max(m, abs_hi(X[r0 + tx + o.ld * k]));
+        for (int k = ty; k < K; k += 4) m = max(m, abs_hi(at_k(o, sc, X[r0 + tx + o.ld * k], k)));
       }
     }
     smax[ty][tx] = m;
@@ -208,7 +215,7 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
       unsigned m = 0;
       if (r < o.rows)
 #pragma unroll 4
-        for (int k = tx; k < K; k += 32) m = max(m, abs_hi(X[k + o.ld * r]));
+        for (int k = tx; k < K; k += 32) m = max(m, abs_hi(at_k(o, sc, X[k + o.ld * r], k)));
       m = __reduce_max_sync(0xffffffffu, m);
       if (tx < 4) smax[tx][ty + 4 * i] = m;
     }
@@ -337,11 +344,12 @@ __device__ __forceinline__ double assemble_scaled(double v, int biased) {
 __device__ __noinline__ double plain_dot(const TcGemm& g, const Unit& t, int row, int col) {
   const double* X = g.a.X + (long long)t.b * g.a.stride;
   const double* Y = g.b.X + (long long)t.b * g.b.stride;
+  const double* ks = g.b.kscale ? g.b.kscale + (long long)t.b * g.b.sk : nullptr;
   const int k1 = min(g.K, t.kb1 * KB);
   double s = 0.0;
   for (int k = t.kb0 * KB; k < k1; ++k)
     s = fma(g.a.trans ? X[k + g.a.ld * row] : X[row + g.a.ld * k],
-            g.b.trans ? Y[k + g.b.ld * col] : Y[col + g.b.ld * k], s);
+            at_k(g.b, ks, g.b.trans ? Y[k + g.b.ld * col] : Y[col + g.b.ld * k], k), s);
   return s;
 }
 
@@ -432,9 +440,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const __grid_constant__
           const Unit t = unit_of(g, u);
           if (skip_unit(g, t)) continue;
           const uint8_t* pa =
-              g.a.P + ((size_t)((g.a.stride ? t.b : 0) * (long long)g.a.row_blocks + t.m) * g.kblks) * A_STAGE;
+              g.a.P + ((size_t)((g.a.batch > 1 ? t.b : 0) * (long long)g.a.row_blocks + t.m) * g.kblks) * A_STAGE;
           const uint8_t* pb =
-              g.b.P + ((size_t)((g.b.stride ? t.b : 0) * (long long)g.b.row_blocks + t.n) * g.kblks) * B_STAGE;
+              g.b.P + ((size_t)((g.b.batch > 1 ? t.b : 0) * (long long)g.b.row_blocks + t.n) * g.kblks) * B_STAGE;
           for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, status)) {
@@ -540,7 +548,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const __grid_constant__
       if (!ok) break;
       const int row = t.m * TM + q * 32 + lane;
       const int c0 = t.n * TN + part * EC;
-      const int ba = g.a.stride ? t.b : 0, bb = g.b.stride ? t.b : 0;
+      const int ba = g.a.batch > 1 ? t.b : 0, bb = g.b.batch > 1 ? t.b : 0;
       const unsigned ia = row < g.M ? g.a.info[(long long)ba * g.a.row_blocks * TM + row] : 0u;
       const unsigned ic = lane < EC && c0 + lane < g.N ? g.b.info[(long long)bb * g.b.row_blocks * TN + c0 + lane] : 0u;
       double* __restrict__ C = g.C + (long long)(t.b * g.slices + t.z) * g.sC + row;
@@ -645,7 +653,7 @@ int tc_panel(qk_ctx* ctx, TcGemm g) {
   auto finish = [&](Operand& o, int rb) {
     o.rb = rb;
     o.row_blocks = (o.rows + rb - 1) / rb;
-    o.batch = o.stride ? g.batch : 1;
+    o.batch = o.stride || o.kscale ? g.batch : 1;
   };
   finish(g.a, TM);
   finish(g.b, TN);
@@ -731,9 +739,21 @@ int tc_panel(qk_ctx* ctx, TcGemm g) {
 int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                long long lda, long long strideA, const double* B, long long ldb, long long strideB,
                double beta, double* C, long long ldc, long long strideC, int batch, bool always) {
+  return qk_gemm_tc_ex(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, nullptr, 0, beta, C,
+                       ldc, strideC, batch, false, always);
+}
+
+int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
+                  long long lda, long long strideA, const double* B, long long ldb, long long strideB,
+                  const double* kscale, long long sK, double beta, double* C, long long ldc,
+                  long long strideC, int batch, bool lower, bool always) {
   if (m <= 0 || n <= 0 || batch <= 0) return QK_OK;
+  if (kscale && !always) return qk_fail(ctx, QK_ERR_ARG, "scaled GEMM: tensor-core path only");
+  if (!always && lower && !qk_gemm_tc_pays(ctx, m, n / 2 + 1, k, batch))
+    return qk_dgemm_lower(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
+                          strideC, batch);
   // (k below 2^20 keeps the integer sums within 95 bits)
-  if (k <= 0 || k > (1 << 20) || !(always || qk_gemm_tc_pays(ctx, m, n, k, batch)))
+  if (k <= 0 || k > (1 << 20) || !(always || lower || qk_gemm_tc_pays(ctx, m, n, k, batch)))
     return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
                     strideC, batch);
   const bool TA = (ta == 'T' || ta == 't'), TB = (tb == 'T' || tb == 't');
@@ -743,20 +763,25 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
   g.beta = beta;
   g.ldc = ldc;
   g.sC = strideC;
-  g.lower = 0;
+  g.lower = lower ? 1 : 0;
   const size_t row_bytes = (size_t)((k + KB - 1) / KB) * 64 * NS;
-  auto panel = [&](int rows, long long stride, int rb) {
-    const size_t per = row_bytes * (stride ? batch : 1);
-    long long p = (long long)(PANEL_BYTES / per) / rb * rb;
+  // batch entries per launch: the planes of one operand within the bound (and grid.y of the split-K
+  // reduction); then row panels where a single entry exceeds it
+  const size_t entry = row_bytes * (size_t)(m > n ? m : n);
+  long long b_step = (long long)(PANEL_BYTES / entry);
+  b_step = b_step < 1 ? 1 : (b_step > 65535 ? 65535 : b_step);
+  if (b_step > batch) b_step = batch;
+  auto panel = [&](int rows, int rb) {
+    long long p = (long long)(PANEL_BYTES / row_bytes) / rb * rb;
     if (p < rb) p = rb;
     return p < rows ? (int)p : rows;
   };
-  const int b_step = batch > 65535 ? 65535 : batch;  // (grid.y of the split-K reduction)
-  const int pm = panel(m, strideA, TM), pn = panel(n, strideB, TN);
-  for (int b0 = 0; b0 < batch; b0 += b_step)
+  const int pm = b_step > 1 ? m : panel(m, TM), pn = b_step > 1 ? n : panel(n, TN);
+  if (lower && (pm < m || pn < n)) return qk_fail(ctx, QK_ERR_ARG, "tensor-core GEMM: lower form too large");
+  for (int b0 = 0; b0 < batch; b0 += (int)b_step)
     for (int j0 = 0; j0 < n; j0 += pn)
       for (int i0 = 0; i0 < m; i0 += pm) {
-        g.batch = batch - b0 < b_step ? batch - b0 : b_step;
+        g.batch = batch - b0 < b_step ? batch - b0 : (int)b_step;
         g.M = m - i0 < pm ? m - i0 : pm;
         g.N = n - j0 < pn ? n - j0 : pn;
         g.a.X = A + b0 * strideA + (TA ? (long long)i0 * lda : i0);
@@ -765,6 +790,8 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
         g.a.rows = g.M;
         g.a.trans = TA;
         g.b.X = B + b0 * strideB + (TB ? j0 : (long long)j0 * ldb);
+        g.b.kscale = kscale ? kscale + b0 * sK : nullptr;
+        g.b.sk = sK;
         g.b.ld = ldb;
         g.b.stride = batch > 1 ? strideB : 0;
         g.b.rows = g.N;

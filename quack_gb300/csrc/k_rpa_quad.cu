@@ -18,8 +18,11 @@
 //   * ln det(I + Q) - tr Q: blocked FP64 Cholesky carried on S = (Schur complement) - I, so that
 //     each pivot contributes (log1p(s) - s) - (Q_ii - s), both second order in Q: no
 //     cancellation of the two first-order terms at large w.
-// Used by the mixed tier for the EcRPA of the G0W0 energies; every other EcRPA comes from the
-// Casida eigenvalues.
+// Used for the EcRPA of the G0W0 energies; every other EcRPA comes from the Casida eigenvalues.  The
+// FP64 tier takes half as many points again, a factor to 1e-15 and exact-product GEMMs for Q and the
+// Cholesky updates (k_gemm_tc.cu), which leaves the accuracy of the eigenvalue route (error ~1e-13
+// of EcRPA): 14 ms at nS = 3600, r = 600 from the tensor (10 ms of it the pivoted Cholesky) against
+// 65 ms for the eigenvalues, 4.4 against 42 ms at nS = 2800, r = 480 from the factor.
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -229,14 +232,15 @@ __global__ void k_lt_transpose(int nS, int r, int rmax, const double* __restrict
   }
 }
 
-// FP32 weights c_q(i) = 4 d_i / (d_i^2 + w_q^2) of every point (Q_q = L^T diag(c_q) L)
+// weights c_q(i) = 4 d_i / (d_i^2 + w_q^2) of every point (Q_q = L^T diag(c_q) L)
+template <class T>
 __global__ void k_quad_weights(int nS, int nq, const double* __restrict__ dd,
-                               const double* __restrict__ om, float* __restrict__ wq) {
+                               const double* __restrict__ om, T* __restrict__ wq) {
   const int total = nS * nq;
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
     const int q = idx / nS, i = idx - q * nS;
     const double d = dd[i], w = om[q];
-    wq[idx] = (float)(4.0 * d / fma(d, d, w * w));
+    wq[idx] = (T)(4.0 * d / fma(d, d, w * w));
   }
 }
 
@@ -409,7 +413,7 @@ void qk_gauss_legendre_host(int n, double* x, double* w) {
 }
 
 int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, const double* ERI,
-                   const double* Lov, int naux, double* Ec, int* applied, bool gap_only) {
+                   const double* Lov, int naux, double* Ec, int* applied, bool fp64) {
   *applied = 0;
   const int no = nO - nC, nv = N - nO - nR, nS = no * nv;
   if (nS <= 0 || (!ERI && !Lov)) return QK_OK;
@@ -429,9 +433,18 @@ int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
     *applied = 1;
     return QK_OK;
   }
-  if (gap_only || !(mm[0] > 0.0) || !(mm[1] >= mm[0])) return QK_OK;
-  const int nq = quad_points(mm[1] / mm[0]);
+  if (!(mm[0] > 0.0) || !(mm[1] >= mm[0])) return QK_OK;
+  int nq = quad_points(mm[1] / mm[0]);
   if (nq == 0) return QK_OK;
+  if (fp64) {
+    // the error falls geometrically with the number of points: 1e-9 Ha at nq, ~1e-13 at 3/2 nq
+    nq += nq / 2;
+    if (nq > 128) return QK_OK;
+    // The r x r factorisations pay below the rank where the eigenvalues cost as much (nS / 3).  The
+    // rank of (ia|jb) from the tensor is only known after its Cholesky, typically a few N: with
+    // nS / 3 below 3 N the attempt would mostly be thrown away (N = 61, nS = 400: 1.3 ms of 7.3).
+    if (Lov ? naux > nS / 3 : nS < 9 * N) return QK_OK;
+  }
 
   // the factor L (nS x r)
   const double* L = Lov;
@@ -452,7 +465,7 @@ int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
     pa.ldk = nS;
     pa.nS = nS;
     pa.rmax = rmax;
-    pa.tol_rel = 1e-12;
+    pa.tol_rel = fp64 ? 1e-15 : 1e-12;
     pa.Lt = Lt;
     pa.r = pv;
     pa.done = (int*)(pv + nS);
@@ -525,8 +538,13 @@ int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
 
   // weights of all points; chunks of points with their Q (nch x r x r) at most ~2 GB
   float* wq = nullptr;
-  QK_TRY(qk_wst(ctx, W_QX, (size_t)nS * nq, &wq));
-  k_quad_weights<<<(nS * nq + 255) / 256, 256, 0, ctx->stream>>>(nS, nq, dd, om, wq);
+  double* wq64 = nullptr;
+  QK_TRY(qk_wst(ctx, W_QX, (size_t)nS * nq, &wq64));
+  wq = (float*)wq64;
+  if (fp64)
+    k_quad_weights<double><<<(nS * nq + 255) / 256, 256, 0, ctx->stream>>>(nS, nq, dd, om, wq64);
+  else
+    k_quad_weights<float><<<(nS * nq + 255) / 256, 256, 0, ctx->stream>>>(nS, nq, dd, om, wq);
   QK_LAUNCHED();
   const long long r2 = (long long)r * r;
   int nch = (int)((size_t)(256u << 20) / (size_t)r2);
@@ -550,8 +568,12 @@ int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
     // products.  (The BF16x3 tensor-core GEMM was measured at 1.3e-5 Ha here: its FP32 tensor-
     // memory accumulation leaves ~1e-6 relative errors in Q, and ln det(1 + Q) - tr Q, second order
     // in Q, does not forgive first-order errors.)
-    QK_TRY(qk_gemm_f32p_lower(ctx, 'T', 'N', r, r, nS, 1.0, L, ldl, 0, L, ldl, 0, 0.0, Q, r, r2,
-                              nc, wq + (size_t)q0 * nS, nS));
+    if (fp64)
+      QK_TRY(qk_gemm_tc_ex(ctx, 'T', 'N', r, r, nS, 1.0, L, ldl, 0, L, ldl, 0, wq64 + (size_t)q0 * nS, nS,
+                           0.0, Q, r, r2, nc, true, true));
+    else
+      QK_TRY(qk_gemm_f32p_lower(ctx, 'T', 'N', r, r, nS, 1.0, L, ldl, 0, L, ldl, 0, 0.0, Q, r, r2,
+                                nc, wq + (size_t)q0 * nS, nS));
     k_quad_diag<<<(r * nc + 255) / 256, 256, 0, ctx->stream>>>(r, nc, Q, qd);
     QK_LAUNCHED();
     for (int kb = 0; kb < r; kb += CB) {
@@ -565,7 +587,11 @@ int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
       QK_LAUNCHED();
       double* P = Q + (kb + nb) + (long long)r * kb;
       double* S22 = Q + (kb + nb) + (long long)r * (kb + nb);
-      QK_TRY(qk_dgemm_lower(ctx, 'N', 'T', m, m, nb, -1.0, P, r, r2, P, r, r2, 1.0, S22, r, r2, nc));
+      if (fp64)
+        QK_TRY(qk_gemm_tc_ex(ctx, 'N', 'T', m, m, nb, -1.0, P, r, r2, P, r, r2, nullptr, 0, 1.0, S22, r,
+                             r2, nc, true, false));
+      else
+        QK_TRY(qk_dgemm_lower(ctx, 'N', 'T', m, m, nb, -1.0, P, r, r2, P, r, r2, 1.0, S22, r, r2, nc));
     }
   }
   k_quad_final<<<1, 32, 0, ctx->stream>>>(nq, wt, acc, Ec);

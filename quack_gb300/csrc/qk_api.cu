@@ -436,10 +436,10 @@ int g0w0_dev(qk_ctx* ctx, const qk_gw_params* prm, const Dims& d, const double* 
   qk_tic(ctx, T_QP);
   QK_TRY(g0w0_qp(ctx, prm, d, flow, eHF, Om, rho, SigC, Z, eGWlin, eGW, ffp));
   qk_toc(ctx, T_QP);
-  // second Casida at eGW for EcRPA (RG0W0.f90:222-225): eigenvalues only; the mixed tier
-  // takes the frequency quadrature of the same energy (r x r problems instead of nS x nS).
-  // Both tiers first check the QP gap: a virtual level below an occupied one makes A - B
-  // indefinite and the energy NaN (phRLR's square roots), which needs no eigenproblem.
+  // second Casida at eGW for EcRPA (RG0W0.f90:222-225): the frequency quadrature of the same
+  // energy (r x r problems instead of nS x nS) in the tier's precision, or where it does not apply
+  // the eigenvalues alone.  The quadrature first checks the QP gap: a virtual level below an
+  // occupied one makes A - B indefinite and the energy NaN (phRLR's square roots).
   qk_tic(ctx, T_CASIDA2);
   int quad = 0;
   if (!prm->TDA_W)  // (with TDA screening A - B plays no part: no square roots, no quadrature)

@@ -151,6 +151,12 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
                long long lda, long long strideA, const double* B, long long ldb, long long strideB,
                double beta, double* C, long long ldc, long long strideC, int batch,
                bool always = false);
+// The general form: op(B)'s k index scaled by kscale[b sK + k] (only with always), lower: only the
+// tiles touching the lower triangle of C.
+int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
+                  long long lda, long long strideA, const double* B, long long ldb, long long strideB,
+                  const double* kscale, long long sK, double beta, double* C, long long ldc,
+                  long long strideC, int batch, bool lower, bool always);
 bool qk_gemm_tc_pays(const qk_ctx* ctx, int m, int n, int k, int batch);
 // The same contract with FP32 products and FP32 partial sums (split-K slices added in FP64);
 // the _lower form computes only the tiles touching the lower triangle of C and can scale the
@@ -176,10 +182,10 @@ int qk_dgemm_lower(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double al
 // from the (ia|jb) block of ERI (pivoted Cholesky) or from Lov (nS x naux).  Writes the energy
 // to the device scalar Ec.  A negative e_a - e_i writes NaN (what the Casida square roots give).
 // *applied = 0 (and nothing written) when the quadrature does not apply (a zero e_a - e_i, a
-// spectrum too wide for the grids, or a factor rank above nS/3) or, with gap_only, whenever
-// the gap is not negative; the caller then takes the eigenvalue route.
+// spectrum too wide for the grids, or a factor rank above nS/3); the caller then takes the
+// eigenvalue route.  fp64: half as many points again, FP64 products, for the FP64 tier.
 int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, const double* ERI,
-                   const double* Lov, int naux, double* Ec, int* applied, bool gap_only = false);
+                   const double* Lov, int naux, double* Ec, int* applied, bool fp64 = false);
 // Gauss-Legendre nodes and weights on [-1, 1] (Newton iteration on P_n).
 void qk_gauss_legendre_host(int n, double* x, double* w);
 
