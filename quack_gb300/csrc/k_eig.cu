@@ -1197,9 +1197,11 @@ __device__ __forceinline__ int sign_bit(double v, int prev_neg) {
   return (((hi & 0x7fffffff) | lo) == 0) ? !prev_neg : (hi < 0);
 }
 
+// (the value p_n(x) = p1 2^(400 s) comes along)
 __device__ __forceinline__ int sturm_count(int n, const double* __restrict__ d,
-                                           const double* __restrict__ e2, double x) {
+                                           const double* __restrict__ e2, double x, double& pn, int& sn) {
   double p0 = 1.0, p1 = __ldg(d) - x;
+  int s = 0;
   int neg = sign_bit(p1, 0);
   int c = neg;
   for (int i = 1; i < n; ++i) {
@@ -1216,12 +1218,16 @@ __device__ __forceinline__ int sturm_count(int n, const double* __restrict__ d,
       if (ex > 1023 + 400) {
         p0 *= 0x1p-400;
         p1 *= 0x1p-400;
+        ++s;
       } else if (ex < 1023 - 400) {
         p0 *= 0x1p+400;
         p1 *= 0x1p+400;
+        --s;
       }
     }
   }
+  pn = p1;
+  sn = s;
   return c;
 }
 
@@ -1304,50 +1310,52 @@ __global__ void k_stebz_grid(int n, const double* __restrict__ d, const double* 
   const double lo = prep[0], hi = prep[1];
   const double h = (hi - lo) / G;
   const double x = lo + h * g;
+  double p;
+  int s;
   cnt[g] = g == 0 ? 0
                   : (g == G ? n
                             : (DF ? sturm_count_df(n, dd, ee, df_from_double(x))
-                                  : sturm_count(n, d, e2, x)));
+                                  : sturm_count(n, d, e2, x, p, s)));
 }
 
-template <int K, bool DF>
-__global__ void __launch_bounds__(128) k_stebz(int n, const double* __restrict__ d,
-                                               const double* __restrict__ e2,
-                                               const float2* __restrict__ dd,
-                                               const float2* __restrict__ ee,
-                                               const double* __restrict__ prep,
-                                               const int* __restrict__ cnt, int G,
-                                               double* __restrict__ w) {
+// the cell [x_g, x_{g+1}) of [lo, hi] with cnt[g] <= j < cnt[g+1] (cnt[0] = 0, cnt[G] = n)
+__device__ __forceinline__ void grid_cell(int j, const int* __restrict__ cnt, int G, double& lo,
+                                          double& hi, int& clo, int& chi) {
+  int a = 0, b = G;
+  while (b - a > 1) {
+    const int mid = (a + b) >> 1;
+    if (cnt[mid] <= j) a = mid;
+    else b = mid;
+  }
+  const double h = (hi - lo) / G;
+  const double x0 = lo + h * a;
+  const double x1 = b == G ? hi : lo + h * b;
+  lo = x0;
+  hi = x1;
+  clo = cnt[a];
+  chi = cnt[b];
+}
+
+template <int K>
+__global__ void __launch_bounds__(128) k_stebz_df(int n, const float2* __restrict__ dd,
+                                                  const float2* __restrict__ ee,
+                                                  const double* __restrict__ prep,
+                                                  const int* __restrict__ cnt, int G,
+                                                  double* __restrict__ w) {
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = gt / K, t = gt % K;
   const bool valid = j < n;
   const int lane = threadIdx.x & 31;
   const unsigned gmask = (K == 32 ? 0xffffffffu : ((1u << K) - 1u)) << (lane & ~(K - 1));
   double lo = prep[0], hi = prep[1];
-  const double pivmin = prep[2];
-  if (cnt && valid) {
-    // the cell [x_g, x_{g+1}) with cnt[g] <= j < cnt[g+1] (cnt[0] = 0, cnt[G] = n)
-    int a = 0, b = G;
-    while (b - a > 1) {
-      const int mid = (a + b) >> 1;
-      if (cnt[mid] <= j) a = mid;
-      else b = mid;
-    }
-    const double h = (hi - lo) / G;
-    const double x0 = lo + h * a;
-    const double x1 = b == G ? hi : lo + h * b;
-    lo = x0;
-    hi = x1;
-  }
-  const double rtol = DF ? 0x1p-45 : 2.0 * DBL_EPSILON;
-  const double atol = DF ? 0x1p-47 * prep[3] : 2.0 * pivmin;
+  int clo, chi;
+  if (cnt && valid) grid_cell(j, cnt, G, lo, hi, clo, chi);
+  const double rtol = 0x1p-45, atol = 0x1p-47 * prep[3];
   for (int it = 0; it < 128; ++it) {
     if (hi - lo <= rtol * fmax(fabs(lo), fabs(hi)) + atol) break;
     const double h = (hi - lo) / (K + 1);
     const double x = lo + h * (t + 1);
-    const int c = !valid ? 0
-                         : (DF ? sturm_count_df(n, dd, ee, df_from_double(x))
-                               : sturm_count(n, d, e2, x));
+    const int c = valid ? sturm_count_df(n, dd, ee, df_from_double(x)) : 0;
     const unsigned le = __ballot_sync(gmask, c <= j) & gmask;
     const int k = __popc(le);
     const double nlo = k > 0 ? lo + h * k : lo;
@@ -1359,34 +1367,109 @@ __global__ void __launch_bounds__(128) k_stebz(int n, const double* __restrict__
   if (valid && t == 0) w[j] = 0.5 * (lo + hi);
 }
 
-void launch_stebz(qk_ctx* ctx, int n, const double* d, const double* e2, const float2* dd,
-                  const float2* ee, const double* prep, const int* cnt, int G, double* w) {
-  const int blocks8 = (int)((8 * (long long)n + 127) / 128);
-  if (dd) {
-    // double-float counts: the FP32 pipe has issue to spare, so 16 lanes per eigenvalue (4.1
-    // bits per sweep) while the warps fit eight per SM sub-partition, else 8
-    const long long slots = 8LL * 4 * 32 * ctx->num_sms;
-    if (slots >= 16LL * n)
-      k_stebz<16, true><<<(int)((16 * (long long)n + 127) / 128), 128, 0, ctx->stream>>>(
-          n, d, e2, dd, ee, prep, cnt, G, w);
-    else
-      k_stebz<8, true><<<blocks8, 128, 0, ctx->stream>>>(n, d, e2, dd, ee, prep, cnt, G, w);
-    return;
+// The same search in FP64, to full precision.  A Sturm sweep takes n steps of three FP64 operations
+// on the SM's FP64 unit, so the sweeps are few: once a bracket holds one
+// eigenvalue between two evaluated points, the characteristic polynomial p_n (whose value comes with
+// the count) is nearly linear in it and the secant predicts the root to about h (h / h1), h the
+// bracket and h1 its width when the eigenvalue was first alone (about the distance to the next).
+// The next points lie about the prediction, in geometric steps from that error out to h, so the
+// bracket shrinks quadratically; where it does not, a plain section follows.  The counts alone
+// decide: a wrong prediction only costs a sweep.  About six sweeps from a grid cell instead of 17 by
+// sections alone.
+template <int K>
+__global__ void __launch_bounds__(32) k_stebz64(int n, const double* __restrict__ d,
+                                                 const double* __restrict__ e2,
+                                                 const double* __restrict__ prep,
+                                                 const int* __restrict__ cnt, int G,
+                                                 double* __restrict__ w) {
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = gt / K, t = gt % K;
+  const bool valid = j < n;
+  const int lane = threadIdx.x & 31, g0 = lane & ~(K - 1);
+  const unsigned gmask = (K == 32 ? 0xffffffffu : ((1u << K) - 1u)) << g0;
+  double lo = prep[0], hi = prep[1];
+  const double pivmin = prep[2];
+  int clo = 0, chi = n;            // counts at lo and hi
+  if (cnt && valid) grid_cell(j, cnt, G, lo, hi, clo, chi);
+  // p_n at the ends, where evaluated (0: not), in units of 2^(400 s)
+  double plo = 0.0, phi = 0.0, h1 = 0.0, r = 0.0;
+  int slo = 0, shi = 0;
+  bool about_r = false;
+  for (int it = 0; it < 128; ++it) {
+    const double h = hi - lo;
+    const double tol = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 2.0 * pivmin;
+    if (h <= tol) break;
+    double x = lo + h / (K + 1) * (t + 1);
+    if (about_r) {
+      const double o0 = fmax(0.375 * tol, 0.5 * h * (h / h1));
+      const int q = t < K / 2 ? K / 2 - 1 - t : t - K / 2;   // 0: nearest to r
+      const double o = o0 * (double)exp2f(log2f((float)(h / o0)) * (float)q * (2.0f / K));
+      x = fmin(hi, fmax(lo, t < K / 2 ? r - o : r + o));
+    }
+    double p = 0.0;
+    int ps = 0;
+    const int c = valid ? sturm_count(n, d, e2, x, p, ps) : 0;
+    const unsigned le = __ballot_sync(gmask, c <= j) & gmask;
+    const int k = __popc(le);                    // points at or below the eigenvalue
+    const int la = g0 + (k > 0 ? k - 1 : 0), lb = g0 + (k < K ? k : K - 1);
+    const double xa = __shfl_sync(gmask, x, la), xb = __shfl_sync(gmask, x, lb);
+    const double pa = __shfl_sync(gmask, p, la), pb = __shfl_sync(gmask, p, lb);
+    const int ca = __shfl_sync(gmask, c, la), cb = __shfl_sync(gmask, c, lb);
+    const int sa = __shfl_sync(gmask, ps, la), sb = __shfl_sync(gmask, ps, lb);
+    const double nlo = k > 0 ? xa : lo, nhi = k < K ? xb : hi;
+    if (!(nlo < nhi) || (!about_r && nlo == lo && nhi == hi)) break;
+    if (k > 0) { plo = pa; slo = sa; clo = ca; }
+    if (k < K) { phi = pb; shi = sb; chi = cb; }
+    lo = nlo;
+    hi = nhi;
+    const double hn = hi - lo;
+    const bool poor = about_r && hn * (K + 1) > h;  // a section would have done better
+    about_r = false;
+    if (chi == clo + 1 && plo != 0.0 && phi != 0.0 && abs(slo - shi) <= 1) {
+      if (h1 == 0.0) {
+        h1 = hn;                                 // first alone
+      } else if (!poor) {
+        const double fa = fabs(plo) * (slo > shi ? 0x1p400 : 1.0);
+        const double fb = fabs(phi) * (shi > slo ? 0x1p400 : 1.0);
+        const double f = fa / (fa + fb);
+        if (f > 0.0 && f < 1.0) {
+          r = lo + hn * f;
+          about_r = true;
+        }
+      }
+    }
   }
-  const long long slots = 4LL * 32 * ctx->num_sms;  // one warp per SM sub-partition
-  int K = slots >= 8LL * n ? 8 : slots >= 4LL * n ? 4 : slots >= 2LL * n ? 2 : 1;
-  const int tk = qk_tune_get(ctx, TUNE_STEBZ_K, n, 0);  // tuned width, if any
-  if (tk == 1 || tk == 2 || tk == 4 || tk == 8) K = tk;
-  const int blocks = (int)((K * (long long)n + 127) / 128);
+  if (valid && t == 0) w[j] = 0.5 * (lo + hi);
+}
+
+void launch_stebz_df(qk_ctx* ctx, int n, const float2* dd, const float2* ee, const double* prep,
+                     const int* cnt, int G, double* w) {
+  // the FP32 pipe has issue to spare, so 16 lanes per eigenvalue (4.1 bits per sweep) while the
+  // warps fit eight per SM sub-partition, else 8
+  const long long slots = 8LL * 4 * 32 * ctx->num_sms;
+  if (slots >= 16LL * n)
+    k_stebz_df<16><<<(int)((16 * (long long)n + 127) / 128), 128, 0, ctx->stream>>>(n, dd, ee, prep,
+                                                                                    cnt, G, w);
+  else
+    k_stebz_df<8><<<(int)((8 * (long long)n + 127) / 128), 128, 0, ctx->stream>>>(n, dd, ee, prep,
+                                                                                  cnt, G, w);
+}
+
+void launch_stebz64(qk_ctx* ctx, int n, const double* d, const double* e2, const double* prep,
+                    const int* cnt, int G, double* w) {
+  // up to six warps per SM, in blocks of one so that they spread evenly (an SM has one FP64 unit,
+  // 16 cycles a warp instruction): fewer lanes take more sweeps, more lanes queue for the unit.
+  // Best of 4, 8, 16, 32 at n = 100..3600: 32 up to 600, 16 at 1131 and 1575, 8 at 2800 and 3600.
+  const long long slots = 6LL * 32 * ctx->num_sms;
+  int K = slots >= 32LL * n ? 32 : slots >= 16LL * n ? 16 : slots >= 8LL * n ? 8 : 4;
+  const int tk = qk_tune_get(ctx, TUNE_STEBZ_K, n, 0);  // tuned width, if any (below 4 counts as 4)
+  if (tk) K = tk >= 32 ? 32 : tk >= 16 ? 16 : tk >= 8 ? 8 : 4;
+  const int blocks = (int)((K * (long long)n + 31) / 32);  // one warp each
   switch (K) {
-    case 8: k_stebz<8, false><<<blocks, 128, 0, ctx->stream>>>(n, d, e2, nullptr, nullptr, prep,
-                                                              cnt, G, w); break;
-    case 4: k_stebz<4, false><<<blocks, 128, 0, ctx->stream>>>(n, d, e2, nullptr, nullptr, prep,
-                                                              cnt, G, w); break;
-    case 2: k_stebz<2, false><<<blocks, 128, 0, ctx->stream>>>(n, d, e2, nullptr, nullptr, prep,
-                                                              cnt, G, w); break;
-    default: k_stebz<1, false><<<blocks, 128, 0, ctx->stream>>>(n, d, e2, nullptr, nullptr, prep,
-                                                               cnt, G, w); break;
+    case 32: k_stebz64<32><<<blocks, 32, 0, ctx->stream>>>(n, d, e2, prep, cnt, G, w); break;
+    case 16: k_stebz64<16><<<blocks, 32, 0, ctx->stream>>>(n, d, e2, prep, cnt, G, w); break;
+    case 8: k_stebz64<8><<<blocks, 32, 0, ctx->stream>>>(n, d, e2, prep, cnt, G, w); break;
+    default: k_stebz64<4><<<blocks, 32, 0, ctx->stream>>>(n, d, e2, prep, cnt, G, w); break;
   }
 }
 
@@ -1398,10 +1481,14 @@ __device__ __forceinline__ double rand_pm1(unsigned long long i, unsigned long l
   return ((double)(z >> 11) * (1.0 / 9007199254740992.0)) * 2.0 - 1.0;
 }
 
+// |x| as an integer that orders like it (a comparison on the FP64 pipe takes 64 cycles)
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
 // reciprocal of a U pivot, tiny pivots perturbed to +-tiny first (stored once, so that the
 // back substitutions multiply instead of divide on their dependency chain)
 __device__ __forceinline__ double pivot_rcp(double u, double tiny) {
-  if (fabs(u) < tiny) u = (u < 0.0) ? -tiny : tiny;
+  if (abs_bits(u) < abs_bits(tiny)) u = (u < 0.0) ? -tiny : tiny;
   return qk_rcp(u);
 }
 
@@ -1447,16 +1534,21 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
       const double ck = e[k];
       const double ak1 = d[k + 1] - x;
       const double bk1 = (k + 1 < n - 1) ? e[k + 1] : 0.0;
-      if (fabs(ck) <= fabs(r0)) {
-        const double m = (r0 != 0.0) ? ck * qk_rcp(r0) : 0.0;
-        at(U0, k) = pivot_rcp(r0, tiny); at(U1, k) = r1; at(U2, k) = r2; at(ML, k) = m;
+      if (abs_bits(ck) <= abs_bits(r0)) {
+        // (one reciprocal for the multiplier and the stored pivot, unless the pivot is tiny)
+        const double rr = qk_rcp(r0);
+        const double m = abs_bits(r0) ? ck * rr : 0.0;
+        at(U0, k) = abs_bits(r0) < abs_bits(tiny) ? pivot_rcp(r0, tiny) : rr;
+        at(U1, k) = r1; at(U2, k) = r2; at(ML, k) = m;
         at(SW, k) = 0.0;
         r0 = ak1 - m * r1;
         r1 = bk1 - m * r2;
         r2 = 0.0;
       } else {
-        const double m = r0 * qk_rcp(ck);
-        at(U0, k) = pivot_rcp(ck, tiny); at(U1, k) = ak1; at(U2, k) = bk1; at(ML, k) = m;
+        const double rr = qk_rcp(ck);
+        const double m = r0 * rr;
+        at(U0, k) = abs_bits(ck) < abs_bits(tiny) ? pivot_rcp(ck, tiny) : rr;
+        at(U1, k) = ak1; at(U2, k) = bk1; at(ML, k) = m;
         at(SW, k) = 1.0;
         const double n0 = r1 - m * ak1;
         const double n1 = r2 - m * bk1;
@@ -1467,11 +1559,19 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
     }
     at(U0, n - 1) = pivot_rcp(r0, tiny); at(U1, n - 1) = 0.0; at(U2, n - 1) = 0.0;
     // ---- start vector ----
-    for (int i = 0; i < n; ++i) Zt[(size_t)jj + N * i] = rand_pm1(i, jj);
+    // (its largest entry and, from the back substitutions, the iterates' are found on the way: a
+    // pass of its own over the vector costs a memory latency per load batch)
+    unsigned long long mxb = 0;
+    int imx = 0;
+    for (int i = 0; i < n; ++i) {
+      const double v = rand_pm1(i, jj);
+      Zt[(size_t)jj + N * i] = v;
+      mxb = max(mxb, abs_bits(v));
+    }
     for (int it = 0; it < iters; ++it) {
       // scale to unit inf-norm
-      double mx = 0.0;
-      for (int i = 0; i < n; ++i) mx = fmax(mx, fabs(Zt[(size_t)jj + N * i]));
+      const double mx = __longlong_as_double((long long)mxb);
+      mxb = 0;
       const double sc = mx > 0.0 ? 1.0 / mx : 1.0;
       // forward: apply P and L^{-1}.  The loads of a batch of SB steps are issued before its
       // stores (they read entries the batch has not written yet), so the memory latency is paid
@@ -1530,6 +1630,7 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
         for (int u = 0; u < SB; ++u) {
           const double yv = (zv[u] - a1[u] * y1 - a2[u] * y2) * a0[u];
           Zt[(size_t)jj + N * (k - u)] = yv;
+          if (abs_bits(yv) >= mxb) { mxb = abs_bits(yv); imx = k - u; }  // (the first of equal ones)
           y2 = y1;
           y1 = yv;
         }
@@ -1537,6 +1638,7 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
       for (; k >= 0; --k) {
         const double yv = (Zt[(size_t)jj + N * k] - at(U1, k) * y1 - at(U2, k) * y2) * at(U0, k);
         Zt[(size_t)jj + N * k] = yv;
+        if (abs_bits(yv) >= mxb) { mxb = abs_bits(yv); imx = k; }
         y2 = y1;
         y1 = yv;
       }
@@ -1544,24 +1646,44 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
       for (int kk = j; kk < jj; ++kk) {
         double dot = 0.0;
         for (int i = 0; i < n; ++i) dot += Zt[(size_t)jj + N * i] * Zt[(size_t)kk + N * i];
-        for (int i = 0; i < n; ++i) Zt[(size_t)jj + N * i] -= dot * Zt[(size_t)kk + N * i];
+        mxb = 0;
+        imx = 0;
+        for (int i = 0; i < n; ++i) {
+          const double v = Zt[(size_t)jj + N * i] - dot * Zt[(size_t)kk + N * i];
+          Zt[(size_t)jj + N * i] = v;
+          if (abs_bits(v) > mxb) { mxb = abs_bits(v); imx = i; }
+        }
       }
     }
     // normalise (2-norm), largest component positive
-    double mx = 0.0, s2 = 0.0;
-    int imx = 0;
-    for (int i = 0; i < n; ++i) {
-      const double v = Zt[(size_t)jj + N * i];
-      if (fabs(v) > mx) { mx = fabs(v); imx = i; }
-    }
+    double s2 = 0.0;
+    const double mx = __longlong_as_double((long long)mxb);
     const double sc0 = mx > 0.0 ? 1.0 / mx : 1.0;
-    for (int i = 0; i < n; ++i) {
-      const double v = Zt[(size_t)jj + N * i] * sc0;
-      s2 += v * v;
+    int i = 0;
+    for (; i + SB <= n; i += SB) {
+      double v[SB];
+#pragma unroll
+      for (int u = 0; u < SB; ++u) v[u] = Zt[(size_t)jj + N * (i + u)];
+#pragma unroll
+      for (int u = 0; u < SB; ++u) {
+        const double t = v[u] * sc0;
+        s2 += t * t;
+      }
+    }
+    for (; i < n; ++i) {
+      const double t = Zt[(size_t)jj + N * i] * sc0;
+      s2 += t * t;
     }
     double sc = sc0 / sqrt(s2);
     if (Zt[(size_t)jj + N * imx] < 0.0) sc = -sc;
-    for (int i = 0; i < n; ++i) Zt[(size_t)jj + N * i] *= sc;
+    for (i = 0; i + SB <= n; i += SB) {
+      double v[SB];
+#pragma unroll
+      for (int u = 0; u < SB; ++u) v[u] = Zt[(size_t)jj + N * (i + u)];
+#pragma unroll
+      for (int u = 0; u < SB; ++u) Zt[(size_t)jj + N * (i + u)] = v[u] * sc;
+    }
+    for (; i < n; ++i) Zt[(size_t)jj + N * i] *= sc;
   }
 }
 
@@ -2021,11 +2143,12 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
       k_stebz_grid<true><<<(STEBZ_GRID + 128) / 128, 128, 0, ctx->stream>>>(
           n, d, e2, dd, ee, prep, STEBZ_GRID, cnt);
     else
-      k_stebz_grid<false><<<(STEBZ_GRID + 128) / 128, 128, 0, ctx->stream>>>(
+      k_stebz_grid<false><<<(STEBZ_GRID + 32) / 32, 32, 0, ctx->stream>>>(
           n, d, e2, nullptr, nullptr, prep, STEBZ_GRID, cnt);
     QK_LAUNCHED();
   }
-  launch_stebz(ctx, n, d, e2, dd, ee, prep, cnt, STEBZ_GRID, w);
+  if (tri_df) launch_stebz_df(ctx, n, dd, ee, prep, cnt, STEBZ_GRID, w);
+  else launch_stebz64(ctx, n, d, e2, prep, cnt, STEBZ_GRID, w);
   QK_LAUNCHED();
   if (!want_vectors) {
     k_tri_unscale<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, prep, w);

@@ -9,7 +9,7 @@
 //                 (size = n)
 //   dgemm_path    FP64 GEMM on DFMA (1) or on the DMMA tensor path (2); qk_dgemm_dev also
 //                 takes 3, exact digit products on tcgen05                      (size = m*n)
-//   stebz_k       lanes per eigenvalue of the k-section bisection {2,4,8}        (size = n)
+//   stebz_k       lanes per eigenvalue of the FP64 bisection {4,8,16,32}         (size = n)
 // qk_autotune times every candidate on buffers of the caller's problem sizes (CUDA events on the
 // context stream, best of two runs) and records the fastest; qk_tune_save / qk_tune_load keep
 // the table as JSON so that a later process starts tuned.
