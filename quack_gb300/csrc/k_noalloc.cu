@@ -18,6 +18,7 @@
 // keeps the last call's contents, so calls whose kernels overlap on the GPU (different streams
 // or host threads on one device) race with each other; serialise them.
 #include "qk_internal.cuh"
+#include "qk_poles.cuh"
 
 #define QK_NOALLOC_MAX_N 1024
 #define QK_NOALLOC_MAX_CHUNKS 128
@@ -27,79 +28,39 @@ static __device__ __align__(256) double qk_noalloc_scratch[QK_NOALLOC_SCRATCH_DO
 
 namespace {
 
-constexpr int NA_WARPS = 8;
-
-// same pole sums as RGW_self_energy_diag.f90:44-84 (one thread per orbital p, warps split m),
-// partials per (m chunk, p) written to part[chunk*N + p] (+ stride for dSig and the occupied part)
-__global__ void __launch_bounds__(NA_WARPS * 32)
+// the pole sums of RGW_self_energy_diag.f90:44-84, a CTA per (tile of 8 orbitals, m chunk)
+__global__ void __launch_bounds__(qk_poles::WARPS * 32, 2)
     k_sigma_partial_noalloc(int N, int nC, int nO, int nR, int nS, int nchunks, int mper, double eta,
                             const double* __restrict__ e, const double* __restrict__ Om,
                             const double* __restrict__ rho, double* __restrict__ part) {
-  extern __shared__ double se[];
-  __shared__ double s0[NA_WARPS][32], s1[NA_WARPS][32], s2[NA_WARPS][32];
-  for (int i = threadIdx.x; i < N; i += blockDim.x) se[i] = e[i];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p = nC + blockIdx.x * 32 + lane;
+  using namespace qk_poles;
+  __shared__ Tile T;
   const int pend = N - nR;
-  __syncthreads();
-  double sig = 0.0, ds = 0.0, so = 0.0;
-  if (p < pend) {
-    const double w = se[p], eta2 = eta * eta;
-    const long long N1 = N, N2 = N1 * N1;
-    const int m0 = blockIdx.y * mper, m1 = min(nS, m0 + mper);
-    for (int m = m0 + warp; m < m1; m += NA_WARPS) {
-      const double om = Om[m];
-      const double* r = rho + p + N2 * m;
-      for (int q = nC; q < nO; ++q) {
-        const double x = r[N1 * q], num = 2.0 * x * x, eps = w - se[q] + om;
-        const double e2 = eps * eps, rr = 1.0 / (e2 + eta2);
-        so += num * eps * rr;
-        ds -= num * (e2 - eta2) * rr * rr;
-      }
-      for (int q = nO; q < pend; ++q) {
-        const double x = r[N1 * q], num = 2.0 * x * x, eps = w - se[q] - om;
-        const double e2 = eps * eps, rr = 1.0 / (e2 + eta2);
-        sig += num * eps * rr;
-        ds -= num * (e2 - eta2) * rr * rr;
-      }
-    }
-    sig += so;
+  const int base = nC + blockIdx.x * PT;
+  const int np = min(PT, pend - base);
+  if (threadIdx.x < np) {
+    T.p[threadIdx.x] = base + threadIdx.x;
+    T.w[threadIdx.x] = e[base + threadIdx.x];
   }
-  s0[warp][lane] = sig;
-  s1[warp][lane] = ds;
-  s2[warp][lane] = so;
   __syncthreads();
-  if (warp == 0 && p < pend) {
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int w = 0; w < NA_WARPS; ++w) { a += s0[w][lane]; b += s1[w][lane]; c += s2[w][lane]; }
-    const size_t o = (size_t)blockIdx.y * N + p, stride = (size_t)nchunks * N;
-    part[o] = a;
-    part[o + stride] = b;
-    part[o + 2 * stride] = c;
-  }
+  Range g;
+  g.N = N;
+  g.nO = nO;
+  g.q0 = nC;
+  g.q1 = pend;
+  g.m0 = blockIdx.y * mper;
+  g.m1 = min(nS, g.m0 + mper);
+  tile_sums<KIND_ETA>(T, np, g, e, Om, rho, eta, 0.0, part + (size_t)blockIdx.y * N,
+                      (size_t)nchunks * N);
 }
 
 __global__ void k_sigma_final_noalloc(int N, int nC, int nO, int nR, int nchunks,
                                       const double* __restrict__ part, double* __restrict__ Sig,
                                       double* __restrict__ Z, double* __restrict__ EcGM) {
   __shared__ double red[32];
-  const size_t stride = (size_t)nchunks * N;
-  double gm = 0.0;
-  for (int p = threadIdx.x; p < N; p += blockDim.x) {
-    double s = 0.0, d = 0.0, o = 0.0;
-    if (p >= nC && p < N - nR) {
-      for (int c = 0; c < nchunks; ++c) {
-        s += part[(size_t)c * N + p];
-        d += part[(size_t)c * N + p + stride];
-        o += part[(size_t)c * N + p + 2 * stride];
-      }
-      if (p >= nO) gm += o;
-    }
-    Sig[p] = s;
-    Z[p] = 1.0 / (1.0 - d);
-  }
-  gm = qk_block_sum(gm, red);
-  if (threadIdx.x == 0) *EcGM = -2.0 * gm;
+  const double gm = qk_poles::final_sums(N, nC, nO, nR, nchunks, part, Sig, Z);
+  const double tot = qk_block_sum(gm, red);
+  if (threadIdx.x == 0) *EcGM = -2.0 * tot;
 }
 
 // device address of the scratch array on the current device (the host-side symbol is only a
@@ -133,19 +94,14 @@ extern "C" int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOr
   if (cudaGetDevice(&dev) != cudaSuccess) return QK_ERR_CUDA;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return QK_ERR_CUDA;
+  // one 32-lane group of m a chunk, more above 128 chunks (the scratch array's size); every
+  // partial sum that the reduction reads is written by the sweep
   const int nact = N - nR - nC;
-  const int ptiles = (nact + 31) / 32;
-  int nchunks = (4 * sms + ptiles - 1) / ptiles;
-  const int maxch = (nS + NA_WARPS - 1) / NA_WARPS;
-  if (nchunks > maxch) nchunks = maxch;
-  if (nchunks > QK_NOALLOC_MAX_CHUNKS) nchunks = QK_NOALLOC_MAX_CHUNKS;
-  if (nchunks < 1) nchunks = 1;
-  const int mper = (nS + nchunks - 1) / nchunks;
-  nchunks = (nS + mper - 1) / mper;
+  const int ptiles = (nact + qk_poles::PT - 1) / qk_poles::PT;
+  const int groups = (nS + 31) / 32;
+  const int mper = 32 * ((groups + QK_NOALLOC_MAX_CHUNKS - 1) / QK_NOALLOC_MAX_CHUNKS);
+  const int nchunks = (nS + mper - 1) / mper;
   cudaStream_t s = (cudaStream_t)stream;
-  // the array keeps the previous call's partial sums: clear the part this call reads
-  if (cudaMemsetAsync(part, 0, sizeof(double) * 3 * (size_t)nchunks * N, s) != cudaSuccess)
-    return QK_ERR_CUDA;
   // launch statuses are taken from the launches themselves, so an earlier error left by the
   // caller's own work is neither reported as this call's nor cleared
   {
@@ -155,7 +111,7 @@ extern "C" int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOr
     double* p11 = part;
     void* args[] = {&a0, &a1, &a2, &a3, &a4, &a5, &a6, &a7, &p8, &p9, &p10, &p11};
     if (cudaLaunchKernel((const void*)k_sigma_partial_noalloc, dim3(ptiles, nchunks),
-                         dim3(NA_WARPS * 32), args, N * sizeof(double), s) != cudaSuccess)
+                         dim3(qk_poles::WARPS * 32), args, 0, s) != cudaSuccess)
       return QK_ERR_CUDA;
   }
   {

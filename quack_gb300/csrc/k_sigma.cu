@@ -15,6 +15,7 @@
 #include <cfloat>
 #include <mutex>
 #include "qk_internal.cuh"
+#include "qk_poles.cuh"
 
 namespace {
 
@@ -50,122 +51,35 @@ struct SigArgs {
   double* part;        // 3 * nchunks * N : sig, dsig, occ-part
 };
 
-__global__ void __launch_bounds__(SIG_WARPS * 32) k_sigma_partial(SigArgs a) {
-  extern __shared__ double se[];  // N energies
-  __shared__ double ssig[SIG_WARPS][32], sds[SIG_WARPS][32], socc[SIG_WARPS][32];
-  const int nl = a.nact ? *a.nact : 0;
-  if (a.list && (int)blockIdx.x * 32 >= nl) return;  // no active orbital in this tile
-  const int N = a.N;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) se[i] = a.eq[i];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pend = N - a.nR;
-  int p;
-  bool pok;
-  if (a.list) {
-    const int idx = blockIdx.x * 32 + lane;
-    pok = idx < nl;
-    p = pok ? a.list[idx] : pend;
-  } else {
-    p = a.nC + blockIdx.x * 32 + lane;
-    pok = p < pend;
+// FP64 sweep: a CTA per (tile of 8 orbitals, chunk); the chunk is an (m range, q range) pair
+template <int KIND>
+__global__ void __launch_bounds__(qk_poles::WARPS * 32, 2) k_sigma_partial(SigArgs a) {
+  using namespace qk_poles;
+  __shared__ Tile T;
+  const int pend = a.N - a.nR;
+  const int base = blockIdx.x * PT;
+  const int np = min(PT, (a.list ? *a.nact : pend - a.nC) - base);
+  if (np <= 0) return;  // no active orbital in this tile
+  if (threadIdx.x < np) {
+    const int p = a.list ? a.list[base + threadIdx.x] : a.nC + base + threadIdx.x;
+    T.p[threadIdx.x] = p;
+    T.w[threadIdx.x] = a.wp ? a.wp[p] : a.eq[p];
   }
   __syncthreads();
-  double sig = 0.0, ds = 0.0, socc_acc = 0.0;
-  if (pok) {
-    const double w = a.wp ? a.wp[p] : se[p];
-    const double eta2 = a.eta * a.eta;
-    const long long N1 = N, N2 = N1 * N1;
-    // chunk = (m range, q range)
-    const int mc = blockIdx.y % a.mchunks, qg = blockIdx.y / a.mchunks;
-    const int m0 = mc * a.mper;
-    const int m1 = min(a.nS, m0 + a.mper);
-    const int qa = a.nC + qg * a.qper, qb = min(pend, qa + a.qper);
-    const int qo0 = qa, qo1 = min(a.nO, qb), qv0 = max(a.nO, qa), qv1 = qb;
-    for (int m = m0 + warp; m < m1; m += SIG_WARPS) {
-      const double om = __ldg(a.Om + m);
-      const double* r = a.rho + p + N2 * m;
-      double so = 0.0;
-      // eta = 0 takes the fast path; otherwise occupied part: eps = w - e_i + Om_m
-      if (!a.doSRG && a.eta == 0.0) {
-        // eta = 0: num*eps/(eps^2) = num/eps and num*eps^2/(eps^2)^2 = num/eps^2
-        double s1 = 0.0, s2 = 0.0, d1 = 0.0;
-        for (int q = qo0; q < qo1; ++q) {
-          const double x = __ldg(r + N1 * q);
-          const double ir = rcp_nr(w - se[q] + om);
-          const double t = (x * x) * ir;
-          s1 += t;
-          d1 = fma(t, ir, d1);
-        }
-        for (int q = qv0; q < qv1; ++q) {
-          const double x = __ldg(r + N1 * q);
-          const double ir = rcp_nr(w - se[q] - om);
-          const double t = (x * x) * ir;
-          s2 += t;
-          d1 = fma(t, ir, d1);
-        }
-        socc_acc += 2.0 * s1;
-        sig += 2.0 * s2;
-        ds -= 2.0 * d1;
-        continue;
-      }
-      for (int q = qo0; q < qo1; ++q) {
-        const double x = __ldg(r + N1 * q);
-        const double num = 2.0 * x * x;
-        const double eps = w - se[q] + om;
-        if (!a.doSRG) {
-          const double e2 = eps * eps;
-          const double rr = rcp_nr(e2 + eta2);
-          so += num * eps * rr;
-          ds -= num * (e2 - eta2) * rr * rr;
-        } else {
-          const double reg = 1.0 - exp(-2.0 * a.flow * eps * eps);
-          const double ie = rcp_nr(eps);
-          so += num * reg * ie;
-          ds -= num * reg * ie * ie;
-        }
-      }
-      socc_acc += so;
-      // virtual part: eps = w - e_a - Om_m
-      for (int q = qv0; q < qv1; ++q) {
-        const double x = __ldg(r + N1 * q);
-        const double num = 2.0 * x * x;
-        const double eps = w - se[q] - om;
-        if (!a.doSRG) {
-          const double e2 = eps * eps;
-          const double rr = rcp_nr(e2 + eta2);
-          sig += num * eps * rr;
-          ds -= num * (e2 - eta2) * rr * rr;
-        } else {
-          const double reg = 1.0 - exp(-2.0 * a.flow * eps * eps);
-          const double ie = rcp_nr(eps);
-          sig += num * reg * ie;
-          ds -= num * reg * ie * ie;
-        }
-      }
-    }
-    sig += socc_acc;
-  }
-  ssig[warp][lane] = sig;
-  sds[warp][lane] = ds;
-  socc[warp][lane] = socc_acc;
-  __syncthreads();
-  if (warp == 0 && p < pend) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int w = 0; w < SIG_WARPS; ++w) {
-      s0 += ssig[w][lane];
-      s1 += sds[w][lane];
-      s2 += socc[w][lane];
-    }
-    const size_t o = (size_t)blockIdx.y * N + p;
-    const size_t stride = (size_t)a.nchunks * N;
-    a.part[o] = s0;
-    a.part[o + stride] = s1;
-    a.part[o + 2 * stride] = s2;
-  }
+  const int mc = blockIdx.y % a.mchunks, qg = blockIdx.y / a.mchunks;
+  Range g;
+  g.N = a.N;
+  g.nO = a.nO;
+  g.q0 = a.nC + qg * a.qper;
+  g.q1 = min(pend, g.q0 + a.qper);
+  g.m0 = mc * a.mper;
+  g.m1 = min(a.nS, g.m0 + a.mper);
+  tile_sums<KIND>(T, np, g, a.eq, a.Om, a.rho, a.eta, a.flow, a.part + (size_t)blockIdx.y * a.N,
+                  (size_t)a.nchunks * a.N);
 }
 
-// Mixed-tier sweep (eta = 0, no SRG).  Same outputs as k_sigma_partial (lanes = orbitals p, CTAs
-// over (p tile, chunk)), but a chunk is an (m range, q range) pair and the 8 warps split the q
+// Mixed-tier sweep (eta = 0, no SRG).  Same outputs as k_sigma_partial; lanes = orbitals p, CTAs
+// over (p tile, chunk), a chunk is an (m range, q range) pair and the 8 warps split the q
 // of their range, each warp running over the whole m range, so that the per-(p,q) setup is done
 // once: c = w - e_q as a float pair (c_hi, c_lo) by TwoSum in FP32 from float pairs of w and e_q,
 // and the window [lo, hi) of the m with |w - e_q +- Om_m| < tau (Om ascending: two bisections).
@@ -411,6 +325,16 @@ __global__ void k_sigma_final(int N, int nC, int nO, int nR, int nchunks,
   }
   gm = qk_block_sum(gm, red);
   if (threadIdx.x == 0 && EcGM) *EcGM = -2.0 * gm;
+}
+
+// the same for the many chunks of the FP64 sweep: a warp per orbital, lanes over the chunks
+__global__ void k_sigma_final64(int N, int nC, int nO, int nR, int nchunks,
+                                const double* __restrict__ part, double* __restrict__ Sig,
+                                double* __restrict__ Z, double* __restrict__ EcGM) {
+  __shared__ double red[32];
+  const double gm = qk_poles::final_sums(N, nC, nO, nR, nchunks, part, Sig, Z);
+  const double tot = qk_block_sum(gm, red);
+  if (threadIdx.x == 0 && EcGM) *EcGM = -2.0 * tot;
 }
 
 // Newton bookkeeping state (device): w, df, nIt, active, nact
@@ -911,7 +835,8 @@ __global__ void k_cert_final(int N, int nC, int nR, int nchunks, const double* _
 static int sigma_sweep(qk_ctx* ctx, int doSRG, double eta, double flow, int N, int nC, int nO, int nR,
                        int nS, const double* eq, const double* wp, const double* Om,
                        const double* rho, const int* list, const int* nact, double** part_out,
-                       int* nchunks_out, const qk_sigma_ff* ff = nullptr, int nact_max = -1) {
+                       int* nchunks_out, const qk_sigma_ff* ff = nullptr, int nact_max = -1,
+                       bool* fp64_out = nullptr) {
   // p tiles: all orbitals, or (with a compacted list) an upper bound on the active count.  The
   // partition of every orbital's terms into chunks (the summation order) is fixed by N and nS
   // alone -- never by how many orbitals are still searching -- so an orbital's Sigma(w) is the
@@ -967,30 +892,42 @@ static int sigma_sweep(qk_ctx* ctx, int doSRG, double eta, double flow, int N, i
       QK_LAUNCHED();
     }
   } else {
-    const int ptiles = (nact_p + 31) / 32;                // launched
-    const int ptiles_all = (nall + 31) / 32 > 0 ? (nall + 31) / 32 : 1;
-    int mchunks = (cm * ctx->num_sms + ptiles_all - 1) / ptiles_all;
-    const int maxch = (nS + SIG_WARPS - 1) / SIG_WARPS;
-    if (mchunks > maxch) mchunks = maxch;
-    if (mchunks < 1) mchunks = 1;
-    const int mper = (nS + mchunks - 1) / mchunks;
-    mchunks = (nS + mper - 1) / mper;
-    // two q groups as well, so that the last few still-searching orbitals keep more SMs busy
-    // (more groups cost staging overhead when all orbitals are active)
-    int qgroups = nq >= 32 ? 2 : 1;
+    // m chunks of one 32-lane group each (more groups a chunk above 256 of them, which bounds the
+    // partial sums); the q range is split so that one tile of orbitals, the end of a Newton
+    // search, still fills the SMs (4 q or more a warp: below that the reduction shows), and
+    // further, down to one q a warp, where all tiles together would leave SMs idle.  A Newton
+    // search of N = 120 with stragglers (SRG) went from 41 to 8.6 ms with the sweep, one of
+    // N = 200 from 19.6 to 8.1 ms
+    const int ptiles = (nact_p + qk_poles::PT - 1) / qk_poles::PT;  // launched
+    const int ptiles_all = (nall + qk_poles::PT - 1) / qk_poles::PT > 0
+                               ? (nall + qk_poles::PT - 1) / qk_poles::PT : 1;
+    const int groups = (nS + 31) / 32 > 0 ? (nS + 31) / 32 : 1;
+    const int mper = 32 * ((groups + 255) / 256);
+    const int mchunks = (nS + mper - 1) / mper > 0 ? (nS + mper - 1) / mper : 1;
+    int qgroups = (cm * ctx->num_sms / 4 + mchunks / 2) / mchunks;
+    if (qgroups > nq / (4 * qk_poles::WARPS)) qgroups = nq / (4 * qk_poles::WARPS);
+    int qfill = ctx->num_sms / (ptiles_all * mchunks);
+    if (qfill > nq / qk_poles::WARPS) qfill = nq / qk_poles::WARPS;
+    if (qgroups < qfill) qgroups = qfill;
+    if (qgroups < 1) qgroups = 1;
     const int qper = (nq + qgroups - 1) / qgroups;
-    qgroups = (nq + qper - 1) / qper;
+    qgroups = qper > 0 ? (nq + qper - 1) / qper : 1;
     nchunks = mchunks * qgroups;
     a.nchunks = nchunks; a.mper = mper; a.mchunks = mchunks; a.qper = qper;
     QK_TRY(qk_wst(ctx, W_MISC, (size_t)3 * nchunks * N + 64, &part));
     a.part = part;
     if (ptiles > 0 && nS > 0) {
-      k_sigma_partial<<<dim3(ptiles, nchunks), SIG_WARPS * 32, N * sizeof(double), ctx->stream>>>(a);
+      const dim3 grid(ptiles, nchunks);
+      const int nt = qk_poles::WARPS * 32;
+      if (doSRG) k_sigma_partial<qk_poles::KIND_SRG><<<grid, nt, 0, ctx->stream>>>(a);
+      else if (eta == 0.0) k_sigma_partial<qk_poles::KIND_ETA0><<<grid, nt, 0, ctx->stream>>>(a);
+      else k_sigma_partial<qk_poles::KIND_ETA><<<grid, nt, 0, ctx->stream>>>(a);
       QK_LAUNCHED();
     }
   }
   *part_out = part;
   *nchunks_out = nchunks;
+  if (fp64_out) *fp64_out = !use_ff;
   return QK_OK;
 }
 
@@ -1021,9 +958,11 @@ int qk_sigma_diag(qk_ctx* ctx, int doSRG, double eta, double flow, int N, int nC
                   double* Z, double* EcGM, const qk_sigma_ff* ff) {
   double* part;
   int nch;
+  bool fp64 = false;
   QK_TRY(sigma_sweep(ctx, doSRG, eta, flow, N, nC, nO, nR, nS, e, nullptr, Om, rho, nullptr,
-                     nullptr, &part, &nch, ff));
-  k_sigma_final<<<1, 1024, 0, ctx->stream>>>(N, nC, nO, nR, nch, part, Sig, Z, EcGM);
+                     nullptr, &part, &nch, ff, -1, &fp64));
+  if (fp64) k_sigma_final64<<<1, 1024, 0, ctx->stream>>>(N, nC, nO, nR, nch, part, Sig, Z, EcGM);
+  else k_sigma_final<<<1, 1024, 0, ctx->stream>>>(N, nC, nO, nR, nch, part, Sig, Z, EcGM);
   QK_LAUNCHED();
   return QK_OK;
 }
