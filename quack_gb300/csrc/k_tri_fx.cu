@@ -482,15 +482,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
 // tiles, lane = row.  It updates A(i, c), adds y u'_c to its row's sum, parks y in shared memory,
 // and the lanes then sum the tile's columns (4 lanes per column, 8 rows each) against u'_i.  Every
 // tile's sums are rounded to 64 bits on their own and added to p by integer atomics, so p does not
-// depend on the number of CTAs, the runs or the order.  An element costs ~50 issue slots (12 wide
-// multiply-adds at 2 each), half of what the row-wise form of the cluster kernel takes per
-// symmetric pair, and half its L2 traffic, which is why the triangle is kept here.  The O(n) vector
-// work is repeated by every CTA (the same bits), as in k_sytrd.
-// Measured, eigenvalues alone, k_sytrd -> this kernel: n = 700 9.9 -> 6.1 ms, 1575 25.7 -> 15.5, 3600
-// 109.7 -> 64.7 (tridiagonalisation 97.8 -> 53).  A column takes 12.4k cycles at 700 and 30.6k at 3600: the
-// vector work 5.3k / 8.9k (L2 latency, block sums, the reflector), the triangle 2.2k / 16k, the grid
-// barrier 4.6k / 5.1k.  Tried and not kept: the tiles through a ring of asynchronous copies instead of
-// one tile ahead in registers (the triangle 16k -> 19k cycles).
+// depend on the number of CTAs, the runs or the order.  An element costs ~65 instructions (16 wide
+// multiply-adds), half of what the row-wise form of the cluster kernel takes per symmetric pair, and
+// half its L2 traffic, which is why the triangle is kept here.  The O(n) vector work is repeated by
+// every CTA (the same bits), as in k_sytrd.  What only the host reads (d, e, tau, V) is written
+// between the arrival at the barrier and the wait.
+// Measured, eigenvalues alone, k_sytrd -> this kernel: n = 700 9.9 -> 4.7 ms, 1575 25.7 -> 12.7, 3600
+// 109.7 -> 55.7.  Cycles of a column at n = 700 / 1296 / 3600: loads of p and x with the products for K
+// 1.4k / 1.7k / 2.5k (an L2 latency and more), K's block sum 0.8k, w and x 0.6k / 0.9k / 1.9k, the
+// reflector with the norm's block sum 1.7k, u' 0.3k / 0.4k / 0.9k, the triangle 1.6k / 2.9k / 14.6k (two
+// thirds of its time instructions issue), the barrier with the CTAs' differences 4.2k / 4.2k / 5.8k.
+// Each of these was worth its 3 to 8 %: the matrix's addresses stepped by lda instead of formed by
+// 64-bit products, the tile parked in split form, u and w read as one 16-byte word, no load after the
+// barrier's last poll, p_j from shared memory.  Tried and not kept: the tiles through a ring of
+// asynchronous copies instead of one tile ahead in registers (the triangle 16k -> 19k cycles), two or
+// four vector elements of a thread together (1 to 4 % slower).
 // ---------------------------------------------------------------------------------------------
 constexpr int GT = 512, GW = GT / 32;     // threads, warps
 constexpr int TC = 8, TLD = 33;           // tile columns, padded rows of a warp's shared tile
@@ -506,42 +512,45 @@ __device__ __forceinline__ void grid_parts_sum(long long v, long long* red, long
   out = t;
 }
 
-// 8 columns of one tile: update, row sums, transposed sums.  EDGE: the tile meets the diagonal or
-// the last row.
+// the last reflector's and w's element of a column, read as one 16-byte word
+struct alignas(16) FxPair {
+  Fx u, w;
+};
+
+// 8 columns of one tile (col: this row of the first): update, row sums, transposed sums.  EDGE: the
+// tile meets the diagonal or the last row.
 template <bool EDGE>
-__device__ __forceinline__ void fx_tile(const long long (&x)[TC], long long* col, long long lda, int i, int c0, int n, bool rowok,
-                                        bool upd, Fx ui, Fx wi, const Fx* __restrict__ U,
-                                        const Fx* __restrict__ W, const Fx* __restrict__ Un,
-                                        long long* tile, int lane, int row0, long long& racc,
+__device__ __forceinline__ void fx_tile(const long long (&x)[TC], long long* col, long long lda, int i,
+                                        int c0, int n, bool rowok, FxPair r,
+                                        const FxPair* __restrict__ UW, const Fx* __restrict__ Un,
+                                        Fx* tile, int lane, int row0, long long& racc,
                                         long long* pnext) {
   long long hh = 0, cr = 0;
 #pragma unroll
   for (int q = 0; q < TC; ++q) {
     const int c = c0 + q;
     const bool ok = !EDGE || (rowok && c <= i);
-    long long y = x[q];
     const Fx v = Un[EDGE ? min(c, n - 1) : c];
-    if (upd) {
-      const Fx u = U[EDGE ? min(c, n - 1) : c], w = W[EDGE ? min(c, n - 1) : c];
-      y -= fx_mul2x(ui, w, wi, u);
-      if (ok) __stcg(col + lda * c, y);
-    }
+    const FxPair k = UW[EDGE ? min(c, n - 1) : c];
+    long long y = x[q] - fx_mul2x(r.u, k.w, r.w, k.u);
+    if (ok) __stcg(col, y);
+    col += lda;
     if (EDGE && !ok) y = 0;
     const Fx ys = fx_split(y);
     hh += wide(ys.h, v.h);
     cr += wide(ys.h, v.l) + wide(ys.l, v.h) + ll_term(ys.l, v.l);
-    tile[q * TLD + lane] = EDGE && c >= i ? 0 : y;      // strictly lower
+    tile[q * TLD + lane] = EDGE && c >= i ? Fx{0, 0} : ys;      // strictly lower
   }
   racc += (hh << 2) + ((cr + CR_HALF) >> 29);
   __syncwarp();
   // column q of the tile: lanes q, q + 8, q + 16, q + 24 sum 8 rows each
   const int q = lane & (TC - 1), r8 = (lane >> 3) * 8;
-  const long long* tp = tile + q * TLD + r8;
+  const Fx* tp = tile + q * TLD + r8;
   hh = cr = 0;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const Fx v = Un[EDGE ? min(row0 + r8 + r, n - 1) : row0 + r8 + r];
-    const Fx ys = fx_split(tp[r]);
+  for (int k = 0; k < 8; ++k) {
+    const Fx v = Un[EDGE ? min(row0 + r8 + k, n - 1) : row0 + r8 + k];
+    const Fx ys = tp[k];
     hh += wide(ys.h, v.h);
     cr += wide(ys.h, v.l) + wide(ys.l, v.h) + ll_term(ys.l, v.l);
   }
@@ -569,15 +578,18 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
   __shared__ long long redk[GW], red0[GW], red1[GW];
   __shared__ unsigned redm[GW];
   __shared__ int s_small;
+  __shared__ long long s_pj;             // p_j and u_j of the column at hand
+  __shared__ Fx s_uj;
   __shared__ double s_dred[GW];
   __shared__ Scal sc;
   const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = grp.size(), rank = grp.rank();
   const int gthread = rank * GT + tid, totthreads = G * GT;
   unsigned epoch = 0;
-  Fx* Ub = (Fx*)sm;                      // [2][n]
-  Fx* Wv = Ub + 2 * n;                   // [n]
-  long long* tile = (long long*)(Wv + n) + (size_t)warp * (TC * TLD);
+  FxPair* UW = (FxPair*)sm;              // [n] u of the last reflector and w (p, until w is known)
+  Fx* Un = (Fx*)(UW + n);                // [n] u'
+  long long* Xc = (long long*)Un;        // x, until u' takes its place element by element
+  Fx* tile = Un + n + (size_t)warp * (TC * TLD);
   long long* Ai = (long long*)a.A;
   double* rs = a.work + 3 * (size_t)n;   // row sums of |A| and A^2 (before the loop only)
   double* fs = rs + n;
@@ -638,6 +650,8 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     for (int i = c + tid; i < n; i += GT)
       __stcg(Ai + i + a.lda * c, fx_from_double(__ldcg(a.A + i + a.lda * c), E));
   for (int i = gthread; i < 3 * n; i += totthreads) __stcg(pb + i, 0ll);
+  for (int i = tid; i < n; i += GT) Un[i] = Fx{0, 0};  // the first column has no update: u = p = 0
+  if (tid == 0) s_uj = Fx{0, 0};
   if (!qk_grid_barrier(a.bar, G, epoch, a.status)) return;
 
   for (int j = 0; j < n; ++j) {
@@ -645,46 +659,42 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     const long long* p = pb + (size_t)(j % 3) * n;
     long long* pnext = pb + (size_t)((j + 1) % 3) * n;
     long long* pz = pb + (size_t)((j + 2) % 3) * n;
-    const Fx* U = Ub + (j & 1) * n;
-    Fx* Un = Ub + ((j & 1) ^ 1) * n;
-    long long* Xc = (long long*)Un;      // x, until u' takes its place element by element
     for (int i = gthread; i < n; i += totthreads) __stcg(pz + i, 0ll);
     // ---- vector work (every CTA) ----
-    const int cnt = n - j;
     long long Ks = 0;
-    for (int t0 = tid; t0 < cnt; t0 += 4 * GT) {
+    for (int t0 = j + tid; t0 < n; t0 += 4 * GT) {
       long long pv[4], xv[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int i = j + t0 + q * GT;
-        pv[q] = i < n && j > 0 ? __ldcg(p + i) : 0;
-        xv[q] = i < n ? __ldcg(Ai + i + a.lda * j) : 0;
+        const int i = t0 + q * GT;
+        if (i < n) {
+          pv[q] = __ldcg(p + i);
+          xv[q] = __ldcg(Ai + i + a.lda * j);
+        }
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int i = j + t0 + q * GT;
+        const int i = t0 + q * GT;
         if (i < n) {
+          const Fx u = Un[i];
           Xc[i] = xv[q];
-          ((long long*)Wv)[i] = pv[q];
-          if (j > 0) Ks += fx_mul(fx_split(pv[q]), U[i]);
+          UW[i] = FxPair{u, Fx{(int)(unsigned)pv[q], (int)(pv[q] >> 32)}};
+          if (i == j) s_pj = pv[q];
+          Ks += fx_mul(fx_split(pv[q]), u);
         }
       }
     }
-    if (j > 0) grid_parts_sum(Ks, redk, Ks);
-    const Fx K = fx_split(Ks);
-    const Fx uj = j > 0 ? U[j] : Fx{0, 0};
-    const long long pj = j > 0 ? __ldcg(p + j) : 0;
-    const Fx wj = fx_split(pj - fx_mul(K, uj) + 1);
+    grid_parts_sum(Ks, redk, Ks);
+    const Fx K = fx_split(Ks), uj = s_uj;
+    const Fx wj = fx_split(s_pj - fx_mul(K, uj) + 1);
     long long s0 = 0, s1 = 0;
     for (int i = j + tid; i < n; i += GT) {
-      long long x = Xc[i];
-      if (j > 0) {
-        const Fx u = U[i];
-        const Fx w = fx_split(((long long*)Wv)[i] - fx_mul(K, u) + 1);
-        Wv[i] = w;
-        x -= fx_mul2(u, wj, w, uj);
-        Xc[i] = x;
-      }
+      const FxPair k = UW[i];
+      const long long pi = (long long)(((unsigned long long)(unsigned)k.w.l << 32) | (unsigned)k.w.h);
+      const Fx w = fx_split(pi - fx_mul(K, k.u) + 1);
+      const long long x = Xc[i] - fx_mul2(k.u, wj, w, uj);
+      UW[i].w = w;
+      Xc[i] = x;
       if (i > j) {
         const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
         s0 += wide(h, h);
@@ -746,31 +756,18 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     {
       const Fx fx = fx_split(t.f);
       for (int i = j + 1 + tid; i < n; i += GT) {
-        long long u = 0;
-        if (!t.zero) u = i == j + 1 ? t.u1 : fx_mul(fx_split(Xc[i] << t.sh), fx);
-        Un[i] = fx_split(u + 1);
+        long long u = fx_mul(fx_split(Xc[i] << t.sh), fx);
+        if (i == j + 1) u = t.u1;
+        if (t.zero) u = 0;
+        const Fx us = fx_split(u + 1);
+        Un[i] = us;
+        if (i == j + 1) s_uj = us;
       }
     }
     __syncthreads();
-    // ---- outputs: d, e, tau by one thread, a slice of the V column by every CTA ----
-    if (rank == 0 && tid == 0) {
-      a.d[j] = fx_to_double(t.dj, E + 1 - 62);
-      if (j < n - 1) {
-        a.e[j] = t.zero ? fx_to_double(t.alpha, E + 1 - 62)
-                        : fx_to_double(t.neg ? t.nx : -t.nx, E + 1 - 62 - t.sh);
-        const Fx u1 = fx_split(t.u1);
-        a.tau[j] = fx_to_double(fx_mul(u1, u1), 1 - 62);
-      }
-    }
-    if (j < n - 1) {
-      const Fx g = fx_split(t.u1 < 0 ? -t.g : t.g);
-      for (int i = j + 1 + gthread; i < n; i += totthreads)
-        a.V[i + a.ldv * j] = i == j + 1 ? 1.0 : fx_to_double(fx_mul(Un[i], g), 1 - 62);
-    }
     // ---- big pass: rows and columns beyond j ----
     const int r0 = j + 1, mm = n - r0;
     if (mm > 0) {
-      const bool upd = j > 0;
       const int nb = (mm + 31) >> 5;
       const int items = 2 * nb * (nb + 1);             // row block b holds tiles 0 .. 4 b + 3
       const int totwarps = G * GW;
@@ -783,19 +780,18 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
         int off = 2 * bi * (bi + 1);
         int i = r0 + 32 * bi + lane;
         bool rowok = i < n;
-        Fx ui = U[min(i, n - 1)], wi = Wv[min(i, n - 1)];
+        FxPair row = UW[min(i, n - 1)];
         long long racc = 0;
         long long x[TC], xn[TC];
         auto edge_of = [&](int b, int c) { return c + TC > r0 + 32 * b || r0 + 32 * b + 32 > n; };
-        auto load = [&](long long (&dst)[TC], int row, bool rok, int b, int c0) {
-          const long long* col = Ai + row;
+        auto load = [&](long long (&dst)[TC], int ri, bool rok, int b, int c0) {
+          const long long* col = Ai + ri + a.lda * c0;
           if (!edge_of(b, c0)) {
 #pragma unroll
-            for (int q = 0; q < TC; ++q) dst[q] = __ldcg(col + a.lda * (c0 + q));
+            for (int q = 0; q < TC; ++q, col += a.lda) dst[q] = __ldcg(col);
           } else {
 #pragma unroll
-            for (int q = 0; q < TC; ++q)
-              dst[q] = rok && c0 + q <= row ? __ldcg(col + a.lda * (c0 + q)) : 0;
+            for (int q = 0; q < TC; ++q, col += a.lda) dst[q] = rok && c0 + q <= ri ? __ldcg(col) : 0;
           }
         };
         load(x, i, rowok, bi, r0 + TC * (it0 - off));
@@ -812,11 +808,11 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
             load(xn, ni, ni < n, nbi, r0 + TC * (it + 1 - noff));
           }
           if (edge_of(bi, c0))
-            fx_tile<true>(x, Ai + i, a.lda, i, c0, n, rowok, upd, ui, wi, U, Wv, Un, tile, lane,
-                          r0 + 32 * bi, racc, pnext);
+            fx_tile<true>(x, Ai + i + a.lda * c0, a.lda, i, c0, n, rowok, row, UW, Un, tile, lane, r0 + 32 * bi,
+                          racc, pnext);
           else
-            fx_tile<false>(x, Ai + i, a.lda, i, c0, n, rowok, upd, ui, wi, U, Wv, Un, tile, lane,
-                           r0 + 32 * bi, racc, pnext);
+            fx_tile<false>(x, Ai + i + a.lda * c0, a.lda, i, c0, n, rowok, row, UW, Un, tile, lane, r0 + 32 * bi,
+                           racc, pnext);
           if (nbi != bi || it + 1 == it1) {
             if (rowok) atomicAdd((unsigned long long*)(pnext + i), (unsigned long long)racc);
             racc = 0;
@@ -824,15 +820,31 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
             off = noff;
             i = r0 + 32 * bi + lane;
             rowok = i < n;
-            ui = U[min(i, n - 1)];
-            wi = Wv[min(i, n - 1)];
+            row = UW[min(i, n - 1)];
           }
 #pragma unroll
           for (int q = 0; q < TC; ++q) x[q] = xn[q];
         }
       }
     }
-    if (!qk_grid_barrier(a.bar, G, epoch, a.status)) return;
+    qk_grid_arrive(a.bar);
+    // ---- outputs, while the other CTAs arrive: d, e, tau by one thread, a slice of the V column by
+    // one warp of every CTA ----
+    if (rank == 0 && tid == 64) {
+      a.d[j] = fx_to_double(sc.dj, E + 1 - 62);
+      if (j < n - 1) {
+        a.e[j] = sc.zero ? fx_to_double(sc.alpha, E + 1 - 62)
+                         : fx_to_double(sc.neg ? sc.nx : -sc.nx, E + 1 - 62 - sc.sh);
+        const Fx u1 = fx_split(sc.u1);
+        a.tau[j] = fx_to_double(fx_mul(u1, u1), 1 - 62);
+      }
+    }
+    if (warp == 1) {
+      const Fx g = fx_split(sc.u1 < 0 ? -sc.g : sc.g);
+      for (int i = j + 1 + rank + G * lane; i < n; i += 32 * G)
+        a.V[i + a.ldv * j] = i == j + 1 ? 1.0 : fx_to_double(fx_mul(Un[i], g), 1 - 62);
+    }
+    if (!qk_grid_wait(a.bar, G, epoch, a.status)) return;
   }
 }
 

@@ -371,26 +371,39 @@ __device__ __forceinline__ unsigned qk_ld_acquire(const unsigned* p) {
 // those writes become visible with it), the poll is an acquire load, and the arrivals of all CTAs
 // form one release sequence on the counter, so the load that sees the full count synchronises
 // with every CTA's arrival; the second __syncthreads passes that on to the whole CTA.
-__device__ __forceinline__ bool qk_grid_barrier(unsigned* counter, unsigned nblocks,
-                                                unsigned& epoch, int* status) {
-  __shared__ int s_ok;
+// The status words are read beside the first poll, not before the arrival or after the last poll:
+// as loads of their own they put two L2 round trips into every barrier.
+// In two halves: what a CTA does between them (by threads other than thread 0) is hidden behind
+// the other CTAs' arrivals and is ordered by the next barrier only.
+__device__ __forceinline__ void qk_grid_arrive(unsigned* counter) {
   __syncthreads();
+  if (threadIdx.x == 0)
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+}
+__device__ __forceinline__ bool qk_grid_wait(unsigned* counter, unsigned nblocks, unsigned& epoch,
+                                             int* status) {
+  __shared__ int s_ok;
   if (threadIdx.x == 0) {
+    const int seen = *(volatile int*)status;
+    const unsigned limit = qk_spin_limit(status);
     int ok = 1;
     epoch++;
-    unsigned target = epoch * nblocks;
-    const unsigned limit = qk_spin_limit(status);
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    const unsigned target = epoch * nblocks;
     unsigned spins = 0;
     while (qk_ld_acquire(counter) < target) {
       if (++spins > limit) { atomicOr(status, QKD_BARRIER_TIMEOUT); ok = 0; break; }
       if (spins > 64) __nanosleep(64);
     }
-    if (ok && (*((volatile int*)status) & QKD_BARRIER_TIMEOUT)) ok = 0;
+    if (seen & QKD_BARRIER_TIMEOUT) ok = 0;
     s_ok = ok;
   }
   __syncthreads();
   return s_ok != 0;
+}
+__device__ __forceinline__ bool qk_grid_barrier(unsigned* counter, unsigned nblocks,
+                                                unsigned& epoch, int* status) {
+  qk_grid_arrive(counter);
+  return qk_grid_wait(counter, nblocks, epoch, status);
 }
 
 // 1/x in FP64: the hardware's approximate FP64 reciprocal (rcp.approx.ftz.f64) refined by two
