@@ -1687,45 +1687,61 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
   }
 }
 
-// Forward compact-WY T factors (upper triangular, dlarft 'F','C') of every reflector block,
-// one CTA per block: T_ii = tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i) with G = V_b^T V_b.
-// G and T are BT_NB x BT_NB per block (leading dimension BT_NB); the last block may hold fewer
-// than BT_NB reflectors (the rest of its T is zero).
-constexpr int LARFT_SMEM = (BT_NB * (BT_NB + 1) + BT_NB) * 8;
-__global__ void __launch_bounds__(BT_NB) k_larft_all(int nref, const double* __restrict__ G,
-                                                     const double* __restrict__ tau,
-                                                     double* __restrict__ T) {
-  extern __shared__ double lsm[];
-  double* sT = lsm;                       // [BT_NB][BT_NB + 1]
-  double* z = lsm + BT_NB * (BT_NB + 1);  // [BT_NB]
-  const int b = blockIdx.x, t = threadIdx.x;
-  const int kb = b * BT_NB;
+// Forward compact-WY T factors (upper triangular, dlarft 'F','C') of every reflector block:
+// T_ii = tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i) with G = V_b^T V_b.  G and T are
+// BT_NB x BT_NB per block (leading dimension BT_NB); the last block may hold fewer than BT_NB
+// reflectors (the rest of its T is zero).
+// T(t, i) needs only row t of T, so a warp takes a row, its lanes the columns i: as soon as T(t, c)
+// is known, every later column adds T(t, c) G(c, i) to one of its two sums (c - t even or odd, the
+// order of a dot product with two chains).  With a CTA per block instead, each column a step of dot
+// products over the rows, the SM's FP64 pipe held a block for 0.47 ms; LARFT_ROWS rows a CTA take
+// 15 us (28 blocks of n = 3600: 60 us).
+constexpr int LARFT_ROWS = 4;
+__global__ void __launch_bounds__(LARFT_ROWS * 32) k_larft_all(int nref, const double* __restrict__ G,
+                                                               const double* __restrict__ tau,
+                                                               double* __restrict__ T) {
+  constexpr int R = BT_NB / 32;
+  __shared__ double sG[32][BT_NB + 1];      // 32 rows c of G
+  const int lane = threadIdx.x & 31, t0 = blockIdx.x * LARFT_ROWS, t = t0 + (threadIdx.x >> 5);
+  const int kb = blockIdx.y * BT_NB;
   const int nb = (nref - kb) < BT_NB ? (nref - kb) : BT_NB;
-  const double* Gb = G + (size_t)b * BT_NB * BT_NB;
-  const double* tb = tau + kb;
-  for (int idx = t; idx < BT_NB * (BT_NB + 1); idx += blockDim.x) sT[idx] = 0.0;
-  __syncthreads();
-  for (int i = 0; i < nb; ++i) {
-    if (t < i) z[t] = Gb[t + BT_NB * i];
+  const double* Gb = G + (size_t)blockIdx.y * BT_NB * BT_NB;
+  double s0[R], s1[R], tv[R], tl[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    s0[r] = s1[r] = tv[r] = 0.0;
+    tl[r] = lane + 32 * r < nb ? tau[kb + lane + 32 * r] : 0.0;
+  }
+#pragma unroll
+  for (int rc = 0; rc < R; ++rc) {
+    const int c0 = 32 * rc;
+    if (c0 >= nb || c0 + 31 < t0) continue;
     __syncthreads();
-    if (t < i) {
-      double s0 = 0.0, s1 = 0.0;
-      int c = t;
-      for (; c + 1 < i; c += 2) {
-        s0 = fma(sT[t * (BT_NB + 1) + c], z[c], s0);
-        s1 = fma(sT[t * (BT_NB + 1) + c + 1], z[c + 1], s1);
-      }
-      if (c < i) s0 = fma(sT[t * (BT_NB + 1) + c], z[c], s0);
-      sT[t * (BT_NB + 1) + i] = -tb[i] * (s0 + s1);
+    for (int idx = threadIdx.x; idx < 32 * (nb - c0); idx += LARFT_ROWS * 32) {
+      const int cc = idx & 31, i = c0 + (idx >> 5);
+      sG[cc][i] = c0 + cc < i ? Gb[c0 + cc + BT_NB * i] : 0.0;
     }
-    if (t == 0) sT[i * (BT_NB + 1) + i] = tb[i];
     __syncthreads();
+    for (int cc = 0; cc < 32; ++cc) {
+      const int c = c0 + cc;
+      if (c < t || c >= nb) continue;
+      double v = -tl[rc] * (s0[rc] + s1[rc]);
+      if (c == t) v = tl[rc];
+      v = __shfl_sync(0xffffffffu, v, cc);
+      if (lane == cc) tv[rc] = v;
+      // (columns i <= c are done; what they add here is not used)
+      if ((c - t) & 1) {
+#pragma unroll
+        for (int r = rc; r < R; ++r) s1[r] = fma(v, sG[cc][lane + 32 * r], s1[r]);
+      } else {
+#pragma unroll
+        for (int r = rc; r < R; ++r) s0[r] = fma(v, sG[cc][lane + 32 * r], s0[r]);
+      }
+    }
   }
-  double* Tb = T + (size_t)b * BT_NB * BT_NB;
-  for (int idx = t; idx < BT_NB * BT_NB; idx += blockDim.x) {
-    const int r = idx % BT_NB, c = idx / BT_NB;
-    Tb[idx] = sT[r * (BT_NB + 1) + c];
-  }
+  double* Tb = T + (size_t)blockIdx.y * BT_NB * BT_NB;
+#pragma unroll
+  for (int r = 0; r < R; ++r) Tb[t + BT_NB * (lane + 32 * r)] = tv[r];
 }
 
 // The two large products of a back-transformation block: FP64 GEMM, or (mixed tier) the
@@ -1768,14 +1784,7 @@ int eig_tfactors(qk_ctx* ctx, int n, const double* V, const double* tau, const d
     const double* Vb = V + (size_t)n * kb;
     QK_TRY(gemm('T', 'N', nb, nb, n, 1.0, Vb, n, 0, Vb, n, 0, 0.0, G + B2 * full, BT_NB, 0, 1));
   }
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(k_larft_all, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    LARFT_SMEM);
-  });
-  QK_CK(attr_err);
-  k_larft_all<<<nblk, BT_NB, LARFT_SMEM, ctx->stream>>>(nref, G, tau, T);
+  k_larft_all<<<dim3(BT_NB / LARFT_ROWS, nblk), LARFT_ROWS * 32, 0, ctx->stream>>>(nref, G, tau, T);
   QK_LAUNCHED();
   *T_out = T;
   return QK_OK;
