@@ -145,15 +145,13 @@ __global__ void __launch_bounds__(128) k_dgemm_dmma(int M, int N, int K, double 
   }
 }
 
-// The same GEMM on the FMA path.  With T = double (DFMA): on GB300 DFMA and DMMA share one FP64
-// datapath and DFMA issues slightly faster (1.2 vs 1.05 TFLOP/s measured), so a plain
-// register-tiled kernel can beat the tensor path: 256 threads, each a 4x4 block of C (rows
-// tx + 16 i, columns ty + 16 j) with 16 independent FMA chains, 8 shared loads per 16 FMA.
-// With T = float the FP64 operands are rounded to FP32 as they are staged and the products and
-// partial sums are FP32 (64x the FP64 issue rate); C stays FP64 (alpha, beta applied in FP64).
-// kscale (FP32 path, batched, no split-K): op(B)(k, n) is scaled by kscale[batch * sK + k] as it
-// is staged, i.e. C = alpha op(A) diag(kscale) op(B) + beta C.
-template <bool TA, bool TB, typename T>
+// The same contract with FP32 products: the FP64 operands are rounded to FP32 as they are staged and
+// the products and partial sums are FP32 (64x the FP64 issue rate); C stays FP64 (alpha, beta applied
+// in FP64).  256 threads, each a 4x4 block of C (rows tx + 16 i, columns ty + 16 j) with 16
+// independent FMA chains, 8 shared loads per 16 FMA.
+// kscale (batched, no split-K): op(B)(k, n) is scaled by kscale[batch * sK + k] as it is staged, i.e.
+// C = alpha op(A) diag(kscale) op(B) + beta C.
+template <bool TA, bool TB>
 __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double alpha,
                                                      const double* __restrict__ A, long long lda,
                                                      long long sA, const double* __restrict__ B,
@@ -162,8 +160,8 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
                                                      long long sC, int kc,
                                                      const float* __restrict__ kscale,
                                                      long long sK) {
-  __shared__ T As[2][BK][BM];
-  __shared__ T Bs[2][BK][BN];
+  __shared__ float As[2][BK][BM];
+  __shared__ float Bs[2][BK][BN];
   const long long bz = blockIdx.z;
   if (kc < 0 && (int)(blockIdx.x + 1) * BM <= (int)blockIdx.y * BN) return;  // lower C only
   int kbeg = 0, kend = K;
@@ -180,16 +178,15 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
 
-  constexpr bool kF32 = sizeof(T) == 4;
-  // FP32: each k tile's 16 products are summed in FP32 and folded into a compensated (hi, lo)
+  // each k tile's 16 products are summed in FP32 and folded into a compensated (hi, lo)
   // pair by TwoSum, so the rounding of the long sum does not grow with K
-  T acc[4][4], lo[4][4];
+  float acc[4][4], lo[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = lo[i][j] = T(0);
+    for (int j = 0; j < 4; ++j) acc[i][j] = lo[i][j] = 0.0f;
 
-  T ra[4], rb[4];
+  float ra[4], rb[4];
   auto ldA = [&](int k0) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -199,7 +196,7 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
       const int gm = m0 + mm, gk = k0 + kk;
       double v = 0.0;
       if (gm < M && gk < kend) v = !TA ? A[gm + lda * gk] : A[gk + lda * gm];
-      ra[r] = (T)v;
+      ra[r] = (float)v;
     }
   };
   auto stA = [&](int st) {
@@ -220,8 +217,8 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
       const int gn = n0 + nn, gk = k0 + kk;
       double v = 0.0;
       if (gn < N && gk < kend) v = !TB ? B[gk + ldb * gn] : B[gn + ldb * gk];
-      rb[r] = (T)v;
-      if (sizeof(T) == 4 && kscale && gk < kend) rb[r] *= (T)kscale[gk];
+      rb[r] = (float)v;
+      if (kscale && gk < kend) rb[r] *= kscale[gk];
     }
   };
   auto stB = [&](int st) {
@@ -243,14 +240,14 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
   for (int k0 = kbeg; k0 < kend; k0 += BK) {
     const bool more = (k0 + BK) < kend;
     if (more) { ldA(k0 + BK); ldB(k0 + BK); }
-    T part[4][4];
+    float part[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) part[i][j] = kF32 ? T(0) : acc[i][j];
+      for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      T af[4], bf[4];
+      float af[4], bf[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) af[i] = As[st][kk][tx + 16 * i];
 #pragma unroll
@@ -264,14 +261,10 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (kF32) {
-          const T a0 = acc[i][j], b0 = part[i][j];
-          const T sum = a0 + b0, bp = sum - a0;
-          lo[i][j] += (a0 - (sum - bp)) + (b0 - bp);
-          acc[i][j] = sum;
-        } else {
-          acc[i][j] = part[i][j];
-        }
+        const float a0 = acc[i][j], b0 = part[i][j];
+        const float sum = a0 + b0, bp = sum - a0;
+        lo[i][j] += (a0 - (sum - bp)) + (b0 - bp);
+        acc[i][j] = sum;
       }
     if (more) { stA(st ^ 1); stB(st ^ 1); }
     __syncthreads();
@@ -295,119 +288,87 @@ __global__ void __launch_bounds__(256) k_gemm_simt(int M, int N, int K, double a
   }
 }
 
-// DFMA GEMM with tall 128 x 32 tiles for outputs with few columns (the quarter transforms of
-// qsGW contract the AO tensor with the nO occupied columns: a 64-wide tile would run mostly on
-// padding).  Same contract as k_gemm_simt<TA, TB, double> (split-K slices, strided batches, no
-// lower-triangle mode): 256 threads, each a 4 x 4 block of C (rows tx + 32 i, columns ty + 8 j),
-// 16 independent FMA chains, 8 shared loads per 16 FMA.
-constexpr int TM = 128, TN = 32;
+// DFMA GEMM: a CTA takes 16 x 16 elements of C, a thread one of them.  An SM issues one FP64 warp
+// instruction per ~16 cycles (DFMA and DMMA share one FP64 datapath), so the two shared loads of an
+// FMA are no burden and register tiling gains nothing; what counts is that all SMs work and none on
+// padding.  Against 64 x 64 tiles (a 4 x 4 block a thread), which it replaced: 48 x 48 x 48 51 -> 5 us
+// (one tile on one SM there), 400 x 128 x 128 34 -> 14 us, 567 x 567 x 128 105 -> 79 us, 2048 x 2048
+// x 256 1815 -> 1750 us, at the FP64 rate.  Same split of K and order of additions: the same bits.
+constexpr int T16 = 16, K16 = 32;
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_gemm_tall(int M, int N, int K, double alpha,
-                                                     const double* __restrict__ A, long long lda,
-                                                     long long sA, const double* __restrict__ B,
-                                                     long long ldb, long long sB, double beta,
-                                                     double* __restrict__ C, long long ldc,
-                                                     long long sC, int kc) {
-  __shared__ double As[2][BK][TM];
-  __shared__ double Bs[2][BK][TN];
+__global__ void __launch_bounds__(256) k_gemm_t16(int M, int N, int K, double alpha,
+                                                  const double* __restrict__ A, long long lda,
+                                                  long long sA, const double* __restrict__ B,
+                                                  long long ldb, long long sB, double beta,
+                                                  double* __restrict__ C, long long ldc,
+                                                  long long sC, int kc) {
+  __shared__ double As[2][K16][T16 + 1], Bs[2][K16][T16 + 1];
   const long long bz = blockIdx.z;
+  const int tm = (M + T16 - 1) / T16;       // tiles of C in one grid dimension, rows fastest
+  const int m0 = (int)(blockIdx.x % tm) * T16, n0 = (int)(blockIdx.x / tm) * T16;
+  if (kc < 0 && m0 + T16 <= n0) return;     // lower C only
   int kbeg = 0, kend = K;
+  C += bz * sC;
   if (kc > 0) {
     kbeg = (int)bz * kc;
     kend = min(K, kbeg + kc);
-    C += bz * sC;
   } else {
     A += bz * sA;
     B += bz * sB;
-    C += bz * sC;
   }
-  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
-  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  double ra[8], rb[2];
-  auto ldA = [&](int k0) {
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const int idx = tid + r * 256;
-      int mm, kk;
-      if (!TA) { mm = idx & (TM - 1); kk = idx >> 7; } else { kk = idx & (BK - 1); mm = idx >> 4; }
-      const int gm = m0 + mm, gk = k0 + kk;
-      ra[r] = (gm < M && gk < kend) ? (!TA ? A[gm + lda * gk] : A[gk + lda * gm]) : 0.0;
-    }
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  double ra[2], rb[2];
+  // an operand's k index runs with the lanes where k is its contiguous direction
+  auto pos = [&](bool kfast, int r, int& x, int& kk) {
+    const int idx = tid + 256 * r;
+    x = kfast ? idx >> 5 : idx & 15;
+    kk = kfast ? idx & 31 : idx >> 4;
   };
-  auto stA = [&](int st) {
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const int idx = tid + r * 256;
-      int mm, kk;
-      if (!TA) { mm = idx & (TM - 1); kk = idx >> 7; } else { kk = idx & (BK - 1); mm = idx >> 4; }
-      As[st][kk][mm] = ra[r];
-    }
-  };
-  auto ldB = [&](int k0) {
+  auto ld = [&](int k0) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int idx = tid + r * 256;
-      int nn, kk;
-      if (!TB) { kk = idx & (BK - 1); nn = idx >> 4; } else { nn = idx & (TN - 1); kk = idx >> 5; }
-      const int gn = n0 + nn, gk = k0 + kk;
-      rb[r] = (gn < N && gk < kend) ? (!TB ? B[gk + ldb * gn] : B[gn + ldb * gk]) : 0.0;
+      int x, kk;
+      pos(TA, r, x, kk);
+      ra[r] = m0 + x < M && k0 + kk < kend ? (TA ? A[k0 + kk + lda * (m0 + x)] : A[m0 + x + lda * (k0 + kk)]) : 0.0;
+      pos(!TB, r, x, kk);
+      rb[r] = n0 + x < N && k0 + kk < kend ? (!TB ? B[k0 + kk + ldb * (n0 + x)] : B[n0 + x + ldb * (k0 + kk)]) : 0.0;
     }
   };
-  auto stB = [&](int st) {
+  auto st = [&](int s) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int idx = tid + r * 256;
-      int nn, kk;
-      if (!TB) { kk = idx & (BK - 1); nn = idx >> 4; } else { nn = idx & (TN - 1); kk = idx >> 5; }
-      Bs[st][kk][nn] = rb[r];
+      int x, kk;
+      pos(TA, r, x, kk);
+      As[s][kk][x] = ra[r];
+      pos(!TB, r, x, kk);
+      Bs[s][kk][x] = rb[r];
     }
   };
-  ldA(kbeg);
-  ldB(kbeg);
-  stA(0);
-  stB(0);
+  double acc = 0.0;
+  ld(kbeg);
+  st(0);
   __syncthreads();
-  int st = 0;
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    const bool more = (k0 + BK) < kend;
-    if (more) { ldA(k0 + BK); ldB(k0 + BK); }
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      double af[4], bf[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) af[i] = As[st][kk][tx + 32 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bf[j] = Bs[st][kk][ty + 8 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(af[i], bf[j], acc[i][j]);
-    }
-    if (more) { stA(st ^ 1); stB(st ^ 1); }
+  int s = 0;
+  for (int k0 = kbeg; k0 < kend; k0 += K16) {
+    const bool more = k0 + K16 < kend;
+    if (more) ld(k0 + K16);
+    const int kn = min(K16, kend - k0);
+#pragma unroll 8
+    for (int kk = 0; kk < kn; ++kk) acc = fma(As[s][kk][tx], Bs[s][kk][ty], acc);
+    if (more) st(s ^ 1);
     __syncthreads();
-    st ^= 1;
+    s ^= 1;
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + tx + 32 * i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + ty + 8 * j;
-      if (gn < N) {
-        double* c = C + gm + ldc * (long long)gn;
-        double v = alpha * acc[i][j];
-        if (beta != 0.0) v += beta * (*c);
-        *c = v;
-      }
-    }
+  if (m0 + tx < M && n0 + ty < N) {
+    double* c = C + m0 + tx + ldc * (long long)(n0 + ty);
+    double v = alpha * acc;
+    if (beta != 0.0) v += beta * (*c);
+    *c = v;
   }
 }
+
+
+constexpr int TM = 128, TN = 32;  // tall tiles for outputs with few columns
 
 // Double-float GEMM (the mixed tier's accurate substitute for FP64 on the FP32 pipe): each FP64
 // operand is staged as an FP32 pair a = ah + al (al = fl32(a - ah)), each product is formed
@@ -559,27 +520,25 @@ __global__ void k_splitk_reduce(int m, int n, int S, const double* __restrict__ 
   }
 }
 
-// path: 0 = DMMA, 1 = DFMA, 2 = FP32 products, 3 = DFMA with tall 128 x 32 tiles,
-// 4 / 5 = double-float products (64 x 64 / 128 x 32 tiles)
+// path: 0 = DMMA, 1 = DFMA, 2 = FP32 products, 4 / 5 = double-float products (64 x 64 / 128 x 32
+// tiles)
 template <bool TA, bool TB>
 void launch(int path, dim3 grid, cudaStream_t st, int m, int n, int k, double alpha,
             const double* A, long long lda, long long sA, const double* B, long long ldb,
             long long sB, double beta, double* C, long long ldc, long long sC, int kc,
             const float* kscale, long long sK) {
-  if (path == 3)
-    k_gemm_tall<TA, TB><<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C,
-                                              ldc, sC, kc);
-  else if (path == 4)
+  if (path == 1) {
+    const long long tiles = (long long)((m + T16 - 1) / T16) * ((n + T16 - 1) / T16);
+    k_gemm_t16<TA, TB><<<dim3((unsigned)tiles, 1, grid.z), 256, 0, st>>>(
+        m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, kc);
+  } else if (path == 4)
     k_gemm_df<TA, TB, 64, 64><<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta,
                                                     C, ldc, sC, kc);
   else if (path == 5)
     k_gemm_df<TA, TB, TM, TN><<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta,
                                                     C, ldc, sC, kc);
-  else if (path == 1)
-    k_gemm_simt<TA, TB, double><<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB,
-                                                      beta, C, ldc, sC, kc, nullptr, 0);
   else if (path == 2)
-    k_gemm_simt<TA, TB, float><<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB,
+    k_gemm_simt<TA, TB><<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB,
                                                      beta, C, ldc, sC, kc, kscale, sK);
   else
     k_dgemm_dmma<TA, TB><<<grid, 128, 0, st>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C,
@@ -619,17 +578,19 @@ int gemm_impl(qk_ctx* ctx, bool fp32, char ta, char tb, int m, int n, int k, dou
   int path = df ? 4 : fp32 ? 2
                         : (qk_tune_get(ctx, TUNE_DGEMM_PATH, (long long)m * n, 1) != 2 ? 1 : 0);
   if (df && (lower || kscale)) return qk_fail(ctx, QK_ERR_ARG, "double-float GEMM: full C only");
-  // 128 x 32 tiles where they cover m x n with clearly less padding than 64 x 64 (outputs with
-  // few columns): DFMA -> path 3, double-float -> path 5
-  if ((path == 1 || path == 4) && !lower && !kscale) {
+  // double-float: 128 x 32 tiles where they cover m x n with clearly less padding than 64 x 64
+  // (outputs with few columns)
+  if (path == 4) {
     const long long a64 = (long long)((m + 63) / 64) * 64 * ((n + 63) / 64) * 64;
     const long long a32 = (long long)((m + TM - 1) / TM) * TM * ((n + TN - 1) / TN) * TN;
-    if (8 * a32 < 7 * a64) path = path == 1 ? 3 : 5;
+    if (8 * a32 < 7 * a64) path = 5;
   }
-  const bool tall = path == 3 || path == 5;
-  const int tm = tall ? TM : BM, tn = tall ? TN : BN;
+  // (DFMA: blocks of 64 x 64 elements count for the split of K only)
+  const int tm = path == 5 ? TM : BM, tn = path == 5 ? TN : BN;
   dim3 grid((m + tm - 1) / tm, (n + tn - 1) / tn, batch);
-  if (grid.y > 65535 || grid.z > 65535) return qk_fail(ctx, QK_ERR_ARG, "qk_dgemm: grid too large");
+  if (grid.y > 65535 || grid.z > 65535 ||
+      (path == 1 && (long long)((m + T16 - 1) / T16) * ((n + T16 - 1) / T16) > 0x7fffffffll))
+    return qk_fail(ctx, QK_ERR_ARG, "qk_dgemm: grid too large");
   const long long tiles = (long long)grid.x * grid.y;
   // fewer output tiles than mult CTAs per SM and a long K: split K and reduce
   const int mult = qk_tune_get(ctx, TUNE_SPLITK_MULT, k, 4);

@@ -803,15 +803,17 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
 }
 
 // Whether the tensor-core path is the faster one for this product.  Both costs are in
-// microseconds on one GB300: DFMA runs its padded 64 x 64 tiles at ~1.1 TFLOP/s; a 128 x 64 x 128
-// chunk on the tensor cores takes ~7.2 us per SM, the operands' preparation moves 32 bytes an
-// element, and its launches cost ~10 us against ~6.
+// microseconds on one GB300: DFMA runs its 16 x 16 tiles at ~1.1 TFLOP/s; a 128 x 64 x 128 chunk on
+// the tensor cores takes ~7.2 us per SM, the operands' preparation moves 32 bytes an element, and its
+// launches and their latency cost ~15 us against ~5 (measured, DFMA / tensor cores: 128 x 128 x 400
+// 16 / 30 us, 400 x 128 x 128 14 / 22, 567 x 128 x 128 20 / 23, 128 x 400 x 400 45 / 33, 400 x 400 x
+// 128 46 / 24).
 bool qk_gemm_tc_pays(const qk_ctx* ctx, int m, int n, int k, int batch) {
   if (k < 16) return false;
-  const double pm = (m + 63) / 64 * 64.0, pn = (n + 63) / 64 * 64.0;
-  const double dfma = 6.0 + 2.0 * pm * pn * k * batch / 1.1e6;
+  const double pm = (m + 15) / 16 * 16.0, pn = (n + 15) / 16 * 16.0;
+  const double dfma = 5.0 + 2.0 * pm * pn * k * batch / 1.1e6;
   const double chunks = (double)((m + TM - 1) / TM) * ((n + TN - 1) / TN) * batch * ((k + 127) / 128);
-  const double tc = 10.0 + 7.2 * (double)((long long)(chunks + ctx->num_sms - 1) / ctx->num_sms) +
+  const double tc = 15.0 + 7.2 * (double)((long long)(chunks + ctx->num_sms - 1) / ctx->num_sms) +
                     ((double)m + n) * k * batch * 32.0 / 4e6;
   return tc < dfma;
 }
