@@ -1478,7 +1478,15 @@ __device__ __forceinline__ double rand_pm1(unsigned long long i, unsigned long l
   z ^= z >> 30; z *= 0xBF58476D1CE4E5B9ull;
   z ^= z >> 27; z *= 0x94D049BB133111EBull;
   z ^= z >> 31;
-  return ((double)(z >> 11) * (1.0 / 9007199254740992.0)) * 2.0 - 1.0;
+  // (z >> 11) 2^-52 - 1, exact, put together from integers: three FP64 operations would take a warp
+  // that has its SM to itself ~200 cycles
+  const long long k = (long long)(z >> 11) - (1ll << 52);
+  if (k == 0) return 0.0;
+  unsigned long long m = (unsigned long long)(k < 0 ? -k : k);
+  const int sh = __clzll((long long)m) - 11;              // leading bit to 52
+  m <<= sh;
+  const unsigned long long sign = k < 0 ? 1ull << 63 : 0ull;
+  return __longlong_as_double((long long)(sign | ((m - (1ull << 52)) + ((unsigned long long)(1023 - sh) << 52))));
 }
 
 // |x| as an integer that orders like it (a comparison on the FP64 pipe takes 64 cycles)
@@ -1492,16 +1500,38 @@ __device__ __forceinline__ double pivot_rcp(double u, double tiny) {
   return qk_rcp(u);
 }
 
+// one forward elimination step: the pivot row's entry is returned, yk becomes the next row's
+__device__ __forceinline__ double fwd_step(double& yk, double yk1, double m, bool swap) {
+  const double top = swap ? yk1 : yk, bot = swap ? yk : yk1;
+  yk = __fma_rn(-m, top, bot);
+  return top;
+}
+
 // Inverse iteration.  Thread j leads the cluster that starts at eigenvalue j (clusters are
-// maximal runs with consecutive gaps <= CLUSTER_REL*||T||_1).  Workspace W holds five
-// interleaved arrays (U0,U1,U2,mult,swap) of n entries per thread: W[(arr*n + i)*n + j].
-// The iterate lives directly in the output row Zt[jj + n*i].
+// maximal runs with consecutive gaps <= CLUSTER_REL*||T||_1).  A vector's factors (U0, U1, U2, the
+// multipliers and the row swaps) and its iterate take 5 n doubles and n flags:
+//  - SM: in shared memory, for the L threads of a CTA.  The sweeps are chains of dependent FP64
+//    operations, and from global memory most of a chain was waiting for its next operands (n = 567:
+//    1.1 ms).
+//  - otherwise in global memory, W[(arr*n + i)*n + j] with the iterate in the output row
+//    Zt[jj + n*i], 32 threads a CTA.
+// The arithmetic is the same.  An FP64 operation takes a warp that has its SM sub-partition to itself
+// 64 to 120 cycles, dependent or not, so their number per row is what counts: comparisons and the
+// random start run on the integer pipe, and FAST (the FP64 tier) leaves out the scaling of the
+// iterates (T is scaled to a norm of about 1) and one step of the pivots' reciprocals; the mixed tier
+// keeps the operations its results were validated with.
+// Cycles per row and three iterations at n = 567, before -> now: factorisation 1010 -> 810, start
+// 330 -> 170, forward 1150 -> 340, back 1320 -> 1100, norm 290 -> 210.
+constexpr int STEIN_ROW = 41;  // bytes of shared memory per row and thread
+template <bool SM, bool FAST>
 __global__ void k_stein(int n, const double* __restrict__ d, const double* __restrict__ e,
                         const double* __restrict__ w, const double* __restrict__ prep,
                         double* __restrict__ W, double* __restrict__ Zt,
-                        const int* __restrict__ status, int iters) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
+                        const int* __restrict__ status, int iters, int L) {
+  extern __shared__ double stein_sm[];
+  const int lane = threadIdx.x;
+  const int j = blockIdx.x * L + lane;
+  if (lane >= L || j >= n) return;
   // after a failed tridiagonalisation (barrier expired) T is meaningless -- possibly one cluster
   // of n equal eigenvalues, whose Gram-Schmidt would take seconds: the call fails anyway
   if (*(const volatile int*)status & QKD_BARRIER_TIMEOUT) return;
@@ -1512,13 +1542,19 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
   while (jend + 1 < n && w[jend + 1] - w[jend] <= ortol) ++jend;
 
   const size_t N = (size_t)n;
-  double* U0 = W + 0 * N * N;
-  double* U1 = W + 1 * N * N;
-  double* U2 = W + 2 * N * N;
-  double* ML = W + 3 * N * N;
-  double* SW = W + 4 * N * N;
-  auto at = [&](double* arr, int i) -> double& { return arr[(size_t)i * N + j]; };
-  const double tiny = DBL_EPSILON * tnrm;
+  const size_t AS = SM ? N * L : N * N;      // stride of the arrays, of a row, and the thread's column
+  const size_t RS = SM ? (size_t)L : N;
+  double* base = SM ? stein_sm + lane : W + j;
+  double *U0 = base, *U1 = base + AS, *U2 = base + 2 * AS, *ML = base + 3 * AS, *SW = base + 4 * AS;
+  unsigned char* swb = (unsigned char*)(stein_sm + 5 * AS) + lane;   // (SM: SW holds the iterate)
+  auto at = [&](double* arr, int i) -> double& { return arr[RS * i]; };
+  auto set_swap = [&](int i, bool v) {
+    if (SM) swb[RS * i] = v;
+    else at(SW, i) = v ? 1.0 : 0.0;
+  };
+  auto swapped = [&](int i) { return SM ? swb[RS * i] != 0 : at(SW, i) != 0.0; };
+  // (tnrm >= 1/2 unless T = 0: pivots of at least 2^-53 bound the iterates, see FAST)
+  const double tiny = FAST && tnrm == 0.0 ? DBL_EPSILON : DBL_EPSILON * tnrm;
   double xprev = -INFINITY;
 
   for (int jj = j; jj <= jend; ++jj) {
@@ -1534,86 +1570,61 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
       const double ck = e[k];
       const double ak1 = d[k + 1] - x;
       const double bk1 = (k + 1 < n - 1) ? e[k + 1] : 0.0;
-      if (abs_bits(ck) <= abs_bits(r0)) {
-        // (one reciprocal for the multiplier and the stored pivot, unless the pivot is tiny)
-        const double rr = qk_rcp(r0);
-        const double m = abs_bits(r0) ? ck * rr : 0.0;
-        at(U0, k) = abs_bits(r0) < abs_bits(tiny) ? pivot_rcp(r0, tiny) : rr;
-        at(U1, k) = r1; at(U2, k) = r2; at(ML, k) = m;
-        at(SW, k) = 0.0;
-        r0 = ak1 - m * r1;
-        r1 = bk1 - m * r2;
-        r2 = 0.0;
-      } else {
-        const double rr = qk_rcp(ck);
-        const double m = r0 * rr;
-        at(U0, k) = abs_bits(ck) < abs_bits(tiny) ? pivot_rcp(ck, tiny) : rr;
-        at(U1, k) = ak1; at(U2, k) = bk1; at(ML, k) = m;
-        at(SW, k) = 1.0;
-        const double n0 = r1 - m * ak1;
-        const double n1 = r2 - m * bk1;
-        r0 = n0;
-        r1 = n1;
-        r2 = 0.0;
-      }
+      // one reciprocal for the multiplier and the stored pivot (unless that is tiny), and selected
+      // operands: as two branches, a warp whose threads differ computes both reciprocals
+      const bool sw = abs_bits(ck) > abs_bits(r0);
+      const double pv = sw ? ck : r0, a1 = sw ? ak1 : r1, a2 = sw ? bk1 : r2;
+      const double b0 = sw ? r0 : ck, b1 = sw ? r1 : ak1, b2 = sw ? r2 : bk1;
+      const double rr = FAST ? qk_rcp3(pv) : qk_rcp(pv);
+      const double m = abs_bits(pv) ? b0 * rr : 0.0;
+      at(U0, k) = abs_bits(pv) < abs_bits(tiny) ? pivot_rcp(pv, tiny) : rr;
+      at(U1, k) = a1; at(U2, k) = a2; at(ML, k) = m;
+      set_swap(k, sw);
+      r0 = b1 - m * a1;
+      r1 = b2 - m * a2;
+      r2 = 0.0;
     }
     at(U0, n - 1) = pivot_rcp(r0, tiny); at(U1, n - 1) = 0.0; at(U2, n - 1) = 0.0;
     // ---- start vector ----
+    double* zp = SM ? SW : Zt + jj;          // the iterate
+    auto z = [&](int i) -> double& { return zp[RS * i]; };
     // (its largest entry and, from the back substitutions, the iterates' are found on the way: a
     // pass of its own over the vector costs a memory latency per load batch)
     unsigned long long mxb = 0;
     int imx = 0;
     for (int i = 0; i < n; ++i) {
       const double v = rand_pm1(i, jj);
-      Zt[(size_t)jj + N * i] = v;
+      z(i) = v;
       mxb = max(mxb, abs_bits(v));
     }
     for (int it = 0; it < iters; ++it) {
-      // scale to unit inf-norm
+      // scale to unit inf-norm (FAST: not between the iterations, a factor of 2^54 each)
       const double mx = __longlong_as_double((long long)mxb);
       mxb = 0;
-      const double sc = mx > 0.0 ? 1.0 / mx : 1.0;
+      const double sc = !FAST && mx > 0.0 ? 1.0 / mx : 1.0;
       // forward: apply P and L^{-1}.  The loads of a batch of SB steps are issued before its
       // stores (they read entries the batch has not written yet), so the memory latency is paid
       // once per batch instead of once per step of the dependency chain.
-      double yk = Zt[jj] * sc;
+      double yk = z(0) * sc;
       int k = 0;
       for (; k + SB <= n - 1; k += SB) {
-        double zv[SB], mv[SB], sv[SB];
+        double zv[SB], mv[SB];
+        bool sv[SB];
 #pragma unroll
         for (int u = 0; u < SB; ++u) {
-          zv[u] = Zt[(size_t)jj + N * (k + 1 + u)];
+          zv[u] = z(k + 1 + u);
           mv[u] = at(ML, k + u);
-          sv[u] = at(SW, k + u);
+          sv[u] = swapped(k + u);
         }
 #pragma unroll
         for (int u = 0; u < SB; ++u) {
-          double yk1 = zv[u] * sc;
-          if (sv[u] != 0.0) {
-            const double t = yk;
-            yk = yk1;
-            yk1 = t - mv[u] * yk;
-          } else {
-            yk1 = yk1 - mv[u] * yk;
-          }
-          Zt[(size_t)jj + N * (k + u)] = yk;
-          yk = yk1;
+          z(k + u) = fwd_step(yk, FAST ? zv[u] : __dmul_rn(zv[u], sc), mv[u], sv[u]);
         }
       }
       for (; k < n - 1; ++k) {
-        double yk1 = Zt[(size_t)jj + N * (k + 1)] * sc;
-        const double m = at(ML, k);
-        if (at(SW, k) != 0.0) {
-          const double t = yk;
-          yk = yk1;
-          yk1 = t - m * yk;
-        } else {
-          yk1 = yk1 - m * yk;
-        }
-        Zt[(size_t)jj + N * k] = yk;
-        yk = yk1;
+        z(k) = fwd_step(yk, FAST ? z(k + 1) : __dmul_rn(z(k + 1), sc), at(ML, k), swapped(k));
       }
-      Zt[(size_t)jj + N * (n - 1)] = yk;
+      z(n - 1) = yk;
       // back substitution with U (pivots stored as reciprocals), batched the same way
       double y1 = 0.0, y2 = 0.0;
       k = n - 1;
@@ -1621,7 +1632,7 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
         double zv[SB], a0[SB], a1[SB], a2[SB];
 #pragma unroll
         for (int u = 0; u < SB; ++u) {
-          zv[u] = Zt[(size_t)jj + N * (k - u)];
+          zv[u] = z(k - u);
           a0[u] = at(U0, k - u);
           a1[u] = at(U1, k - u);
           a2[u] = at(U2, k - u);
@@ -1629,15 +1640,15 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
 #pragma unroll
         for (int u = 0; u < SB; ++u) {
           const double yv = (zv[u] - a1[u] * y1 - a2[u] * y2) * a0[u];
-          Zt[(size_t)jj + N * (k - u)] = yv;
+          z(k - u) = yv;
           if (abs_bits(yv) >= mxb) { mxb = abs_bits(yv); imx = k - u; }  // (the first of equal ones)
           y2 = y1;
           y1 = yv;
         }
       }
       for (; k >= 0; --k) {
-        const double yv = (Zt[(size_t)jj + N * k] - at(U1, k) * y1 - at(U2, k) * y2) * at(U0, k);
-        Zt[(size_t)jj + N * k] = yv;
+        const double yv = (z(k) - at(U1, k) * y1 - at(U2, k) * y2) * at(U0, k);
+        z(k) = yv;
         if (abs_bits(yv) >= mxb) { mxb = abs_bits(yv); imx = k; }
         y2 = y1;
         y1 = yv;
@@ -1645,12 +1656,12 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
       // MGS against earlier members of the cluster
       for (int kk = j; kk < jj; ++kk) {
         double dot = 0.0;
-        for (int i = 0; i < n; ++i) dot += Zt[(size_t)jj + N * i] * Zt[(size_t)kk + N * i];
+        for (int i = 0; i < n; ++i) dot += z(i) * Zt[(size_t)kk + N * i];
         mxb = 0;
         imx = 0;
         for (int i = 0; i < n; ++i) {
-          const double v = Zt[(size_t)jj + N * i] - dot * Zt[(size_t)kk + N * i];
-          Zt[(size_t)jj + N * i] = v;
+          const double v = z(i) - dot * Zt[(size_t)kk + N * i];
+          z(i) = v;
           if (abs_bits(v) > mxb) { mxb = abs_bits(v); imx = i; }
         }
       }
@@ -1658,33 +1669,62 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
     // normalise (2-norm), largest component positive
     double s2 = 0.0;
     const double mx = __longlong_as_double((long long)mxb);
-    const double sc0 = mx > 0.0 ? 1.0 / mx : 1.0;
+    const double sc0 = !FAST && mx > 0.0 ? 1.0 / mx : 1.0;
     int i = 0;
     for (; i + SB <= n; i += SB) {
       double v[SB];
 #pragma unroll
-      for (int u = 0; u < SB; ++u) v[u] = Zt[(size_t)jj + N * (i + u)];
+      for (int u = 0; u < SB; ++u) v[u] = z(i + u);
 #pragma unroll
       for (int u = 0; u < SB; ++u) {
-        const double t = v[u] * sc0;
+        const double t = FAST ? v[u] : v[u] * sc0;
         s2 += t * t;
       }
     }
     for (; i < n; ++i) {
-      const double t = Zt[(size_t)jj + N * i] * sc0;
+      const double t = FAST ? z(i) : z(i) * sc0;
       s2 += t * t;
     }
     double sc = sc0 / sqrt(s2);
-    if (Zt[(size_t)jj + N * imx] < 0.0) sc = -sc;
+    if (z(imx) < 0.0) sc = -sc;
     for (i = 0; i + SB <= n; i += SB) {
       double v[SB];
 #pragma unroll
-      for (int u = 0; u < SB; ++u) v[u] = Zt[(size_t)jj + N * (i + u)];
+      for (int u = 0; u < SB; ++u) v[u] = z(i + u);
 #pragma unroll
       for (int u = 0; u < SB; ++u) Zt[(size_t)jj + N * (i + u)] = v[u] * sc;
     }
-    for (; i < n; ++i) Zt[(size_t)jj + N * i] *= sc;
+    for (; i < n; ++i) Zt[(size_t)jj + N * i] = z(i) * sc;
   }
+}
+
+// One warp per CTA either way, so that the warps go to as many SMs as there are.  In shared memory
+// while all n vectors are resident at once (n <= 900 or so on 152 SMs), as few threads per CTA as fill
+// the SMs; a second round of CTAs costs more than the waits for global memory (eigenvector stage, n =
+// 800: 1.82 ms in shared, 1.92 in global memory; n = 1000: 3.58 against 2.51).
+template <bool FAST>
+int launch_stein(qk_ctx* ctx, int n, const double* d, const double* e, const double* w,
+                 const double* prep, double* Zt, int iters) {
+  const size_t vec = (size_t)n * STEIN_ROW, cap = 226 * 1024;
+  const int per_sm = (int)(cap / vec);                     // vectors resident on an SM
+  if ((long long)per_sm * ctx->num_sms >= n && n <= 32 * ctx->num_sms) {
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+      attr_err = cudaFuncSetAttribute(k_stein<true, FAST>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    });
+    QK_CK(attr_err);
+    const int L = (n + ctx->num_sms - 1) / ctx->num_sms;
+    k_stein<true, FAST><<<(n + L - 1) / L, 32, vec * L, ctx->stream>>>(
+        n, d, e, w, prep, nullptr, Zt, ctx->d_status, iters, L);
+  } else {
+    double* W = nullptr;
+    QK_TRY(qk_wst(ctx, W_EIGWORK, 5 * (size_t)n * n, &W));
+    k_stein<false, FAST><<<(n + 31) / 32, 32, 0, ctx->stream>>>(n, d, e, w, prep, W, Zt,
+                                                                ctx->d_status, iters, 32);
+  }
+  return QK_OK;
 }
 
 // Forward compact-WY T factors (upper triangular, dlarft 'F','C') of every reflector block:
@@ -2166,16 +2206,12 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
   if (tm) qk_toc(ctx, T_BISECT);
   if (!want_vectors) return QK_OK;
   // ---- 3. eigenvectors of T by inverse iteration ----
-  double* Wst = nullptr;
-  QK_TRY(qk_wst(ctx, W_EIGWORK, 5 * N * N, &Wst));
   if (tm) qk_tic(ctx, T_STEIN);
-  // one warp per block: the threads' sweeps are latency-bound chains, so the warps go to as
-  // many SMs as there are (each with its own load/store and FP64 units)
   // iterations from the random start: three in FP64 (as dstein's convergence plus its two
   // extra steps), two in the mixed tier, whose eigenvalues come from the double-float bisection
   // and whose vectors feed FP32 products
-  k_stein<<<(n + 31) / 32, 32, 0, ctx->stream>>>(n, d, e, w, prep, Wst, Zt, ctx->d_status,
-                                                 tri_df ? 2 : 3);
+  if (tri_df) QK_TRY(launch_stein<false>(ctx, n, d, e, w, prep, Zt, 2));
+  else QK_TRY(launch_stein<true>(ctx, n, d, e, w, prep, Zt, 3));
   QK_LAUNCHED();
   k_tri_unscale<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, prep, w);
   QK_LAUNCHED();
