@@ -25,9 +25,12 @@
 //   u' = unit vector of x_(j+1..) + sign(alpha) |x| e_1, e_j = -sign(alpha) |x|   (dlarfg's choice)
 //   rows r > j: A_r -= 2 (u_r w + w_r u), p'_r = A_r u', broadcast p'_r and A_(r,j+1).
 // Measured (one GB300), eigenvalues alone (this kernel plus the bisection), before -> now: n = 48
-// 0.77 -> 0.42 ms, 128 1.84 -> 0.87, 256 3.55 -> 1.60, 400 5.55 -> 2.61, 600 8.43 -> 4.63.  A column
-// takes ~7.6k cycles at n = 400: the vector work ~3.1k (block sums, the reflector's scalars), the
-// rows ~2.9k, the cluster barrier with its wait ~1.7k.
+// 0.77 -> 0.30 ms, 128 1.84 -> 0.59, 256 3.55 -> 1.2, 400 5.55 -> 2.04, 600 8.43 -> 3.9.  Cycles of a
+// column at n = 400 (48): K 0.8k (0.75k), w and x 0.4k (0.1k), the norm's sums and the reflector 1.5k
+// (1.7k), u' 0.3k (0.1k), the rows 2.6k (2.0k), the cluster barrier with its wait 1.7k (1.1k), of
+// which the release of the remote stores is about 0.9k.  The O(n) loops are kept rolled: unrolled by
+// the compiler they cost 2 to 3 % (a thread runs them once or twice).  Tried and not kept: K from the
+// row pass by remote stores (K 0.55k, but the rows 0.6k more), three and four rows of a warp at a time.
 #include <cooperative_groups.h>
 #include <mutex>
 #include "qk_internal.cuh"
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
   __shared__ int s_small;
   __shared__ unsigned redm[VW];
   __shared__ double cmax[MAX_CL], cfro[MAX_CL];
-  __shared__ Scal sc;
+  __shared__ Scal scb[2];                          // by column parity
 
   // ---- ||A||_inf and ||A||_F^2: a warp per own row, lanes along the row (the lower triangle is
   // referenced) ----
@@ -355,10 +358,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
     const long long* X = Xb + par * n;
     const Fx* U = Ub + par * n;
     Fx* Un = Ub + (par ^ 1) * n;
+    Scal& sc = scb[par];
     if (tid < VT) {
       // ---- K = u^T p ----
       long long Ksum = 0;
       if (j > 0) {
+#pragma unroll 1
         for (int i = j + tid; i < n; i += VT) Ksum += fx_mul(fx_split(P[i]), U[i]);
         Ksum = warp_sum64(Ksum);
         if (lane == 0) redk[warp] = Ksum;
@@ -370,6 +375,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
       const Fx uj = U[j];
       const Fx wj = fx_split(P[j] - fx_mul(K, uj) + 1);
       long long s0 = 0, s1 = 0;
+#pragma unroll 1
       for (int i = j + tid; i < n; i += VT) {
         const Fx u = U[i];
         const Fx w = fx_split(P[i] - fx_mul(K, u) + 1);
@@ -403,6 +409,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
         vec_bar();
         if (!s_small) break;
         unsigned long long mx = 0;            // leading bits of max |x|
+#pragma unroll 1
         for (int i = j + 1 + tid; i < n; i += VT) {
           const long long x = Xc[i];
           const unsigned long long ax = (unsigned long long)(x < 0 ? -x : x);
@@ -416,6 +423,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
         xs = m ? 55 - (int)m : -1;            // max |x| << xs in [2^54, 2^55); -1: x = 0
         s0 = s1 = 0;
         if (xs > 0)
+#pragma unroll 1
           for (int i = j + 1 + tid; i < n; i += VT) {
             const long long x = Xc[i] << xs;
             const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
@@ -435,6 +443,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
         const Fx f = fx_split(sc.f);
         const int sh = sc.sh;
         const bool zero = sc.zero != 0;
+#pragma unroll 1
         for (int i = j + 1 + tid; i < n; i += VT) {
           long long u = 0;
           if (!zero) u = i == j + 1 ? sc.u1 : fx_mul(fx_split(Xc[i] << sh), f);
@@ -452,25 +461,38 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_fx(const __grid_constant__ F
       // (the first own row beyond column j + 1)
       if (lr0 * CL + rank <= j + 1) ++lr0;
     } else {
-      // ---- output warp ----
-      const Scal t = sc;
-      if (rank == 0 && lane == 0) {
-        a.d[j] = fx_to_double(t.dj, E + 1 - 62);
-        if (j < n - 1) {
-          a.e[j] = t.zero ? fx_to_double(t.alpha, E + 1 - 62)
-                          : fx_to_double(t.neg ? t.nx : -t.nx, E + 1 - 62 - t.sh);
+      // ---- output warp: it arrives first and writes while the others go on; what it reads stays
+      // until the second column from here ----
+      cl.barrier_arrive();
+      const Scal& t = scb[par];
+      if (rank == 0 && lane < 3) {
+        // lane 0: d, lane 1: e, lane 2: tau
+        long long v = t.dj;
+        int k = E + 1 - 62;
+        double* out = a.d + j;
+        if (lane == 1) {
+          v = t.zero ? t.alpha : (t.neg ? t.nx : -t.nx);
+          if (!t.zero) k -= t.sh;
+          out = a.e + j;
+        } else if (lane == 2) {
           const Fx u1 = fx_split(t.u1);
-          a.tau[j] = fx_to_double(fx_mul(u1, u1), 1 - 62);
+          v = fx_mul(u1, u1);
+          k = 1 - 62;
+          out = a.tau + j;
         }
+        const double x = fx_to_double(v, k);
+        if (lane == 0 || j < n - 1) *out = x;
       }
       if (j < n - 1) {
         // v = u / u1 (unit first entry): u 2 g, with the sign of u1
         const Fx g = fx_split(t.u1 < 0 ? -t.g : t.g);
+#pragma unroll 1
         for (int i = j + 1 + 32 * rank + lane; i < n; i += 32 * CL)
           a.V[i + a.ldv * j] = i == j + 1 ? 1.0 : fx_to_double(fx_mul(Un[i], g), 1 - 62);
       }
     }
-    cl.sync();
+    if (warp < NWARPS) cl.barrier_arrive();
+    cl.barrier_wait();
   }
 }
 
@@ -640,6 +662,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     const double qnan = __longlong_as_double(0x7FF8000000000000ll);
     for (int i = gthread; i < n; i += totthreads) a.d[i] = a.e[i] = a.tau[i] = qnan;
     for (int j = rank; j < n - 1; j += G)
+#pragma unroll 1
       for (int i = j + 1 + tid; i < n; i += GT) a.V[i + a.ldv * j] = qnan;
     return;
   }
@@ -659,6 +682,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     const long long* p = pb + (size_t)(j % 3) * n;
     long long* pnext = pb + (size_t)((j + 1) % 3) * n;
     long long* pz = pb + (size_t)((j + 2) % 3) * n;
+#pragma unroll 1
     for (int i = gthread; i < n; i += totthreads) __stcg(pz + i, 0ll);
     // ---- vector work (every CTA) ----
     long long Ks = 0;
@@ -688,6 +712,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     const Fx K = fx_split(Ks), uj = s_uj;
     const Fx wj = fx_split(s_pj - fx_mul(K, uj) + 1);
     long long s0 = 0, s1 = 0;
+#pragma unroll 1
     for (int i = j + tid; i < n; i += GT) {
       const FxPair k = UW[i];
       const long long pi = (long long)(((unsigned long long)(unsigned)k.w.l << 32) | (unsigned)k.w.h);
@@ -725,6 +750,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
       __syncthreads();
       if (!s_small) break;
       unsigned long long mx = 0;
+#pragma unroll 1
       for (int i = j + 1 + tid; i < n; i += GT) {
         const long long x = Xc[i];
         const unsigned long long ax = (unsigned long long)(x < 0 ? -x : x);
@@ -738,6 +764,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
       xs = mb ? a.xbits - (int)mb : -1;     // max |x| << xs below 2^xbits
       s0 = s1 = 0;
       if (xs > 0)
+#pragma unroll 1
         for (int i = j + 1 + tid; i < n; i += GT) {
           const long long x = Xc[i] << xs;
           const int lo = (int)(unsigned)x, h = (int)(x >> 32) + (int)((unsigned)lo >> 31);
@@ -755,6 +782,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     const Scal t = sc;
     {
       const Fx fx = fx_split(t.f);
+#pragma unroll 1
       for (int i = j + 1 + tid; i < n; i += GT) {
         long long u = fx_mul(fx_split(Xc[i] << t.sh), fx);
         if (i == j + 1) u = t.u1;
@@ -841,6 +869,7 @@ __device__ __forceinline__ void tri_fx_grid_body(const qk_tri_fx_grid_args& a, c
     }
     if (warp == 1) {
       const Fx g = fx_split(sc.u1 < 0 ? -sc.g : sc.g);
+#pragma unroll 1
       for (int i = j + 1 + rank + G * lane; i < n; i += 32 * G)
         a.V[i + a.ldv * j] = i == j + 1 ? 1.0 : fx_to_double(fx_mul(Un[i], g), 1 - 62);
     }
