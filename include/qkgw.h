@@ -48,7 +48,7 @@ enum {
                               no SRG the pole sums of Sigma/dSigma (linearised stage and Newton)
                               take the terms with |w - e +- Om| >= 0.01 Ha in FP32 and the
                               near-pole terms in FP64; G0W0's EcRPA at eGW by frequency
-                              quadrature.  The Casida eigenvalues, the Newton update and DIIS stay
+                              quadrature with FP32 products (the FP64 form's keeps FP64 accuracy).  The Casida eigenvalues, the Newton update and DIIS stay
                               FP64. */
 };
 
@@ -337,7 +337,8 @@ int qk_RGW_phBSE_dev(qk_ctx* ctx, const qk_bse_params* prm, int nOrb, int nC, in
  *   route to ~1e-8 Ha.  A negative e_a - e_i gives NaN (as the Casida square roots do) and the
  *   QKD_NEG_AMB status.  *applied = 0 (EcRPA untouched) when it does not apply: a zero
  *   e_a - e_i, d_max/d_min > 60000, or a numerical rank of (ia|jb) above nS/3.  The mixed tier
- *   of qk_RG0W0 / qk_RG0W0_L_dev uses it for the EcRPA at the G0W0 energies.
+ *   of qk_RG0W0 / qk_RG0W0_L_dev uses it for the EcRPA at the G0W0 energies; the FP64 tier has its
+ *   own form there (more points, FP64 products), with the eigenvalue route's accuracy.
  * qk_gauss_legendre: the quadrature's nodes x (ascending) and weights w on [-1, 1], host only. */
 int qk_RPA_ecorr_quad_dev(qk_ctx* ctx, int nOrb, int nC, int nO, int nR, int naux,
                           const double* d_e, const double* d_ERI, const double* d_L,
@@ -396,8 +397,9 @@ int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOrb, int nC, 
  * No counterpart in the reference.  Runtime launch parameters of this library's kernels, tuned
  * per size bucket floor(log2(size)): "bf16x3_chunk" (k blocks per TMEM chunk of the BF16x3 GEMM,
  * size = K), "splitk_mult" (split-K target CTAs per SM of the DMMA GEMM, size = K),
- * "sigma_chunks" (m chunks of the pole sweeps per SM, size = nS), "sytrd_grid" (quarters of the
- * SMs in the cooperative tridiagonalisation, size = n), "dgemm_path" (1 DFMA, 2 DMMA; for
+ * "sigma_chunks" (how far the pole sweeps split their q range, 4 = to one CTA per SM and tile of
+ * orbitals, size = nS), "sytrd_grid" (quarters of the
+ * SMs in the cooperative tridiagonalisations, size = n), "dgemm_path" (1 DFMA, 2 DMMA; for
  * qk_dgemm_dev also 3, exact integer digit products on tcgen05 -- what the drivers use for FP64
  * products large enough -- whose error is relative to the largest elements of a row of op(A) and a
  * column of op(B); size = m n),
@@ -415,7 +417,8 @@ int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOrb, int nC, 
  * the Halley step from eGWlin, 1 the model's prediction everywhere, 2 the Halley step
  * everywhere; results are the reference start's in every case) and "dsyev_df" (1: qk_dsyev_dev
  * tridiagonalises in double-float arithmetic on the FP32 pipe, as the mixed tier's Casida solve
- * does; 0, the default, in FP64). */
+ * does; 2: in fixed point as the FP64-tier drivers do, which loses elements below 2^-62 of the
+ * matrix's norm; 0, the default, in FP64). */
 int qk_autotune(qk_ctx* ctx, int nOrb, int nS, int flags);
 int qk_tune_set(qk_ctx* ctx, const char* name, long long size, int value);
 int qk_tune_query(const qk_ctx* ctx, const char* name, long long size);

@@ -114,8 +114,8 @@ struct TriArgs {
   int use_smem;
 };
 
-// CTA group of a tridiagonalisation: the whole grid (k_sytrd; the sizes stay in special
-// registers) or a slice of it (k_sytrd_grouped; the sizes live in shared memory)
+// CTA group of a tridiagonalisation: the whole grid (k_sytrd, k_sytrd_df; the sizes stay in
+// special registers) or a slice of it (k_sytrd_df_grouped; the sizes live in shared memory)
 struct TriGridWhole {
   __device__ __forceinline__ int size() const { return (int)gridDim.x; }
   __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
@@ -126,13 +126,9 @@ struct TriGridSlice {
   __device__ __forceinline__ int rank() const { return *(const volatile int*)(s + 1); }
 };
 
-// The tridiagonalisation of one matrix by a group of co-resident CTAs.  With kFixed, every
-// rounded quantity is independent of the group size: ||A||_F is summed over fixed column chunks
-// and each tile's row partial sum is split into the exact accumulators on its own (not summed
-// over a warp's run of tiles, whose extent depends on the group size), so the result is the same
-// bits for any number of CTAs -- the grouped launch then sizes the groups freely.
-template <class Grp, bool kFixed>
-__device__ __forceinline__ void sytrd_body(const TriArgs a, const Grp grp) {
+// The FP64 tridiagonalisation of one matrix by the whole (cooperative) grid.
+__global__ void __launch_bounds__(TRI_THREADS) k_sytrd(const TriArgs a) {
+  const TriGridWhole grp{};
   extern __shared__ double sm[];
   __shared__ double s_pj, s_dj, s_alpha, s_sc[7], s_fro;
   __shared__ int s_g1;  // exponent of the first accumulator grid
@@ -158,7 +154,7 @@ __device__ __forceinline__ void sytrd_body(const TriArgs a, const Grp grp) {
 
   // ---- ||A||_F (bounds every p element's partial sums): fixed per-thread order, per-CTA slot,
   // then every CTA adds the slots in the same order, so all CTAs hold the same value ----
-  if (!kFixed) {
+  {
     double fs = 0.0;
     for (int c = grp.rank(); c < n; c += grp.size()) {
       const double* col = a.A + a.lda * c;
@@ -172,28 +168,6 @@ __device__ __forceinline__ void sytrd_body(const TriArgs a, const Grp grp) {
     if (tid == 0) {
       double t = 0.0;
       for (int b = 0; b < grp.size(); ++b) t += __ldcg(a.fslot + b);
-      s_fro = sqrt(t);
-    }
-    __syncthreads();
-  } else {
-    // chunks of 32 columns, one slot each (n <= 32768), summed in chunk order
-    const int nch = (n + 31) / 32;
-    for (int ch = grp.rank(); ch < nch; ch += grp.size()) {
-      double fs = 0.0;
-      const int c1 = 32 * ch + 32 < n ? 32 * ch + 32 : n;
-      for (int c = 32 * ch; c < c1; ++c) {
-        const double* col = a.A + a.lda * c;
-        for (int i = c + tid; i < n; i += nt) {
-          const double x = __ldcg(col + i);
-          fs = fma(i == c ? x : x + x, x, fs);
-        }
-      }
-      tri_block_sum(fs, ytile, nt, [&](double t) { __stcg(a.fslot + ch, t); });
-    }
-    if (!qk_grid_barrier(a.bar, grp.size(), epoch, a.status)) return;
-    if (tid == 0) {
-      double t = 0.0;
-      for (int b = 0; b < nch; ++b) t += __ldcg(a.fslot + b);
       s_fro = sqrt(t);
     }
     __syncthreads();
@@ -351,22 +325,13 @@ __device__ __forceinline__ void sytrd_body(const TriArgs a, const Grp grp) {
         int i = 0;
         bool rowok = false;
         double ri = 0.0, si = 0.0, rowacc = 0.0;
-        double rb1 = 0.0, rb2 = 0.0;  // kFixed: the row's tile sums, already split (exact)
         for (int it = it0; it < it1; ++it) {
           while (it >= off + 2 * bi + 2) {
             off += 2 * bi + 2;
             ++bi;
           }
           if (bi != cur) {
-            if (kFixed) {
-              if (cur >= 0 && wantp && rowok) {
-                atomicAdd(pnext + i, rb1);
-                atomicAdd(pnext2 + i, rb2);
-              }
-              rb1 = rb2 = 0.0;
-            } else if (cur >= 0 && wantp && rowok) {
-              tri_exact_add(pnext + i, pnext2 + i, rowacc, s_g1);
-            }
+            if (cur >= 0 && wantp && rowok) tri_exact_add(pnext + i, pnext2 + i, rowacc, s_g1);
             cur = bi;
             i = r0 + 32 * bi + lane;
             rowok = i < n;
@@ -413,25 +378,10 @@ __device__ __forceinline__ void sytrd_body(const TriArgs a, const Grp grp) {
             const int c = c0 + u;
             if (hh == 0 && c < n && c <= r0 + 32 * bi + 31)
               tri_exact_add(pnext + c, pnext2 + c, cs, s_g1);
-            if (kFixed) {
-              // this tile's row sum into the row's exact register accumulators
-              const int g1 = s_g1;
-              const double q1 = tri_trunc(rowacc, g1);
-              rb1 = __dadd_rn(rb1, q1);
-              rb2 = __dadd_rn(rb2, tri_trunc(__dsub_rn(rowacc, q1), g1 - 41));
-              rowacc = 0.0;
-            }
           }
           __syncwarp();
         }
-        if (kFixed) {
-          if (wantp && rowok) {
-            atomicAdd(pnext + i, rb1);
-            atomicAdd(pnext2 + i, rb2);
-          }
-        } else if (wantp && rowok) {
-          tri_exact_add(pnext + i, pnext2 + i, rowacc, s_g1);
-        }
+        if (wantp && rowok) tri_exact_add(pnext + i, pnext2 + i, rowacc, s_g1);
       }
     }
     if (!qk_grid_barrier(a.bar, grp.size(), epoch, a.status)) return;
@@ -442,10 +392,6 @@ __device__ __forceinline__ void sytrd_body(const TriArgs a, const Grp grp) {
     tau_k = tau1;
     scal_k = scal1;
   }
-}
-
-__global__ void __launch_bounds__(TRI_THREADS) k_sytrd(TriArgs a) {
-  sytrd_body<TriGridWhole, false>(a, TriGridWhole{});
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -644,7 +590,7 @@ __device__ __forceinline__ double df_f2d(float f) {
 // hi + lo as a double: exact (|lo| < ulp(hi), 48 bits in all), one FP64 addition
 __device__ __forceinline__ double df_to_double(float2 a) { return __dadd_rn(df_f2d(a.x), df_f2d(a.y)); }
 
-// The same factorisation as sytrd_body (the same fused rank-2 update and symmetric mat-vec over
+// The same factorisation as k_sytrd (the same fused rank-2 update and symmetric mat-vec over
 // the same tiles, the same reflector formulas and exact accumulators), with the matrix and the
 // vectors u_k, p~_k, u_{k+1} in double-float.  The lower triangle of A is converted in place
 // (float2 in each double's slot) after the Frobenius norm has been found, scaled by the power of
@@ -655,6 +601,9 @@ __device__ __forceinline__ double df_to_double(float2 a) { return __dadd_rn(df_f
 // outputs d, e, tau, the reflector scale factors and the unscaled reflectors are stored as
 // double-floats in the slots of their doubles, and k_tri_df_finish converts them afterwards (d and
 // e scaled back by 2^ex; the reflectors do not depend on the scaling).
+// kFixed (the grouped launch): every rounded quantity is independent of the group size -- ||A||_F is
+// summed over fixed column chunks and each tile's row sum is split into the exact accumulators on its
+// own -- so the result is the same bits for any number of CTAs and the groups are sized freely.
 template <class Grp, bool kFixed>
 __device__ __forceinline__ void sytrd_df_body(const TriArgs a, const Grp grp) {
   extern __shared__ double sm[];
@@ -743,7 +692,7 @@ __device__ __forceinline__ void sytrd_df_body(const TriArgs a, const Grp grp) {
         __stcg(pz2 + i, 0.0);
       }
     }
-    // ---- small phase (redundant in every CTA), as in sytrd_body, on the FP32 pipe ----
+    // ---- small phase (redundant in every CTA), as in k_sytrd, on the FP32 pipe ----
     const int j = k + 1;
     float2 tau1, scal1;
     {
@@ -1076,20 +1025,7 @@ struct TriGroup {
   TriArgs req[TRI_GROUP_MAX];
 };
 
-__global__ void __launch_bounds__(TRI_THREADS) k_sytrd_grouped(const __grid_constant__ TriGroup g) {
-  __shared__ int s_grp[2];
-  int r = 0;
-  while (r + 1 < g.nreq && (int)blockIdx.x >= g.cta0[r + 1]) ++r;
-  if ((int)blockIdx.x >= g.cta0[g.nreq]) return;
-  if (threadIdx.x == 0) {
-    s_grp[0] = g.cta0[r + 1] - g.cta0[r];
-    s_grp[1] = (int)blockIdx.x - g.cta0[r];
-  }
-  __syncthreads();
-  sytrd_body<TriGridSlice, true>(g.req[r], TriGridSlice{s_grp});
-}
-
-// the same for double-float requests (the mixed tier), DF_THREADS per CTA
+// double-float requests (the mixed tier), DF_THREADS per CTA
 constexpr int DF_THREADS = 512;
 __global__ void __launch_bounds__(DF_THREADS)
     k_sytrd_df_grouped(const __grid_constant__ TriGroup g) {
@@ -1860,7 +1796,7 @@ namespace {
 
 // CTAs per request: proportional to the n^3 work, at least one, at most what the matrix can use
 // (one 32 x 128 trailing block per CTA, as in the single-matrix launch), all within one CTA per
-// SM.  The grouped kernel's arithmetic does not depend on a group's size (sytrd_body<., true>),
+// SM.  The grouped kernels' arithmetic does not depend on a group's size (sytrd_df_body<., true>),
 // so this split, which changes with the launch's other matrices, never changes a result.
 void tri_split(const std::vector<qk_tri_service::Req>& rq, int sms, int* cta0) {
   const int R = (int)rq.size();
@@ -1902,7 +1838,7 @@ void tri_split(const std::vector<qk_tri_service::Req>& rq, int sms, int* cta0) {
   for (int r = 0; r < R; ++r) cta0[r + 1] = cta0[r] + g[r];
 }
 
-// one launch for the pending requests of one arithmetic (FP64 and double-float cooperative)
+// one launch for the pending requests of one kernel
 int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& rq, int mode) {
   const int R = (int)rq.size();
   if (R == 0) return QK_OK;
@@ -1924,11 +1860,11 @@ int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& 
     sv->matrices += R;
     return QK_OK;
   }
-  const bool df = mode == TRI_DF;
+  if (mode != TRI_DF) return QK_ERR_ARG;  // (FP64 requests do not come here)
   TriGroup g;
   g.nreq = R;
   size_t smem = 0;
-  const int nt = df ? DF_THREADS : TRI_THREADS;
+  const int nt = DF_THREADS;
   for (int r = 0; r < R; ++r) {
     g.req[r] = rq[r].ta;
     const size_t need = (size_t)(nt / 32) * TRI_TC * TRI_TLD * 8 + 3 * (size_t)g.req[r].n * 8;
@@ -1945,14 +1881,14 @@ int tri_launch_part(qk_tri_service* sv, const std::vector<qk_tri_service::Req>& 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, df ? k_sytrd_df_grouped : k_sytrd_grouped, g) != cudaSuccess)
+  if (cudaLaunchKernelEx(&cfg, k_sytrd_df_grouped, g) != cudaSuccess)
     return QK_ERR_CUDA;
   sv->launches++;
   sv->matrices += R;
   return QK_OK;
 }
 
-// launches for all pending requests (called with the lock held): one per arithmetic present, one
+// launches for all pending requests (called with the lock held): one per kernel needed, one
 // after the other on the service stream, each over all SMs
 void tri_launch_locked(qk_tri_service* sv) {
   int st = QK_OK;
@@ -2003,8 +1939,6 @@ qk_tri_service* qk_tri_service_new(qk_ctx* parent, int n_workers) {
   }
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncSetAttribute(k_sytrd_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TRI_SMEM_MAX);
     cudaFuncSetAttribute(k_sytrd_df_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          TRI_SMEM_MAX);
   });
@@ -2147,7 +2081,7 @@ int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, in
     ta.bar = ctx->d_bar;
     ta.status = ctx->d_status;
     ta.use_smem = use_smem;
-    if (ctx->tri_service && use_smem && !ctx->capturing) {
+    if (tri_df && ctx->tri_service && use_smem && !ctx->capturing) {
       // batch worker: the matrix joins the other workers' in one grouped launch
       QK_TRY(tri_submit(ctx->tri_service, ctx, ta));
     } else {

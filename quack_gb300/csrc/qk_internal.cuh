@@ -227,12 +227,12 @@ int qk_bse_dev(qk_ctx* ctx, int TDA_W, int TDA, int singlet, int triplet, int ex
 
 // dense symmetric eigensolver pieces.  backtransform: 0 = leave Zt as the eigenvectors of the
 // tridiagonal matrix, 1 = back-transform in FP64, 2 = back-transform with FP32 products.
-// tri_df: tridiagonalise in double-float arithmetic on the FP32 pipe (the mixed tier; the
-// tridiagonal matrix, reflectors, eigenvalues and eigenvectors stay FP64); the lower triangle of
-// A is overwritten either way.
+// tri (below): in double-float arithmetic on the FP32 pipe for the mixed tier (the tridiagonal matrix,
+// reflectors, eigenvalues and eigenvectors stay FP64); the lower triangle of A is overwritten either way.
 // Grouped tridiagonalisation service of the batched driver: workers' tridiagonalisations are
-// collected until every active worker has submitted one (or finished), then run as ONE
-// cooperative launch of k_sytrd_grouped with a CTA group per matrix.
+// collected until every active worker has submitted one (or finished), then run as one launch per
+// kernel they need (k_tri_fx with a cluster per matrix, k_tri_fx_grid_grouped and k_sytrd_df_grouped
+// with a CTA group per matrix).
 qk_tri_service* qk_tri_service_new(qk_ctx* parent, int n_workers);
 void qk_tri_service_worker_done(qk_tri_service* svc);
 void qk_tri_service_free(qk_tri_service* svc);
