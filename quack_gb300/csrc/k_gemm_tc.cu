@@ -75,7 +75,7 @@ struct Operand {           // op(A) as rows x K, or op(B)^T as rows x K
   uint8_t* P;              // digit planes: [batch][row block][k block][digit][rb rows][64 B]
   unsigned* info;          // per row: high word of max |x| (exponent; Inf and NaN codes)
   unsigned* part;          // partial maxima [batch][k slab][row] (slabs > 0)
-  int slabs;               // 0: the slicing kernel scans its rows itself (K <= SELF_K)
+  int slabs;               // 0: the slicing kernel finds the maxima itself (K <= SELF_K)
 };
 
 struct TcGemm {
@@ -155,12 +155,18 @@ __device__ __forceinline__ unsigned long long digits_of(double x, int exmax) {
   return q + 0x8080808080808080ull;
 }
 
-// Digit planes of 32 rows x 32 k per block of 128 threads: the doubles are staged in shared memory,
-// then a thread takes 8 consecutive k of one row and writes one 16-byte piece per plane (a warp
-// writes 512 contiguous bytes).  Memory-bound by design: 8 bytes read, 16 written per element.
+// Digit planes of 32 rows per block of 128 threads: the doubles are staged in shared memory, then a
+// thread takes 8 consecutive k of one row and writes one 16-byte piece per plane (a warp writes 512
+// contiguous bytes).  Memory-bound by design: 8 bytes read, 16 written per element.
+// SELF (K <= SELF_K): a block takes all k of its rows and finds their maxima on the way (with a block
+// per 32 k and a scan of the rows in each, rows beyond L2's reach were read once more per block: the
+// AO to MO transformation of 96 functions, 6.15 -> 5.56 ms).
+// Otherwise a block takes 32 k and the maxima come from k_tc_rowmax.
+template <bool SELF>
 __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, int kblks,
                                                   int a_blocks) {
-  __shared__ double t[32][33];
+  constexpr int KBS = SELF ? SELF_K / KB : 1;            // k blocks of a CTA, at most
+  __shared__ double t[KBS][32][33];
   __shared__ unsigned smax[4][32];
   int bid = blockIdx.x;
   const bool isA = bid < a_blocks;
@@ -170,85 +176,88 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
   const int strips = o.row_blocks * (o.rb / 32);
   const int strip = bid % strips;
   bid /= strips;
-  const int kb = bid % kblks, bt = bid / kblks;
-  const int r0 = strip * 32, k0 = kb * KB;
+  const int kb0 = SELF ? 0 : bid % kblks, bt = SELF ? bid : bid / kblks;
+  const int nkb = SELF ? kblks : 1;
+  const int r0 = strip * 32;
   const double* __restrict__ X = o.X + (long long)bt * o.stride;
   const double* sc = o.kscale ? o.kscale + (long long)bt * o.sk : nullptr;
   const size_t rows_pad = (size_t)o.row_blocks * o.rb;
-  double v[8];
-  if (o.trans) {
-    const int k = k0 + tx;
+  unsigned m[8] = {};                                    // trans: of rows ty + 4 i; else m[0]: row tx
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = r0 + ty + 4 * i;
-      v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[k + o.ld * r], k) : 0.0;
-    }
+  for (int q = 0; q < KBS; ++q) {
+    if (q >= nkb) break;
+    const int k0 = (kb0 + q) * KB;
+    double v[8];
+    if (o.trans) {
+      const int k = k0 + tx;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t[ty + 4 * i][tx] = v[i];
-  } else {
-    const int r = r0 + tx;
+      for (int i = 0; i < 8; ++i) {
+        const int r = r0 + ty + 4 * i;
+        v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[k + o.ld * r], k) : 0.0;
+      }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int k = k0 + ty + 4 * i;
-      v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[r + o.ld * k], k) : 0.0;
-    }
+      for (int i = 0; i < 8; ++i) {
+        t[q][ty + 4 * i][tx] = v[i];
+        if (SELF) m[i] = max(m[i], abs_hi(v[i]));
+      }
+    } else {
+      const int r = r0 + tx;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t[tx][ty + 4 * i] = v[i];
-  }
-  // the rows' maxima: from the partial ones, or by a scan of the whole (short) rows
-  if (o.slabs > 0 || !o.trans) {
-    unsigned m = 0;
-    if (r0 + tx < o.rows) {
-      if (o.slabs > 0) {
-        for (int i = ty; i < o.slabs; i += 4)
-          m = max(m, o.part[((size_t)bt * o.slabs + i) * rows_pad + r0 + tx]);
-      } else {
-#pragma unroll 8
-        for (int k = ty; k < K; k += 4) m = max(m, abs_hi(at_k(o, sc, X[r0 + tx + o.ld * k], k)));
+      for (int i = 0; i < 8; ++i) {
+        const int k = k0 + ty + 4 * i;
+        v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[r + o.ld * k], k) : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        t[q][tx][ty + 4 * i] = v[i];
+        if (SELF) m[0] = max(m[0], abs_hi(v[i]));
       }
     }
-    smax[ty][tx] = m;
-  } else {
+  }
+  // the rows' maxima
+  if (SELF && o.trans) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int r = r0 + ty + 4 * i;
-      unsigned m = 0;
-      if (r < o.rows)
-#pragma unroll 4
-        for (int k = tx; k < K; k += 32) m = max(m, abs_hi(at_k(o, sc, X[k + o.ld * r], k)));
-      m = __reduce_max_sync(0xffffffffu, m);
-      if (tx < 4) smax[tx][ty + 4 * i] = m;
+      const unsigned mr = __reduce_max_sync(0xffffffffu, m[i]);
+      if (tx < 4) smax[tx][ty + 4 * i] = mr;
     }
+  } else {
+    if (!SELF && r0 + tx < o.rows)
+      for (int i = ty; i < o.slabs; i += 4)
+        m[0] = max(m[0], o.part[((size_t)bt * o.slabs + i) * rows_pad + r0 + tx]);
+    smax[ty][tx] = m[0];
   }
   __syncthreads();
   const int rl = threadIdx.x >> 2, c = threadIdx.x & 3;  // row, 16-byte piece (8 k)
   const int r = r0 + rl;
   const unsigned info = max(max(smax[0][rl], smax[1][rl]), max(smax[2][rl], smax[3][rl]));
-  if (kb == 0 && c == 0) o.info[bt * rows_pad + r] = info;
+  if (kb0 == 0 && c == 0) o.info[bt * rows_pad + r] = info;
   const int exmax = (int)(info >> 20);
   const bool ok = info < HI_INF;
-  unsigned long long d[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) d[i] = digits_of(ok ? t[rl][c * 8 + i] : 0.0, ok ? exmax : 1);
   const int rb = r / o.rb, rr = r - rb * o.rb;
   const size_t plane = (size_t)o.rb * 64;
-  uint8_t* base = o.P + ((((size_t)bt * o.row_blocks + rb) * kblks + kb) * NS) * plane +
+  uint8_t* base = o.P + ((((size_t)bt * o.row_blocks + rb) * kblks + kb0) * NS) * plane +
                   (size_t)rr * 64 + ((c ^ ((rr >> 1) & 3)) << 4);
+  for (int q = 0; q < nkb; ++q, base += NS * plane) {
+    unsigned long long d[8];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    uint32_t w[4];
+    for (int i = 0; i < 8; ++i) d[i] = digits_of(ok ? t[q][rl][c * 8 + i] : 0.0, ok ? exmax : 1);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      // byte -> float without a conversion instruction: 2^23 + byte, minus 2^23 + 128; the upper
-      // half of the float is the BF16 value (digits have at most 8 significant bits)
-      const unsigned w0 = s < 4 ? (unsigned)(d[2 * i] >> 32) : (unsigned)d[2 * i];
-      const unsigned w1 = s < 4 ? (unsigned)(d[2 * i + 1] >> 32) : (unsigned)d[2 * i + 1];
-      const unsigned sel = 0x7650u | (unsigned)(3 - (s & 3));
-      const float f0 = __uint_as_float(__byte_perm(w0, 0x4B000000u, sel)) - 8388736.0f;
-      const float f1 = __uint_as_float(__byte_perm(w1, 0x4B000000u, sel)) - 8388736.0f;
-      w[i] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632u);
+    for (int s = 0; s < NS; ++s) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // byte -> float without a conversion instruction: 2^23 + byte, minus 2^23 + 128; the upper
+        // half of the float is the BF16 value (digits have at most 8 significant bits)
+        const unsigned w0 = s < 4 ? (unsigned)(d[2 * i] >> 32) : (unsigned)d[2 * i];
+        const unsigned w1 = s < 4 ? (unsigned)(d[2 * i + 1] >> 32) : (unsigned)d[2 * i + 1];
+        const unsigned sel = 0x7650u | (unsigned)(3 - (s & 3));
+        const float f0 = __uint_as_float(__byte_perm(w0, 0x4B000000u, sel)) - 8388736.0f;
+        const float f1 = __uint_as_float(__byte_perm(w1, 0x4B000000u, sel)) - 8388736.0f;
+        w[i] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632u);
+      }
+      *(uint4*)(base + s * plane) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    *(uint4*)(base + s * plane) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -678,9 +687,11 @@ int tc_panel(qk_ctx* ctx, TcGemm g) {
     k_tc_rowmax<<<ab + bb, 256, 0, ctx->stream>>>(g.a, g.b, g.K, ab);
     QK_LAUNCHED();
   }
-  const int sa = g.a.row_blocks * (TM / 32) * g.kblks * g.a.batch;
-  const int sb = g.b.row_blocks * (TN / 32) * g.kblks * g.b.batch;
-  k_tc_slice<<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
+  const int per = g.K <= SELF_K ? 1 : g.kblks;             // blocks of k per strip of 32 rows
+  const int sa = g.a.row_blocks * (TM / 32) * per * g.a.batch;
+  const int sb = g.b.row_blocks * (TN / 32) * per * g.b.batch;
+  if (g.K <= SELF_K) k_tc_slice<true><<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
+  else k_tc_slice<false><<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
   QK_LAUNCHED();
   // few tiles and a long k: split k at chunk boundaries; the rounds of the persistent grid times a
   // slice's chunks (plus half a chunk for the epilogue) decide
