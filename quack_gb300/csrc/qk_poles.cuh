@@ -29,6 +29,17 @@ constexpr int PT = 8;      // orbitals per tile
 constexpr int WARPS = 8;   // warps split the q of a CTA's range
 enum { KIND_ETA0 = 0, KIND_ETA = 1, KIND_SRG = 2 };
 
+// 1/x as qk_rcp3, with the range check on the high word alone ([2^-996, 2^996) here; with both words it
+// cost 10 % of the sweep)
+__device__ __forceinline__ double rcp3(double x) {
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if (h - 0x01B00000u >= 0x7E300000u - 0x01B00000u) return 1.0 / x;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = __fma_rn(-x, r, 1.0);
+  return __fma_rn(r, __fma_rn(e, e, e), r);
+}
+
 // one term: s += x^2 g(eps), d -= x^2 g'(eps)
 //   eta: c0 = eta^2, c1 = -2 eta^2.   SRG: c1 = -2 flow, hthr = high word of sqrt(19 / flow)
 template <int KIND>
@@ -36,12 +47,12 @@ __device__ __forceinline__ void term(double x, double eps, double c0, double c1,
                                      double& s, double& d) {
   const double x2 = __dmul_rn(x, x);
   if (KIND == KIND_ETA) {
-    const double rr = qk_rcp3(__fma_rn(eps, eps, c0));
+    const double rr = rcp3(__fma_rn(eps, eps, c0));
     const double t = __dmul_rn(x2, rr);
     s = __fma_rn(t, eps, s);
     d = __fma_rn(t, __fma_rn(rr, c1, 1.0), d);
   } else {
-    const double ir = qk_rcp3(eps);
+    const double ir = rcp3(eps);
     double t = __dmul_rn(x2, ir);
     if (KIND == KIND_SRG) {
       if (((unsigned)__double2hiint(eps) & 0x7fffffffu) <= hthr)
