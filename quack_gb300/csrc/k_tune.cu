@@ -86,6 +86,7 @@ extern "C" {
 
 int qk_tune_set(qk_ctx* ctx, const char* name, long long size, int value) {
   if (!ctx || !name) return QK_ERR_ARG;
+  ctx->gen++;
   // context-wide settings (size ignored)
   if (!strcmp(name, "newton_maxit")) {
     if (value < 1 || value > 4096) return QK_ERR_ARG;
@@ -134,6 +135,7 @@ int qk_tune_query(const qk_ctx* ctx, const char* name, long long size) {
 
 int qk_autotune(qk_ctx* ctx, int N, int nS, int flags) {
   if (!ctx || N <= 0 || nS <= 0) return QK_ERR_ARG;
+  ctx->gen++;
   (void)flags;
   cudaSetDevice(ctx->device);
   const long long N2 = (long long)N * N;
@@ -288,6 +290,7 @@ int qk_tune_save(const qk_ctx* ctx, const char* path) {
 
 int qk_tune_load(qk_ctx* ctx, const char* path) {
   if (!ctx || !path) return QK_ERR_ARG;
+  ctx->gen++;
   FILE* f = fopen(path, "r");
   if (!f) return QK_ERR_ARG;
   std::string txt;

@@ -531,14 +531,18 @@ int evgw_cycle(qk_ctx* ctx, const qk_gw_params* prm, const Dims& d, const EvBufs
   return QK_OK;
 }
 
-// Build (or reuse) a graph whose WHILE node replays evgw_cycle until the device flag drops.
+// Build (or reuse) a graph whose WHILE node replays evgw_cycle until the device flag drops.  The
+// captured launches hold the caller's pointers, the addresses of every workspace block they use and
+// launch parameters from the tuning table, so all of these are in the key (the last two by the
+// context's generation): a call in between that grows a block or changes a setting makes a new graph.
 int evgw_graph_run(qk_ctx* ctx, const qk_gw_params* prm, const Dims& d, const EvBufs& b) {
   std::vector<long long> key = {(long long)d.N, d.nC, d.nO, d.nR, prm->precision, prm->linearize,
                                 prm->doSRG, prm->max_diis, prm->maxSCF,
                                 (long long)(prm->thresh * 1e15), (long long)(prm->eta * 1e15),
                                 (long long)b.ERI, (long long)b.K, (long long)b.slab,
                                 (long long)b.eHF, (long long)b.eGW, (long long)b.dstate,
-                                (long long)b.L, (long long)b.naux, prm->TDA_W};
+                                (long long)b.L, (long long)b.naux, prm->TDA_W,
+                                (long long)b.SigC, (long long)b.Z, ctx->gen};
   if (!ctx->evgw_exec || ctx->evgw_key != key) {
     if (ctx->evgw_exec) {
       cudaGraphExecDestroy(ctx->evgw_exec);

@@ -40,6 +40,7 @@ int qk_ws(qk_ctx* ctx, int slot, size_t bytes, void** out) {
       cudaFree(b.p);
       b.p = nullptr;
       b.bytes = 0;
+      ctx->gen++;
     }
     size_t want = (bytes + 255) & ~(size_t)255;
     cudaError_t e = cudaMalloc(&b.p, want);
@@ -48,6 +49,7 @@ int qk_ws(qk_ctx* ctx, int slot, size_t bytes, void** out) {
       return qk_cuda_fail(ctx, e, "cudaMalloc(workspace)", __FILE__, __LINE__);
     }
     b.bytes = want;
+    ctx->gen++;
   }
   *out = b.p;
   return QK_OK;

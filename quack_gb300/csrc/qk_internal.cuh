@@ -74,6 +74,7 @@ struct qk_ctx {
   int tune[TUNE_NUM][TUNE_BUCKETS] = {};  // 0 = not tuned (defaults apply)
   cudaGraphExec_t evgw_exec = nullptr;
   std::vector<long long> evgw_key;  // shape/pointer key of the cached evGW graph
+  long long gen = 0;  // raised when a workspace block is replaced or a launch parameter changes
 };
 
 // Factorised-integral drivers on one context (qk_api.cu), reused by the batched driver.
