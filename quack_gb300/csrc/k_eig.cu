@@ -2224,5 +2224,5 @@ extern "C" int qk_dsyev_dev(qk_ctx* ctx, int n, double* d_A, int lda, double* d_
   QK_TRY(qk_status_reset(ctx));
   QK_TRY(qk_eig_sym(ctx, n, d_A, lda, d_w, d_Zt, want_vectors, 1,
                     ctx->dsyev_df == 0 ? TRI_FP64 : ctx->dsyev_df == 1 ? TRI_DF : TRI_FX));
-  return qk_status_check(ctx, QKD_BARRIER_TIMEOUT | QKD_BAD_INDEX);
+  return qk_status_check(ctx, QK_FATAL);
 }

@@ -889,14 +889,12 @@ int begin(qk_ctx* ctx) {
   return qk_status_reset(ctx);
 }
 
-constexpr int FATAL = QKD_BARRIER_TIMEOUT | QKD_BAD_INDEX | QKD_MBAR_TIMEOUT;
-
 int end(qk_ctx* ctx, int st) {
   if (st != QK_OK && st != QK_ERR_NO_CONV) {
     cudaStreamSynchronize(ctx->stream);
     return st;
   }
-  int s2 = qk_status_check(ctx, FATAL);
+  int s2 = qk_status_check(ctx, QK_FATAL);
   return s2 != QK_OK ? s2 : st;
 }
 

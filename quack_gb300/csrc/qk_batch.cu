@@ -107,7 +107,7 @@ extern "C" int qk_gw_batch_L_dev(qk_ctx* ctx, const qk_gw_params* prm, int metho
                            &ns, &conv);
         }
         if (st == QK_OK || st == QK_ERR_NO_CONV) {
-          const int s2 = qk_status_check(w, QKD_BARRIER_TIMEOUT | QKD_BAD_INDEX | QKD_MBAR_TIMEOUT);
+          const int s2 = qk_status_check(w, QK_FATAL);
           if (s2 != QK_OK) st = s2;
         }
       }

@@ -126,6 +126,8 @@ int qk_order_after_default(qk_ctx* ctx);
 // reset and read back the device status word
 int qk_status_reset(qk_ctx* ctx);
 int qk_status_check(qk_ctx* ctx, int fatal_mask);
+// device status bits after which a call's results are not to be used
+constexpr int QK_FATAL = QKD_BARRIER_TIMEOUT | QKD_BAD_INDEX | QKD_MBAR_TIMEOUT;
 
 // stage timing
 void qk_tic(qk_ctx* ctx, int stage);
