@@ -412,8 +412,9 @@ int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOrb, int nC, 
  * of them keeps eGWlin, :78-81) and "spin_limit" (polls of every bounded grid-barrier wait before
  * it gives up and reports QKD_BARRIER_TIMEOUT, QK_ERR_DEVICE from the call; 0 = the built-in
  * limit of about a second) and "fail_alloc" (n > 0: the n-th next workspace allocation that
- * would call cudaMalloc fails instead, with QK_ERR_NOMEM; 0 disarms) -- hooks for the
- * failure-path tests -- and "guess_gate" (learned-guess start rule: 0 where the model agrees with
+ * would call cudaMalloc fails instead, with QK_ERR_NOMEM; 0 disarms) and "tc_panel" (n > 0: at most
+ * about n KiB of digit planes per operand of the tensor-core FP64 products, larger operands in
+ * panels; 0 = 2 GiB) -- hooks for the failure-path tests -- and "guess_gate" (learned-guess start rule: 0 where the model agrees with
  * the Halley step from eGWlin, 1 the model's prediction everywhere, 2 the Halley step
  * everywhere; results are the reference start's in every case) and "dsyev_df" (1: qk_dsyev_dev
  * tridiagonalises in double-float arithmetic on the FP32 pipe, as the mixed tier's Casida solve

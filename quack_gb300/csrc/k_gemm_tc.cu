@@ -656,7 +656,7 @@ size_t plane_bytes(const Operand& o, int kblks) {
 }
 
 // workspace bound per operand: larger operands are taken in row panels
-constexpr size_t PANEL_BYTES = (size_t)1 << 31;
+constexpr size_t TC_PANEL_BYTES = (size_t)1 << 31;
 
 int tc_panel(qk_ctx* ctx, TcGemm g) {
   auto finish = [&](Operand& o, int rb) {
@@ -764,6 +764,7 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
     return qk_dgemm_lower(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
                           strideC, batch);
   // (k below 2^20 keeps the integer sums within 95 bits)
+  if (kscale && (k <= 0 || k > (1 << 20))) return qk_fail(ctx, QK_ERR_ARG, "scaled GEMM: k=%d", k);
   if (k <= 0 || k > (1 << 20) || !(always || lower || qk_gemm_tc_pays(ctx, m, n, k, batch)))
     return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
                     strideC, batch);
@@ -774,24 +775,26 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
   g.beta = beta;
   g.ldc = ldc;
   g.sC = strideC;
-  g.lower = lower ? 1 : 0;
   const size_t row_bytes = (size_t)((k + KB - 1) / KB) * 64 * NS;
   // batch entries per launch: the planes of one operand within the bound (and grid.y of the split-K
-  // reduction); then row panels where a single entry exceeds it
+  // reduction); then row panels where a single entry exceeds it.  The lower form takes square panels:
+  // those on the diagonal in that form, those below it whole
+  const size_t bound = ctx->tc_panel_kb > 0 ? (size_t)ctx->tc_panel_kb << 10 : TC_PANEL_BYTES;
   const size_t entry = row_bytes * (size_t)(m > n ? m : n);
-  long long b_step = (long long)(PANEL_BYTES / entry);
+  long long b_step = (long long)(bound / entry);
   b_step = b_step < 1 ? 1 : (b_step > 65535 ? 65535 : b_step);
   if (b_step > batch) b_step = batch;
   auto panel = [&](int rows, int rb) {
-    long long p = (long long)(PANEL_BYTES / row_bytes) / rb * rb;
+    long long p = (long long)(bound / row_bytes) / rb * rb;
     if (p < rb) p = rb;
     return p < rows ? (int)p : rows;
   };
-  const int pm = b_step > 1 ? m : panel(m, TM), pn = b_step > 1 ? n : panel(n, TN);
-  if (lower && (pm < m || pn < n)) return qk_fail(ctx, QK_ERR_ARG, "tensor-core GEMM: lower form too large");
+  int pm = b_step > 1 ? m : panel(m, TM), pn = b_step > 1 ? n : panel(n, TN);
+  if (lower && (pm < m || pn < n)) pm = pn = panel(m > n ? m : n, TM);
   for (int b0 = 0; b0 < batch; b0 += (int)b_step)
     for (int j0 = 0; j0 < n; j0 += pn)
-      for (int i0 = 0; i0 < m; i0 += pm) {
+      for (int i0 = lower ? j0 : 0; i0 < m; i0 += pm) {
+        g.lower = lower && i0 == j0 ? 1 : 0;
         g.batch = batch - b0 < b_step ? batch - b0 : (int)b_step;
         g.M = m - i0 < pm ? m - i0 : pm;
         g.N = n - j0 < pn ? n - j0 : pn;

@@ -103,6 +103,11 @@ int qk_tune_set(qk_ctx* ctx, const char* name, long long size, int value) {
     ctx->fail_alloc_in = value;
     return QK_OK;
   }
+  if (!strcmp(name, "tc_panel")) {
+    if (value < 0) return QK_ERR_ARG;
+    ctx->tc_panel_kb = value;
+    return QK_OK;
+  }
   if (!strcmp(name, "dsyev_df")) {
     if (value < 0 || value > 2) return QK_ERR_ARG;
     ctx->dsyev_df = value;

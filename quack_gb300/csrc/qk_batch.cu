@@ -63,6 +63,7 @@ extern "C" int qk_gw_batch_L_dev(qk_ctx* ctx, const qk_gw_params* prm, int metho
     // model is only read: its inference writes the worker's own workspace)
     std::memcpy(w->tune, ctx->tune, sizeof(ctx->tune));
     w->newton_maxit = ctx->newton_maxit;
+    w->tc_panel_kb = ctx->tc_panel_kb;
     w->mlp = ctx->mlp;
     QK_TRY(qk_order_after_default(w));
   }
