@@ -142,9 +142,13 @@ __device__ __forceinline__ void tile_sums(Tile& T, int np, const Range& g,
                                           double* __restrict__ part, size_t stride) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double c0 = eta * eta, c1 = KIND == KIND_SRG ? -2.0 * flow : -2.0 * c0;
-  // a flow that is not positive gives the high word of an infinity or a NaN: always the exp
+  // a flow that is not positive gives the high word of an infinity or a NaN: always the exp, but for
+  // |eps| from 2^98 on, where only the padding lanes' 1e30 lies (their zero amplitude times 1 - exp of
+  // a large positive number, with a negative flow, would be a NaN)
   const unsigned hthr =
-      KIND == KIND_SRG ? (unsigned)__double2hiint(sqrt(19.0 / flow)) & 0x7fffffffu : 0u;
+      KIND == KIND_SRG
+          ? min((unsigned)__double2hiint(sqrt(19.0 / flow)) & 0x7fffffffu, (1023u + 98u) << 20)
+          : 0u;
   double s[PT], d[PT];
 #pragma unroll
   for (int j = 0; j < PT; ++j) s[j] = d[j] = 0.0;
