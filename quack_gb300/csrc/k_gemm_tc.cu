@@ -20,8 +20,11 @@
 // below K 2^-60 of max_k |a_ik| max_k |b_kj|, against K 2^-53 of sum_k |a b| for the DFMA chain:
 // over the framework's contractions the result is closer to the exact product than DFMA's.
 // (An operand whose k scales differ wildly, so that sum |a b| is far below max |a| max |b|, would
-// lose that advantage: qk_dgemm_dev, which takes any matrix, stays on DFMA.)  The integers make
-// the result independent of the order of summation.
+// lose that advantage: qk_dgemm_dev, which takes any matrix, stays on DFMA.)  Where k runs over the
+// caller's basis functions, whose norms are the caller's choice (qk_gemm_tc_basis: the AO to MO
+// transformations), op(B)'s scale per k moves to op(A) as a power of two before both are sliced: the
+// result then has the same bits whatever powers of two the functions are scaled by, as with DFMA.
+// The integers make the result independent of the order of summation.
 //
 // Non-finite operands: a row (column) with a NaN gives NaN; an element whose row or column holds
 // an infinity is summed again in FP64 from the operands, so that infinities come out as they do
@@ -72,6 +75,8 @@ struct Operand {           // op(A) as rows x K, or op(B)^T as rows x K
   int row_blocks, batch;   // batch: plane sets (1: shared by all batch entries)
   const double* kscale;    // optional factors of the k index: X(r, k) kscale[k + sk b]
   long long sk;
+  const int* kexp;         // optional exponents of the k index (one operand's negated): X(r, k) 2^kexp[k]
+  int kneg;
   uint8_t* P;              // digit planes: [batch][row block][k block][digit][rb rows][64 B]
   unsigned* info;          // per row: high word of max |x| (exponent; Inf and NaN codes)
   unsigned* part;          // partial maxima [batch][k slab][row] (slabs > 0)
@@ -87,7 +92,14 @@ struct TcGemm {
 };
 
 // ---- operand preparation -----------------------------------------------------------------------
+// x 2^e (|e| <= KEXP_MAX), on the integer pipe where x and the result are normal numbers
+__device__ __forceinline__ double mul_pow2(double x, int e) {
+  const int hi = __double2hiint(x), lo = __double2loint(x), ex = (hi >> 20) & 0x7FF;
+  if (ex != 0 && ex != 0x7FF && (unsigned)(ex + e - 1) < 2046u) return __hiloint2double(hi + (e << 20), lo);
+  return ((hi & 0x7FFFFFFF) | lo) ? x * __hiloint2double((e + 1023) << 20, 0) : x;
+}
 __device__ __forceinline__ double at_k(const Operand& o, const double* ks, double x, int k) {
+  if (o.kexp) return mul_pow2(x, o.kneg ? -__ldg(o.kexp + k) : __ldg(o.kexp + k));
   return ks ? x * ks[k] : x;
 }
 __device__ __forceinline__ unsigned abs_hi(double x) {
@@ -96,6 +108,18 @@ __device__ __forceinline__ unsigned abs_hi(double x) {
 }
 
 constexpr int SELF_K = 128;
+constexpr int KEXP_MAX = 400;
+
+// kexp[k] = exponent of the largest |op(B)(k, j)| (0 where that is zero or not finite), a warp per k
+__global__ void __launch_bounds__(256) k_tc_kexp(Operand b, int K, int* __restrict__ kexp) {
+  const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= K) return;
+  unsigned m = 0;
+  for (int r = lane; r < b.rows; r += 32) m = max(m, abs_hi(b.trans ? b.X[k + b.ld * r] : b.X[r + b.ld * k]));
+  m = __reduce_max_sync(0xffffffffu, m);
+  const int e = (int)(m >> 20) - 1023;
+  if (lane == 0) kexp[k] = m == 0u || m >= HI_INF ? 0 : max(-KEXP_MAX, min(KEXP_MAX, e));
+}
 
 // part[slab][r] = max over the slab's k of the high word of |X(r, k)|; 256 threads.  trans = 0: 32
 // rows x 256 k per block, lanes along the rows; trans = 1: 8 rows x 1024 k, a warp along k.
@@ -160,7 +184,8 @@ __device__ __forceinline__ unsigned long long digits_of(double x, int exmax) {
 // contiguous bytes).  Memory-bound by design: 8 bytes read, 16 written per element.
 // SELF (K <= SELF_K): a block takes all k of its rows and finds their maxima on the way (with a block
 // per 32 k and a scan of the rows in each, rows beyond L2's reach were read once more per block: the
-// AO to MO transformation of 96 functions, 6.15 -> 5.56 ms).
+// AO to MO transformation of 96 functions, 6.15 -> 5.56 ms; 4.73 since a lane's eight loads along k are
+// issued before any of them is scaled).
 // Otherwise a block takes 32 k and the maxima come from k_tc_rowmax.
 template <bool SELF>
 __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, int kblks,
@@ -193,7 +218,11 @@ __global__ void __launch_bounds__(128) k_tc_slice(Operand a, Operand b, int K, i
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = r0 + ty + 4 * i;
-        v[i] = (r < o.rows && k < K) ? at_k(o, sc, X[k + o.ld * r], k) : 0.0;
+        v[i] = (r < o.rows && k < K) ? X[k + o.ld * r] : 0.0;
+      }
+      if ((sc || o.kexp) && k < K) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = at_k(o, sc, v[i], k);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -357,7 +386,7 @@ __device__ __noinline__ double plain_dot(const TcGemm& g, const Unit& t, int row
   const int k1 = min(g.K, t.kb1 * KB);
   double s = 0.0;
   for (int k = t.kb0 * KB; k < k1; ++k)
-    s = fma(g.a.trans ? X[k + g.a.ld * row] : X[row + g.a.ld * k],
+    s = fma(at_k(g.a, nullptr, g.a.trans ? X[k + g.a.ld * row] : X[row + g.a.ld * k], k),
             at_k(g.b, ks, g.b.trans ? Y[k + g.b.ld * col] : Y[col + g.b.ld * k], k), s);
   return s;
 }
@@ -754,10 +783,17 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
                        ldc, strideC, batch, false, always);
 }
 
+int qk_gemm_tc_basis(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
+                     long long lda, const double* B, long long ldb, double beta, double* C,
+                     long long ldc) {
+  return qk_gemm_tc_ex(ctx, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, nullptr, 0, beta, C, ldc, 0, 1,
+                       false, false, true);
+}
+
 int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                   long long lda, long long strideA, const double* B, long long ldb, long long strideB,
                   const double* kscale, long long sK, double beta, double* C, long long ldc,
-                  long long strideC, int batch, bool lower, bool always) {
+                  long long strideC, int batch, bool lower, bool always, bool kequil) {
   if (m <= 0 || n <= 0 || batch <= 0) return QK_OK;
   if (kscale && !always) return qk_fail(ctx, QK_ERR_ARG, "scaled GEMM: tensor-core path only");
   if (!always && lower && !qk_gemm_tc_pays(ctx, m, n / 2 + 1, k, batch))
@@ -775,6 +811,18 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
   g.beta = beta;
   g.ldc = ldc;
   g.sC = strideC;
+  if (kequil) {
+    int* kexp = nullptr;
+    QK_TRY(qk_wst(ctx, W_TCK, (size_t)k, &kexp));
+    g.b.X = B;
+    g.b.ld = ldb;
+    g.b.rows = n;
+    g.b.trans = !TB;
+    k_tc_kexp<<<(k + 7) / 8, 256, 0, ctx->stream>>>(g.b, k, kexp);
+    QK_LAUNCHED();
+    g.a.kexp = g.b.kexp = kexp;
+    g.b.kneg = 1;
+  }
   const size_t row_bytes = (size_t)((k + KB - 1) / KB) * 64 * NS;
   // batch entries per launch: the planes of one operand within the bound (and grid.y of the split-K
   // reduction); then row panels where a single entry exceeds it.  The lower form takes square panels:

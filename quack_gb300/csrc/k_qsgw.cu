@@ -286,21 +286,16 @@ int qk_qs_mo_slab(qk_ctx* ctx, int nBas, int N, int nC, int nO, int nR, const do
   const long long N1 = N, B = nBas;
   const double* cocc = c + B * nC;
   const double* cvir = c + B * nO;
-  auto gemm = [&](char ta, char tb, int m, int n, int k, double alpha, const double* A, long long lda,
-                  long long sA, const double* Bm, long long ldb, long long sB, double beta, double* C,
-                  long long ldc, long long sC, int batch) {
-    return df ? qk_gemm_df(ctx, ta, tb, m, n, k, alpha, A, lda, sA, Bm, ldb, sB, beta, C, ldc, sC, batch)
-              : qk_gemm_tc(ctx, ta, tb, m, n, k, alpha, A, lda, sA, Bm, ldb, sB, beta, C, ldc, sC, batch);
+  // B^3 or fewer rows of src^T times n columns of coefficients
+  auto gemm = [&](long long m, int n, const double* src, const double* Bm, double* dst) {
+    return df ? qk_gemm_df(ctx, 'T', 'N', (int)m, n, nBas, 1.0, src, B, 0, Bm, B, 0, 0.0, dst, m, 0, 1)
+              : qk_gemm_tc_basis(ctx, 'T', 'N', (int)m, n, nBas, 1.0, src, B, Bm, B, 0.0, dst, m);
   };
   // <mu la|nu si> -> (la,nu,si,j) -> (nu,si,j,p) -> (si,j,p,b) -> (j,p,b,q); c is nBas x nOrb
-  QK_TRY(gemm('T', 'N', (int)(B * B * B), no, nBas, 1.0, ERI, B, 0, cocc, B, 0, 0.0, W1,
-              B * B * B, 0, 1));
-  QK_TRY(gemm('T', 'N', (int)(B * B * no), N, nBas, 1.0, W1, B, 0, c, B, 0, 0.0, W2,
-              B * B * no, 0, 1));
-  QK_TRY(gemm('T', 'N', (int)(B * no * N1), nv, nBas, 1.0, W2, B, 0, cvir, B, 0, 0.0, W1,
-              B * no * N1, 0, 1));
-  QK_TRY(gemm('T', 'N', (int)((long long)no * N1 * nv), N, nBas, 1.0, W1, B, 0, c, B, 0, 0.0,
-              W2, (long long)no * N1 * nv, 0, 1));
+  QK_TRY(gemm(B * B * B, no, ERI, cocc, W1));
+  QK_TRY(gemm(B * B * no, N, W1, c, W2));
+  QK_TRY(gemm(B * no * N1, nv, W2, cvir, W1));
+  QK_TRY(gemm(no * N1 * nv, N, W1, c, W2));
   const long long nS = (long long)no * nv;
   k_qs_slab<<<grid_1d(ctx, N1 * N1 * nS), 256, 0, ctx->stream>>>(N, no, nv, W2, slab);
   QK_LAUNCHED();

@@ -1169,8 +1169,8 @@ int aotomo_dev(qk_ctx* ctx, int nBas, int nOrb, const double* dc, double* X, dou
       QK_TRY(qk_gemm_df(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, 0, dc, nBas, 0, 0.0,
                         dst, R[s], 0, 1));
     else
-      QK_TRY(qk_gemm_tc(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, 0, dc, nBas, 0, 0.0,
-                      dst, R[s], 0, 1));
+      QK_TRY(qk_gemm_tc_basis(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, dc, nBas, 0.0,
+                              dst, R[s]));
     double* t = src;
     src = dst;
     dst = t;
@@ -1251,7 +1251,7 @@ int qsgw_dev(qk_ctx* ctx, const qk_gw_params* prm, int nBas, const Dims& d, cons
     QK_CK(cudaMemcpyAsync(out.P, in.PHF, B2 * 8, cudaMemcpyDeviceToDevice, ctx->stream));
   auto gemm = [&](char ta, char tb, int m, int n, int k, double alpha, const double* A, int lda,
                   const double* Bm, int ldb, double beta, double* C, int ldc) {
-    return qk_gemm_tc(ctx, ta, tb, m, n, k, alpha, A, lda, 0, Bm, ldb, 0, beta, C, ldc, 0, 1);
+    return qk_gemm_tc_basis(ctx, ta, tb, m, n, k, alpha, A, lda, Bm, ldb, beta, C, ldc);
   };
   int nSCF = -1, n_diis = 0;
   double Conv = 1.0, hs[32] = {0.0};

@@ -28,7 +28,7 @@ enum {
   W_ERI = 0, W_E, W_M, W_V, W_ZT, W_EIGWORK, W_TRI, W_SLAB, W_RHO, W_XPY, W_XMY, W_VEC, W_PART,
   W_MISC, W_HOST_A, W_HOST_B, W_SPLIT_A, W_SPLIT_B, W_M2, W_SPLITK, W_QPLIST, W_VEC2, W_KMAT, W_BATCHIO, W_MLPIO, W_FEAT, W_GUESS, W_TUNE, W_TMAT, W_TMAT2, W_RHO32, W_OMF, W_TFAC, W_STEBZ,
   W_QUAD, W_QLT, W_QPV, W_QL, W_QX, W_QQ, W_QD, W_BSE, W_BSEU, W_BSER, W_BSEK, W_ERIPACK,
-  W_QSR1, W_QSR2, W_QSJK, W_QSMAT, W_QSDIIS, W_QSIN, W_QPQUEUE, W_ACF, W_TCA, W_TCB, W_TCI, W_NUMBUF
+  W_QSR1, W_QSR2, W_QSJK, W_QSMAT, W_QSDIIS, W_QSIN, W_QPQUEUE, W_ACF, W_TCA, W_TCB, W_TCI, W_TCK, W_NUMBUF
 };
 
 struct qk_tri_service;  // grouped tridiagonalisation for the batch workers (k_eig.cu)
@@ -160,7 +160,11 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
 int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                   long long lda, long long strideA, const double* B, long long ldb, long long strideB,
                   const double* kscale, long long sK, double beta, double* C, long long ldc,
-                  long long strideC, int batch, bool lower, bool always);
+                  long long strideC, int batch, bool lower, bool always, bool kequil = false);
+// k runs over basis functions and B holds their coefficients: independent of the functions' scales.
+int qk_gemm_tc_basis(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
+                     long long lda, const double* B, long long ldb, double beta, double* C,
+                     long long ldc);
 bool qk_gemm_tc_pays(const qk_ctx* ctx, int m, int n, int k, int batch);
 // The same contract with FP32 products and FP32 partial sums (split-K slices added in FP64);
 // the _lower form computes only the tiles touching the lower triangle of C and can scale the
