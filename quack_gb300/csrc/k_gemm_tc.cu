@@ -687,6 +687,7 @@ size_t plane_bytes(const Operand& o, int kblks) {
 // workspace bound per operand: larger operands are taken in row panels
 constexpr size_t TC_PANEL_BYTES = (size_t)1 << 31;
 
+// (QK_ERR_NOMEM before anything has been launched)
 int tc_panel(qk_ctx* ctx, TcGemm g) {
   auto finish = [&](Operand& o, int rb) {
     o.rb = rb;
@@ -710,18 +711,6 @@ int tc_panel(qk_ctx* ctx, TcGemm g) {
   g.b.info = g.a.info + na;
   g.a.part = g.b.info + nb;
   g.b.part = g.a.part + na * g.a.slabs;
-  auto strips = [](const Operand& o) { return (o.rows + (o.trans ? 7 : 31)) / (o.trans ? 8 : 32); };
-  if (g.K > SELF_K) {
-    const int ab = strips(g.a) * g.a.slabs * g.a.batch, bb = strips(g.b) * g.b.slabs * g.b.batch;
-    k_tc_rowmax<<<ab + bb, 256, 0, ctx->stream>>>(g.a, g.b, g.K, ab);
-    QK_LAUNCHED();
-  }
-  const int per = g.K <= SELF_K ? 1 : g.kblks;             // blocks of k per strip of 32 rows
-  const int sa = g.a.row_blocks * (TM / 32) * per * g.a.batch;
-  const int sb = g.b.row_blocks * (TN / 32) * per * g.b.batch;
-  if (g.K <= SELF_K) k_tc_slice<true><<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
-  else k_tc_slice<false><<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
-  QK_LAUNCHED();
   // few tiles and a long k: split k at chunk boundaries; the rounds of the persistent grid times a
   // slice's chunks (plus half a chunk for the epilogue) decide
   const int nch = (g.kblks + CHUNK - 1) / CHUNK;
@@ -754,6 +743,18 @@ int tc_panel(qk_ctx* ctx, TcGemm g) {
     g.ldc = g.M;
     g.sC = (long long)g.M * g.N;
   }
+  auto strips = [](const Operand& o) { return (o.rows + (o.trans ? 7 : 31)) / (o.trans ? 8 : 32); };
+  if (g.K > SELF_K) {
+    const int ab = strips(g.a) * g.a.slabs * g.a.batch, bb = strips(g.b) * g.b.slabs * g.b.batch;
+    k_tc_rowmax<<<ab + bb, 256, 0, ctx->stream>>>(g.a, g.b, g.K, ab);
+    QK_LAUNCHED();
+  }
+  const int per = g.K <= SELF_K ? 1 : g.kblks;             // blocks of k per strip of 32 rows
+  const int sa = g.a.row_blocks * (TM / 32) * per * g.a.batch;
+  const int sb = g.b.row_blocks * (TN / 32) * per * g.b.batch;
+  if (g.K <= SELF_K) k_tc_slice<true><<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
+  else k_tc_slice<false><<<sa + sb, 128, 0, ctx->stream>>>(g.a, g.b, g.K, g.kblks, sa);
+  QK_LAUNCHED();
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
@@ -813,7 +814,11 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
   g.sC = strideC;
   if (kequil) {
     int* kexp = nullptr;
-    QK_TRY(qk_wst(ctx, W_TCK, (size_t)k, &kexp));
+    const int st = qk_wst(ctx, W_TCK, (size_t)k, &kexp);
+    if (qk_oom_dropped(ctx, st))
+      return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
+                      strideC, batch);
+    QK_TRY(st);
     g.b.X = B;
     g.b.ld = ldb;
     g.b.rows = n;
@@ -859,7 +864,13 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
         g.b.rows = g.N;
         g.b.trans = !TB;
         g.C = C + b0 * strideC + i0 + (long long)j0 * ldc;
-        QK_TRY(tc_panel(ctx, g));
+        const int st = tc_panel(ctx, g);
+        // no room for the digit planes: the FMA kernel needs none
+        if (!kscale && qk_oom_dropped(ctx, st))
+          QK_TRY((g.lower ? qk_dgemm_lower : qk_dgemm)(ctx, ta, tb, g.M, g.N, k, alpha, g.a.X, lda, strideA,
+                                                       g.b.X, ldb, strideB, beta, g.C, ldc, strideC,
+                                                       g.batch));
+        else QK_TRY(st);
       }
   return QK_OK;
 }

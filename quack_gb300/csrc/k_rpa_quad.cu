@@ -489,9 +489,8 @@ void qk_gauss_legendre_host(int n, double* x, double* w) {
   if (n % 2 == 1) x[n / 2] = 0.0;
 }
 
-int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, const double* ERI,
+static int ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, const double* ERI,
                    const double* Lov, int naux, double* Ec, int* applied, bool fp64) {
-  *applied = 0;
   const int no = nO - nC, nv = N - nO - nR, nS = no * nv;
   if (nS <= 0 || (!ERI && !Lov)) return QK_OK;
   double *dd = nullptr, *small = nullptr;
@@ -693,4 +692,16 @@ int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
   QK_LAUNCHED();
   *applied = 1;
   return QK_OK;
+}
+
+int qk_rpa_ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, const double* ERI,
+                   const double* Lov, int naux, double* Ec, int* applied, bool fp64) {
+  *applied = 0;
+  const int st = ec_quad(ctx, N, nC, nO, nR, e, ERI, Lov, naux, Ec, applied, fp64);
+  // the FP64 tier's eigenvalues need no memory beyond that of the screening problem before them
+  if (fp64 && qk_oom_dropped(ctx, st)) {
+    *applied = 0;
+    return QK_OK;
+  }
+  return st;
 }

@@ -55,6 +55,13 @@ int qk_ws(qk_ctx* ctx, int slot, size_t bytes, void** out) {
   return QK_OK;
 }
 
+bool qk_oom_dropped(qk_ctx* ctx, int st) {
+  if (st != QK_ERR_NOMEM) return false;
+  (void)cudaGetLastError();  // (not sticky)
+  ctx->err.clear();
+  return true;
+}
+
 int qk_status_reset(qk_ctx* ctx) {
   QK_CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
   return QK_OK;

@@ -126,6 +126,9 @@ inline int qk_wst(qk_ctx* ctx, int slot, size_t count, T** out) {
 int qk_order_after_default(qk_ctx* ctx);
 // reset and read back the device status word
 int qk_status_reset(qk_ctx* ctx);
+// whether st says that the device's memory is exhausted; then the error is taken back, for callers that
+// go on in a way that needs less of it
+bool qk_oom_dropped(qk_ctx* ctx, int st);
 int qk_status_check(qk_ctx* ctx, int fatal_mask);
 // device status bits after which a call's results are not to be used
 constexpr int QK_FATAL = QKD_BARRIER_TIMEOUT | QKD_BAD_INDEX | QKD_MBAR_TIMEOUT;
