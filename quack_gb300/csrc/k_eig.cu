@@ -1391,15 +1391,25 @@ void launch_stebz_df(qk_ctx* ctx, int n, const float2* dd, const float2* ee, con
                                                                                   cnt, G, w);
 }
 
+}  // namespace
+
+// Lanes per eigenvalue: up to six warps per SM, in blocks of one so that they spread evenly (an SM has
+// one FP64 unit, 16 cycles a warp instruction): fewer lanes take more sweeps, more lanes queue for the
+// unit.  Best of 4, 8, 16, 32 at n = 100..3600: 32 up to 600, 16 at 1131 and 1575, 8 at 2800 and 3600.
+// A tuned value counts quarters of that.
+int qk_stebz_lanes(const qk_ctx* ctx, int n) {
+  const long long slots = 6LL * 32 * ctx->num_sms;
+  const int dflt = slots >= 32LL * n ? 32 : slots >= 16LL * n ? 16 : slots >= 8LL * n ? 8 : 4;
+  const int tk = qk_tune_get(ctx, TUNE_STEBZ_K, n, 4);
+  const long long k = (long long)dflt * tk / 4;
+  return k >= 32 ? 32 : k >= 16 ? 16 : k >= 8 ? 8 : 4;
+}
+
+namespace {
+
 void launch_stebz64(qk_ctx* ctx, int n, const double* d, const double* e2, const double* prep,
                     const int* cnt, int G, double* w) {
-  // up to six warps per SM, in blocks of one so that they spread evenly (an SM has one FP64 unit,
-  // 16 cycles a warp instruction): fewer lanes take more sweeps, more lanes queue for the unit.
-  // Best of 4, 8, 16, 32 at n = 100..3600: 32 up to 600, 16 at 1131 and 1575, 8 at 2800 and 3600.
-  const long long slots = 6LL * 32 * ctx->num_sms;
-  int K = slots >= 32LL * n ? 32 : slots >= 16LL * n ? 16 : slots >= 8LL * n ? 8 : 4;
-  const int tk = qk_tune_get(ctx, TUNE_STEBZ_K, n, 0);  // tuned width, if any (below 4 counts as 4)
-  if (tk) K = tk >= 32 ? 32 : tk >= 16 ? 16 : tk >= 8 ? 8 : 4;
+  const int K = qk_stebz_lanes(ctx, n);
   const int blocks = (int)((K * (long long)n + 31) / 32);  // one warp each
   switch (K) {
     case 32: k_stebz64<32><<<blocks, 32, 0, ctx->stream>>>(n, d, e2, prep, cnt, G, w); break;

@@ -9,10 +9,12 @@
 //                 (size = n)
 //   dgemm_path    FP64 GEMM on DFMA (1) or on the DMMA tensor path (2); qk_dgemm_dev also
 //                 takes 3, exact digit products on tcgen05                      (size = m*n)
-//   stebz_k       lanes per eigenvalue of the FP64 bisection {4,8,16,32}         (size = n)
+//   stebz_k       lanes per eigenvalue of the FP64 bisection, quarters of the default's {2,4,8}: half,
+//                 as many, twice as many (4 to 32 lanes)                       (size = n)
 // qk_autotune times every candidate on buffers of the caller's problem sizes (CUDA events on the
 // context stream, best of two runs) and records the fastest; qk_tune_save / qk_tune_load keep
-// the table as JSON so that a later process starts tuned.
+// the table as JSON so that a later process starts tuned.  Version 1 of the file held stebz_k as
+// lanes of an earlier kernel: those entries are left out.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -133,6 +135,7 @@ int qk_tune_query(const qk_ctx* ctx, const char* name, long long size) {
   if (!ctx || !name) return -1;
   if (!strcmp(name, "newton_maxit")) return ctx->newton_maxit;
   if (!strcmp(name, "dsyev_df")) return ctx->dsyev_df;
+  if (!strcmp(name, "stebz_lanes")) return qk_stebz_lanes(ctx, (int)size);
   for (int p = 0; p < TUNE_NUM; ++p)
     if (!strcmp(name, k_tune_names[p])) return ctx->tune[p][bucket_of(size)];
   return -1;
@@ -279,7 +282,7 @@ int qk_tune_save(const qk_ctx* ctx, const char* path) {
   if (!ctx || !path) return QK_ERR_ARG;
   FILE* f = fopen(path, "w");
   if (!f) return QK_ERR_ARG;
-  fprintf(f, "{\"version\": 1, \"entries\": [");
+  fprintf(f, "{\"version\": 2, \"entries\": [");
   bool first = true;
   for (int p = 0; p < TUNE_NUM; ++p)
     for (int b = 0; b < TUNE_BUCKETS; ++b)
@@ -305,6 +308,8 @@ int qk_tune_load(qk_ctx* ctx, const char* path) {
   fclose(f);
   size_t pos = 0;
   int loaded = 0;
+  const size_t pver = txt.find("\"version\"");
+  const int version = pver == std::string::npos ? 1 : atoi(txt.c_str() + txt.find(':', pver) + 1);
   while ((pos = txt.find("\"param\"", pos)) != std::string::npos) {
     const size_t q1 = txt.find('"', txt.find(':', pos) + 1);
     const size_t q2 = txt.find('"', q1 + 1);
@@ -316,7 +321,7 @@ int qk_tune_load(qk_ctx* ctx, const char* path) {
     const int v = atoi(txt.c_str() + txt.find(':', pv) + 1);
     for (int p = 0; p < TUNE_NUM; ++p)
       if (name == k_tune_names[p] && b >= 0 && b < TUNE_BUCKETS && v > 0) {
-        ctx->tune[p][b] = v;
+        if (version >= 2 || p != TUNE_STEBZ_K) ctx->tune[p][b] = v;
         ++loaded;
       }
     pos = pv + 1;

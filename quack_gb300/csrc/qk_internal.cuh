@@ -253,6 +253,7 @@ enum { TRI_FX = 0, TRI_DF = 1, TRI_FP64 = 2, TRI_FX_GRID = 3 /* requests of the 
 int qk_eig_sym(qk_ctx* ctx, int n, double* A, int lda, double* w, double* Zt, int want_vectors,
                int backtransform = 1, int tri = TRI_FX);
 int qk_tri_fx_cluster(int n);
+int qk_stebz_lanes(const qk_ctx* ctx, int n);
 struct qk_tri_fx_args {
   const double* A;
   long long lda;
