@@ -88,11 +88,12 @@ struct PcArgs {
   long long ldk;
   int nS, rmax;
   double tol_rel;
+  int chk;                   // pivots after which the decay is looked at (0: never)
   double* Lt;                // rmax x nS, column-major: Lt[t + rmax * i] = L(i, t)
   double* r;                 // residual diagonal
   int* done;                 // pivoted rows
   unsigned long long* gkey;  // pivot candidates of three consecutive steps (zeroed before launch)
-  int* rank;
+  int* rank;                 // [0] the rank (rmax: not below it), [1] pivots taken
   unsigned* bar;
   int* status;
 };
@@ -116,7 +117,7 @@ __device__ __forceinline__ unsigned long long pc_key(double v, int i) {
 __global__ void __launch_bounds__(1024, 1) k_pchol(PcArgs a) {
   extern __shared__ double lp[];  // the pivot row of L (a.rmax doubles)
   __shared__ unsigned long long s_key;
-  __shared__ double s_rp, s_inv, s_tol;
+  __shared__ double s_rp, s_inv, s_tol, s_r0;
   __shared__ int s_p, s_ok;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gw = blockIdx.x * 32 + warp, totw = gridDim.x * 32;
@@ -165,12 +166,32 @@ __global__ void __launch_bounds__(1024, 1) k_pchol(PcArgs a) {
       s_p = p;
       s_rp = rp;
       s_inv = rp > 0.0 ? qk_rsqrt(rp) : 0.0;
-      if (q == 0) s_tol = a.tol_rel * rp;  // relative to the largest diagonal
+      if (q == 0) {
+        s_tol = a.tol_rel * rp;  // relative to the largest diagonal
+        s_r0 = rp;
+      }
+      // The residual of molecular integrals falls smoothly, a little faster than the exponential of its
+      // first N pivots: log10 is -1.5 there for hydrogen chains of 48 to 96 functions and the rank at
+      // 1e-15 5.0 to 5.1 N.  Where not even twice that pace reaches the tolerance at rmax the attempt
+      // ends.  A tensor made of 3 N unrelated factors has -0.3 after N and falls off a cliff at that
+      // rank: it is left alone (fitted molecular integrals look like molecular integrals up to
+      // their cliff and take the eigenvalues where nS / 3 is below 5 N).
+      if (q == a.chk && q > 0 && rp > s_tol) {
+        const float lg = -log10f((float)(rp / s_r0));
+        if (lg > 0.75f && 2.0f * lg * (float)a.rmax < -log10f((float)a.tol_rel) * (float)q) s_p = -2;
+      }
       if (blockIdx.x == 0) a.gkey[(q + 2) % 3] = 0ull;  // read two steps ago, written next step
     }
     __syncthreads();
     const double rp = s_rp, tol = s_tol, inv = s_inv;
     const int p = s_p;
+    if (p == -2) {
+      if (blockIdx.x == 0 && tid == 0) {
+        a.rank[0] = a.rmax;
+        a.rank[1] = q;
+      }
+      return;
+    }
     if (!(rp > tol) || p < 0 || p >= a.nS) break;  // uniform: every CTA read the same key
     for (int t = tid; t < q; t += blockDim.x) lp[t] = __ldcg(a.Lt + t + (long long)a.rmax * p);
     __syncthreads();
@@ -212,7 +233,7 @@ __global__ void __launch_bounds__(1024, 1) k_pchol(PcArgs a) {
     }
     if (!barrier((q + 1) % 3)) return;
   }
-  if (blockIdx.x == 0 && tid == 0) *a.rank = q;
+  if (blockIdx.x == 0 && tid == 0) a.rank[0] = a.rank[1] = q;
 }
 
 // L (nS x r, column-major) from Lt (rmax x nS): 32 x 32 tiles through shared memory
@@ -517,8 +538,9 @@ static int ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
     nq += nq / 2;
     if (nq > 128) return QK_OK;
     // The r x r factorisations pay below the rank where the eigenvalues cost as much (nS / 3).  The
-    // rank of (ia|jb) from the tensor is only known after its Cholesky, typically a few N: with
-    // nS / 3 below 3 N the attempt would mostly be thrown away (N = 61, nS = 400: 1.3 ms of 7.3).
+    // rank of (ia|jb) from the tensor is only known after its Cholesky: 3 N or so for a tensor made of
+    // fitting factors, and with nS / 3 below that the attempt would always be thrown away (N = 61, nS =
+    // 400: 1.3 ms of 7.3).  Integrals of higher rank show themselves after N pivots (k_pchol).
     if (Lov ? naux > nS / 3 : nS < 9 * N) return QK_OK;
   }
 
@@ -542,6 +564,7 @@ static int ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
     pa.nS = nS;
     pa.rmax = rmax;
     pa.tol_rel = fp64 ? 1e-15 : 1e-12;
+    pa.chk = fp64 ? N : 0;
     pa.Lt = Lt;
     pa.r = pv;
     pa.done = (int*)(pv + nS);
@@ -577,9 +600,11 @@ static int ec_quad(qk_ctx* ctx, int N, int nC, int nO, int nR, const double* e, 
     cfg.numAttrs = 1;
     QK_CK(cudaLaunchKernelEx(&cfg, k_pchol, pa));
     ctx->launches++;
-    int rank = 0;
-    QK_CK(cudaMemcpyAsync(&rank, pa.rank, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    int hr[2] = {0, 0};
+    QK_CK(cudaMemcpyAsync(hr, pa.rank, sizeof(hr), cudaMemcpyDeviceToHost, ctx->stream));
     QK_CK(cudaStreamSynchronize(ctx->stream));
+    const int rank = hr[0];
+    ctx->quad_pivots = hr[1];
     int hst = 0;
     QK_CK(cudaMemcpy(&hst, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost));
     if (hst & QKD_BARRIER_TIMEOUT)

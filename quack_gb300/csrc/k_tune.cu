@@ -135,6 +135,7 @@ int qk_tune_query(const qk_ctx* ctx, const char* name, long long size) {
   if (!ctx || !name) return -1;
   if (!strcmp(name, "newton_maxit")) return ctx->newton_maxit;
   if (!strcmp(name, "dsyev_df")) return ctx->dsyev_df;
+  if (!strcmp(name, "quad_pivots")) return ctx->quad_pivots;
   if (!strcmp(name, "stebz_lanes")) return qk_stebz_lanes(ctx, (int)size);
   for (int p = 0; p < TUNE_NUM; ++p)
     if (!strcmp(name, k_tune_names[p])) return ctx->tune[p][bucket_of(size)];

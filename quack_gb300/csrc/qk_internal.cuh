@@ -55,6 +55,7 @@ struct qk_ctx {
   int newton_maxit = 64;   // Newton steps of the graphical QP solve (RGW_QP_graph.f90:38)
   int guess_gate = 0;      // learned-guess start rule (k_guess: 0 Halley agreement, 1, 2)
   int fail_alloc_in = 0;   // > 0: the n-th next growing workspace allocation fails (test hook)
+  int quad_pivots = 0;     // pivots of the last (ia|jb) factorisation
   int tc_panel_kb = 0;     // > 0: bound of an operand's digit planes in the tensor-core FP64 products, KiB
   int dsyev_df = 0;        // qk_dsyev_dev: 0 FP64 kernel, 1 double-float, 2 as the FP64-tier drivers
   qk_tri_service* tri_service = nullptr;  // batch worker: tridiagonalise through the group launch
