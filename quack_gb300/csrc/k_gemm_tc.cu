@@ -687,6 +687,21 @@ size_t plane_bytes(const Operand& o, int kblks) {
 // workspace bound per operand: larger operands are taken in row panels
 constexpr size_t TC_PANEL_BYTES = (size_t)1 << 31;
 
+// Few tiles and a long k: k is split at chunk boundaries into at most 16 slices.  The rounds of the
+// persistent grid times a slice's chunks (plus half a chunk for the epilogue) decide; returned in
+// chunks.
+double tc_slices(const qk_ctx* ctx, long long tiles, int nch, int& S) {
+  double best = 1e300;
+  S = 1;
+  for (int s = 1; s <= 16 && s <= nch; ++s) {
+    if (s > 1 && tiles * s > 4LL * ctx->num_sms) break;
+    const double rounds = (double)((tiles * s + ctx->num_sms - 1) / ctx->num_sms);
+    const double cost = rounds * ((nch + s - 1) / s + 0.5) + (s > 1 ? 0.5 : 0.0);
+    if (cost < best) { best = cost; S = s; }
+  }
+  return best;
+}
+
 // (QK_ERR_NOMEM before anything has been launched)
 int tc_panel(qk_ctx* ctx, TcGemm g) {
   auto finish = [&](Operand& o, int rb) {
@@ -711,20 +726,10 @@ int tc_panel(qk_ctx* ctx, TcGemm g) {
   g.b.info = g.a.info + na;
   g.a.part = g.b.info + nb;
   g.b.part = g.a.part + na * g.a.slabs;
-  // few tiles and a long k: split k at chunk boundaries; the rounds of the persistent grid times a
-  // slice's chunks (plus half a chunk for the epilogue) decide
   const int nch = (g.kblks + CHUNK - 1) / CHUNK;
   const long long tiles = (long long)g.mt * g.nt * g.batch;
   int S = 1;
-  if (!g.lower) {
-    double best = 1e300;
-    for (int s = 1; s <= 16 && s <= nch; ++s) {
-      if (s > 1 && tiles * s > 4LL * ctx->num_sms) break;
-      const double rounds = (double)((tiles * s + ctx->num_sms - 1) / ctx->num_sms);
-      const double cost = rounds * ((nch + s - 1) / s + 0.5) + (s > 1 ? 0.5 : 0.0);
-      if (cost < best) { best = cost; S = s; }
-    }
-  }
+  if (!g.lower) tc_slices(ctx, tiles, nch, S);
   const int cps = (nch + S - 1) / S;
   S = (nch + cps - 1) / cps;
   g.slices = S;
@@ -877,16 +882,18 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
 
 // Whether the tensor-core path is the faster one for this product.  Both costs are in
 // microseconds on one GB300: DFMA runs its 16 x 16 tiles at ~1.1 TFLOP/s; a 128 x 64 x 128 chunk on
-// the tensor cores takes ~7.2 us per SM, the operands' preparation moves 32 bytes an element, and its
-// launches and their latency cost ~15 us against ~5 (measured, DFMA / tensor cores: 128 x 128 x 400
-// 16 / 30 us, 400 x 128 x 128 14 / 22, 567 x 128 x 128 20 / 23, 128 x 400 x 400 45 / 33, 400 x 400 x
-// 128 46 / 24).
+// the tensor cores takes ~7.2 us per SM and a tile's k is spread over 16 SMs at most, the operands'
+// preparation moves 32 bytes an element, and its launches and their latency cost ~15 us against ~5
+// (measured, DFMA / tensor cores: 128 x 128 x 400 16 / 30 us, 400 x 128 x 128 14 / 22, 567 x 128 x 128
+// 20 / 23, 128 x 400 x 400 45 / 33, 400 x 400 x 128 46 / 24; with a call's 22 us: 48 x 48 x 15360 92 /
+// 113, 64 x 64 x 4096 58 / 60, 64 x 64 x 32768 288 / 195, 20 x 20 x 200000 460 / 951).
 bool qk_gemm_tc_pays(const qk_ctx* ctx, int m, int n, int k, int batch) {
   if (k < 16) return false;
   const double pm = (m + 15) / 16 * 16.0, pn = (n + 15) / 16 * 16.0;
   const double dfma = 5.0 + 2.0 * pm * pn * k * batch / 1.1e6;
-  const double chunks = (double)((m + TM - 1) / TM) * ((n + TN - 1) / TN) * batch * ((k + 127) / 128);
-  const double tc = 15.0 + 7.2 * (double)((long long)(chunks + ctx->num_sms - 1) / ctx->num_sms) +
-                    ((double)m + n) * k * batch * 32.0 / 4e6;
+  const long long tiles = (long long)((m + TM - 1) / TM) * ((n + TN - 1) / TN) * batch;
+  int S;
+  const double chunks = tc_slices(ctx, tiles, (k + 127) / 128, S);
+  const double tc = 15.0 + 7.2 * (chunks - 0.5) + ((double)m + n) * k * batch * 32.0 / 4e6;
   return tc < dfma;
 }
