@@ -41,15 +41,23 @@ enum {
 
 /* precision tiers */
 enum {
-  QK_PREC_FP64 = 0,        /* FP64 throughout (plain form) */
+  QK_PREC_FP64 = 0,        /* plain form: FP64, its large products and reductions on integers.  Products:
+                              exact sums of 62-bit operands (relative to the largest element of a
+                              row and a column).  Eigenproblems: the reduction rounds to 2^-62 of
+                              the matrix's norm, so an eigenvalue carries that of the norm where an
+                              FP64 reduction carries up to 2^-53 of it -- except in a block that is
+                              exactly decoupled, where FP64 would round relative to the block's own
+                              norm (valence Omega next to decoupled cores: 9e-14 Ha at -104 Ha, 1e-11
+                              at -1177).  G0W0's EcRPA at eGW: eigenvalues or, for a factor of low
+                              rank, a frequency quadrature of the same accuracy. */
   QK_PREC_BF16X3 = 1       /* mixed: the excitation-density contraction as BF16x3 split products
                               on tcgen05 (FP32 accumulation, compensated) and the eigenvector
                               back-transformation on compensated FP32 products; with eta = 0 and
                               no SRG the pole sums of Sigma/dSigma (linearised stage and Newton)
                               take the terms with |w - e +- Om| >= 0.01 Ha in FP32 and the
                               near-pole terms in FP64; G0W0's EcRPA at eGW by frequency
-                              quadrature with FP32 products (the FP64 form's keeps FP64 accuracy).  The Casida eigenvalues, the Newton update and DIIS stay
-                              FP64. */
+                              quadrature with FP32 products.  The Casida eigenvalues, the Newton
+                              update and DIIS stay FP64. */
 };
 
 /* Options of the GW line of QuAcK's input/options (QuAcK/read_options.f90:242-267). */
@@ -336,9 +344,11 @@ int qk_RGW_phBSE_dev(qk_ctx* ctx, const qk_bse_params* prm, int nOrb, int nC, in
  *   Q with compensated FP32 products, ln det by FP64 Cholesky; agrees with the eigenvalue
  *   route to ~1e-8 Ha.  A negative e_a - e_i gives NaN (as the Casida square roots do) and the
  *   QKD_NEG_AMB status.  *applied = 0 (EcRPA untouched) when it does not apply: a zero
- *   e_a - e_i, d_max/d_min > 60000, or a numerical rank of (ia|jb) above nS/3.  The mixed tier
+ *   e_a - e_i, d_max/d_min > 60000, or a numerical rank of (ia|jb) above nS/3 (the factor takes a
+ *   positive semidefinite (ia|jb) for granted here).  The mixed tier
  *   of qk_RG0W0 / qk_RG0W0_L_dev uses it for the EcRPA at the G0W0 energies; the FP64 tier has its
- *   own form there (more points, FP64 products), with the eigenvalue route's accuracy.
+ *   own form there (more points, FP64 products), with the eigenvalue route's accuracy, which declines
+ *   an (ia|jb) that the factor does not reproduce.
  * qk_gauss_legendre: the quadrature's nodes x (ascending) and weights w on [-1, 1], host only. */
 int qk_RPA_ecorr_quad_dev(qk_ctx* ctx, int nOrb, int nC, int nO, int nR, int naux,
                           const double* d_e, const double* d_ERI, const double* d_L,
@@ -398,11 +408,10 @@ int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOrb, int nC, 
  * per size bucket floor(log2(size)): "bf16x3_chunk" (k blocks per TMEM chunk of the BF16x3 GEMM,
  * size = K), "splitk_mult" (split-K target CTAs per SM of the DMMA GEMM, size = K),
  * "sigma_chunks" (how far the pole sweeps split their q range, 4 = to one CTA per SM and tile of
- * orbitals, size = nS), "sytrd_grid" (quarters of the
- * SMs in the cooperative tridiagonalisations, size = n), "dgemm_path" (1 DFMA, 2 DMMA; for
- * qk_dgemm_dev also 3, exact integer digit products on tcgen05 -- what the drivers use for FP64
- * products large enough -- whose error is relative to the largest elements of a row of op(A) and a
- * column of op(B); size = m n),
+ * orbitals, size = nS), "sytrd_grid" (quarters of the SMs in the cooperative tridiagonalisations,
+ * size = n), "dgemm_path" (1 DFMA, 2 DMMA; for qk_dgemm_dev also 3, exact integer digit products on
+ * tcgen05 -- what the drivers use for FP64 products large enough -- whose error is relative to the
+ * largest elements of a row of op(A) and a column of op(B); size = m n),
  * "stebz_k" (lanes per eigenvalue in the FP64 bisection, in quarters of the untuned number: 2 half, 4
  * as many, 8 twice as many; qk_tune_query's "stebz_lanes" gives the lanes used; size = n), "qp_persist" (mixed-tier Newton:
  * 1 persistent kernel, 2 per-step sweeps, size = nS).  qk_autotune times all candidates on

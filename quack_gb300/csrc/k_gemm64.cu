@@ -1,14 +1,16 @@
-// k_gemm64.cu -- FP64 GEMM: the FP64 tensor path (DMMA, mma.sync.m8n8k4.f64) and a DFMA path,
-// plus an FP32-product variant with FP64 operands and result (the mixed tier's eigenvector
-// back-transformation).
-//
-// Column-major C = alpha*op(A)*op(B) + beta*C, strided batch.  Used for the AO->MO quarter
-// transforms (AOtoMO/AOtoMO_ERI_RHF.f90:26-53), the FP64 excitation density
-// (GW/RGW_excitation_density.f90:48-50) and the blocked back-transformation of the
-// eigensolver.  Tile 64x64x16, 4 warps (2x2), each warp a 32x32 block of 4x4 DMMA tiles;
-// operands are staged global -> registers -> shared memory with one stage of prefetch.
-// On GB300 the FP64 rate (~1.2 TFLOP/s) is the bound for every FP64 contraction here, so the
-// kernel is shaped for issue rate (16 DMMA per 8 shared loads), not for bandwidth.
+// k_gemm64.cu -- GEMM on the FP64 and FP32 pipes, column-major C = alpha*op(A)*op(B) + beta*C, strided
+// batch:
+//   k_gemm_t16    FP64 FMA, 16 x 16 tiles: qk_dgemm, and what qk_gemm_tc (k_gemm_tc.cu) leaves to it --
+//                 the products too small for the tensor cores, and those without memory for its digit
+//                 planes.  The AO->MO quarter transforms (AOtoMO/AOtoMO_ERI_RHF.f90:26-53), the
+//                 excitation density (GW/RGW_excitation_density.f90:48-50) and the eigensolver's
+//                 back-transformation come through there.
+//   k_dgemm_dmma  the FP64 tensor path (mma.sync.m8n8k4.f64), where a tuning table asks for it:
+//                 64 x 64 x 16 tiles, 4 warps of 32 x 32, one stage of prefetch.  GB300's FP64 rate
+//                 (~1.2 TFLOP/s) bounds both, so it is shaped for issue rate (16 DMMA per 8 shared
+//                 loads), not for bandwidth.
+//   k_gemm_simt   FP32 products of FP64 operands into an FP64 result (the mixed tier)
+//   k_gemm_df     double-float products (the mixed tier of qsGW and of the AO->MO transforms)
 #include "qk_internal.cuh"
 
 namespace {

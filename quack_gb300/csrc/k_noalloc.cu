@@ -90,10 +90,6 @@ extern "C" int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOr
   double* part = nullptr;
   int st = scratch_for_current_device(&part);
   if (st != QK_OK) return st;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return QK_ERR_CUDA;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return QK_ERR_CUDA;
   // one 32-lane group of m a chunk, more above 128 chunks (the scratch array's size); every
   // partial sum that the reduction reads is written by the sweep
   const int nact = N - nR - nC;

@@ -183,8 +183,8 @@ int qk_gemm_f32p_lower(qk_ctx* ctx, char ta, char tb, int m, int n, int k, doubl
                        long long strideC, int batch, const float* kscale = nullptr,
                        long long sK = 0);
 
-// FP64 GEMM that computes only the 64x64 tiles of C touching its lower triangle (rows >= cols);
-// for symmetric rank-k updates whose consumer reads the lower triangle.
+// FP64 GEMM that computes only the tiles of C touching its lower triangle (rows >= cols); for
+// symmetric rank-k updates whose consumer reads the lower triangle.
 int qk_dgemm_lower(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
                    const double* A, long long lda, long long strideA, const double* B,
                    long long ldb, long long strideB, double beta, double* C, long long ldc,
