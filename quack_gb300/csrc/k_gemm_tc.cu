@@ -110,7 +110,7 @@ __device__ __forceinline__ unsigned abs_hi(double x) {
 constexpr int SELF_K = 128;
 constexpr int KEXP_MAX = 400;
 
-// kexp[k] = exponent of the largest |op(B)(k, j)| (0 where that is zero or not finite), a warp per k
+// kexp[k] = exponent of the largest |b(k, j)| (0 where that is zero or not finite), a warp per k
 __global__ void __launch_bounds__(256) k_tc_kexp(Operand b, int K, int* __restrict__ kexp) {
   const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (k >= K) return;
@@ -791,15 +791,16 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
 
 int qk_gemm_tc_basis(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                      long long lda, const double* B, long long ldb, double beta, double* C,
-                     long long ldc) {
+                     long long ldc, qk_basis_exp* be) {
+  qk_basis_exp own = {};
   return qk_gemm_tc_ex(ctx, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, nullptr, 0, beta, C, ldc, 0, 1,
-                       false, false, true);
+                       false, false, be ? be : &own);
 }
 
 int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                   long long lda, long long strideA, const double* B, long long ldb, long long strideB,
                   const double* kscale, long long sK, double beta, double* C, long long ldc,
-                  long long strideC, int batch, bool lower, bool always, bool kequil) {
+                  long long strideC, int batch, bool lower, bool always, qk_basis_exp* be) {
   if (m <= 0 || n <= 0 || batch <= 0) return QK_OK;
   if (kscale && !always) return qk_fail(ctx, QK_ERR_ARG, "scaled GEMM: tensor-core path only");
   if (!always && lower && !qk_gemm_tc_pays(ctx, m, n / 2 + 1, k, batch))
@@ -817,20 +818,23 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
   g.beta = beta;
   g.ldc = ldc;
   g.sC = strideC;
-  if (kequil) {
-    int* kexp = nullptr;
-    const int st = qk_wst(ctx, W_TCK, (size_t)k, &kexp);
-    if (qk_oom_dropped(ctx, st))
-      return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
-                      strideC, batch);
-    QK_TRY(st);
-    g.b.X = B;
-    g.b.ld = ldb;
-    g.b.rows = n;
-    g.b.trans = !TB;
-    k_tc_kexp<<<(k + 7) / 8, 256, 0, ctx->stream>>>(g.b, k, kexp);
-    QK_LAUNCHED();
-    g.a.kexp = g.b.kexp = kexp;
+  if (be) {
+    if (!be->e) {
+      int* kexp = nullptr;
+      const int st = qk_wst(ctx, W_TCK, (size_t)k, &kexp);
+      if (qk_oom_dropped(ctx, st))
+        return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
+                        strideC, batch);
+      QK_TRY(st);
+      g.b.X = be->c ? be->c : B;
+      g.b.ld = be->c ? be->ld : ldb;
+      g.b.rows = be->c ? be->n : n;
+      g.b.trans = be->c || !TB;
+      k_tc_kexp<<<(k + 7) / 8, 256, 0, ctx->stream>>>(g.b, k, kexp);
+      QK_LAUNCHED();
+      be->e = kexp;
+    }
+    g.a.kexp = g.b.kexp = be->e;
     g.b.kneg = 1;
   }
   const size_t row_bytes = (size_t)((k + KB - 1) / KB) * 64 * NS;

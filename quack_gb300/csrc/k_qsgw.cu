@@ -287,9 +287,10 @@ int qk_qs_mo_slab(qk_ctx* ctx, int nBas, int N, int nC, int nO, int nR, const do
   const double* cocc = c + B * nC;
   const double* cvir = c + B * nO;
   // B^3 or fewer rows of src^T times n columns of coefficients
+  qk_basis_exp be{c, B, N, nullptr};
   auto gemm = [&](long long m, int n, const double* src, const double* Bm, double* dst) {
     return df ? qk_gemm_df(ctx, 'T', 'N', (int)m, n, nBas, 1.0, src, B, 0, Bm, B, 0, 0.0, dst, m, 0, 1)
-              : qk_gemm_tc_basis(ctx, 'T', 'N', (int)m, n, nBas, 1.0, src, B, Bm, B, 0.0, dst, m);
+              : qk_gemm_tc_basis(ctx, 'T', 'N', (int)m, n, nBas, 1.0, src, B, Bm, B, 0.0, dst, m, &be);
   };
   // <mu la|nu si> -> (la,nu,si,j) -> (nu,si,j,p) -> (si,j,p,b) -> (j,p,b,q); c is nBas x nOrb
   QK_TRY(gemm(B * B * B, no, ERI, cocc, W1));

@@ -1163,6 +1163,7 @@ int aotomo_dev(qk_ctx* ctx, int nBas, int nOrb, const double* dc, double* X, dou
   // ~1e-13 of sum |a b|) -- the MO coefficients of near-linearly-dependent bases cancel too much
   // for the BF16x3 / FP32-product tiers (the reason qsGW's mixed tier uses it as well)
   const bool df = ctx->stage_precision == QK_PREC_BF16X3;
+  qk_basis_exp be{dc, nBas, nOrb, nullptr};
   for (int s = 0; s < 4; ++s) {
     if (R[s] > INT_MAX) return qk_fail(ctx, QK_ERR_ARG, "AO->MO quarter transform too large");
     if (df)
@@ -1170,7 +1171,7 @@ int aotomo_dev(qk_ctx* ctx, int nBas, int nOrb, const double* dc, double* X, dou
                         dst, R[s], 0, 1));
     else
       QK_TRY(qk_gemm_tc_basis(ctx, 'T', 'N', (int)R[s], nOrb, nBas, 1.0, src, nBas, dc, nBas, 0.0,
-                              dst, R[s]));
+                              dst, R[s], &be));
     double* t = src;
     src = dst;
     dst = t;
