@@ -393,11 +393,11 @@ def run_ours(args):
     }
     # EcRPA at the G0W0 energies (RG0W0.f90:222-225): with a closed QP gap (some e_a < e_i after
     # the Newton solve) it is NaN in both tiers without an eigenproblem, as in the reference;
-    # with an open gap the mixed tier runs the frequency quadrature, the plain tier the FP64
-    # eigenvalue route.  Which branch a tier takes depends on its chaotic Newton roots (both
-    # tiers are deterministic, so each always takes the same one), so the speed-up is also given
-    # for both tiers on the same branch, from the measured stage times: the quadrature (its own
-    # leg, on the HF energies from the ERI tensor) and the plain tier's eigenvalue route.
+    # with an open gap both run the frequency quadrature, each in its precision.  Which branch a
+    # tier takes depends on its chaotic Newton roots (both tiers are deterministic, so each always
+    # takes the same one), so the speed-up is also given for both tiers on the same branch, from the
+    # measured stage times: the mixed quadrature (its own leg, on the HF energies from the ERI
+    # tensor) and the plain tier's stage (where its gap is closed, the FP64 eigenvalues').
     gap = {"mixed": float(e_mix[nO:].min() - e_mix[:nO].max()),
            "plain_fp64": float(e_fp[nO:].min() - e_fp[:nO].max())}
     res["qp_gap_min_Ha"] = gap
@@ -408,7 +408,7 @@ def run_ours(args):
     mix_closed, fp_closed = ms_mix / K - c2m, ms_fp / Kp - c2p
     res["ecrpa_branch"] = {
         "mixed": "open gap: quadrature" if gap["mixed"] > 0 else "closed gap: NaN, no eigenproblem",
-        "plain_fp64": ("open gap: FP64 eigenvalues" if gap["plain_fp64"] > 0
+        "plain_fp64": ("open gap: FP64 quadrature" if gap["plain_fp64"] > 0
                        else "closed gap: NaN, no eigenproblem"),
         "speedup_both_open_gap": (fp_closed + t_eig) / (mix_closed + t_quad),
         "speedup_both_closed_gap": fp_closed / mix_closed,

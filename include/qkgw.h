@@ -413,7 +413,8 @@ int qk_RGW_self_energy_diag_noalloc_dev(double eta, int nBas, int nOrb, int nC, 
  * tcgen05 -- what the drivers use for FP64 products large enough -- whose error is relative to the
  * largest elements of a row of op(A) and a column of op(B); size = m n),
  * "stebz_k" (lanes per eigenvalue in the FP64 bisection, in quarters of the untuned number: 2 half, 4
- * as many, 8 twice as many; qk_tune_query's "stebz_lanes" gives the lanes used; size = n), "qp_persist" (mixed-tier Newton:
+ * as many, 8 twice as many; qk_tune_query's "stebz_lanes" gives the lanes used, "quad_pivots"
+ * the pivots of the last factorisation of (ia|jb) for EcRPA; size = n), "qp_persist" (mixed-tier Newton:
  * 1 persistent kernel, 2 per-step sweeps, size = nS).  qk_autotune times all candidates on
  * problems of the given sizes (allocates temporary buffers) and keeps the fastest; the table
  * can be saved to / loaded from a JSON file.
