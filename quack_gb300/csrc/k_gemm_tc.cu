@@ -20,10 +20,11 @@
 // below K 2^-60 of max_k |a_ik| max_k |b_kj|, against K 2^-53 of sum_k |a b| for the DFMA chain:
 // over the framework's contractions the result is closer to the exact product than DFMA's.
 // (An operand whose k scales differ wildly, so that sum |a b| is far below max |a| max |b|, would
-// lose that advantage: qk_dgemm_dev, which takes any matrix, stays on DFMA.)  Where k runs over the
-// caller's basis functions, whose norms are the caller's choice (qk_gemm_tc_basis: the AO to MO
-// transformations), op(B)'s scale per k moves to op(A) as a power of two before both are sliced: the
-// result then has the same bits whatever powers of two the functions are scaled by, as with DFMA.
+// lose that advantage: qk_dgemm_dev, which takes any matrix, and qsGW's Fock algebra stay on DFMA.)
+// Where k runs over the caller's basis functions, whose norms are the caller's choice, and op(B) holds
+// orbital coefficients (qk_gemm_tc_basis), their scale per k moves to op(A) as a power of two before
+// both are sliced: the result then has the same bits whatever powers of two the functions are scaled
+// by, as with DFMA.
 // The integers make the result independent of the order of summation.
 //
 // Non-finite operands: a row (column) with a NaN gives NaN; an element whose row or column holds
@@ -110,7 +111,7 @@ __device__ __forceinline__ unsigned abs_hi(double x) {
 constexpr int SELF_K = 128;
 constexpr int KEXP_MAX = 400;
 
-// kexp[k] = exponent of the largest |b(k, j)| (0 where that is zero or not finite), a warp per k.  A launch
+// kexp[k] = exponent of the largest |c(k, j)| (0 where that is zero or not finite), a warp per k.  A launch
 // of its own, ~3 us: once per transformation (26 functions 129 us with one per quarter, 117 with one, 120
 // without scales; 30: 164, 153, 150; 60: 839, 823, 958).
 __global__ void __launch_bounds__(256) k_tc_kexp(Operand b, int K, int* __restrict__ kexp) {
@@ -794,9 +795,8 @@ int qk_gemm_tc(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha,
 int qk_gemm_tc_basis(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                      long long lda, const double* B, long long ldb, double beta, double* C,
                      long long ldc, qk_basis_exp* be) {
-  qk_basis_exp own = {};
   return qk_gemm_tc_ex(ctx, ta, tb, m, n, k, alpha, A, lda, 0, B, ldb, 0, nullptr, 0, beta, C, ldc, 0, 1,
-                       false, false, be ? be : &own);
+                       false, false, be);
 }
 
 int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
@@ -828,10 +828,10 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
         return qk_dgemm(ctx, ta, tb, m, n, k, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc,
                         strideC, batch);
       QK_TRY(st);
-      g.b.X = be->c ? be->c : B;
-      g.b.ld = be->c ? be->ld : ldb;
-      g.b.rows = be->c ? be->n : n;
-      g.b.trans = be->c || !TB;
+      g.b.X = be->c;
+      g.b.ld = be->ld;
+      g.b.rows = be->n;
+      g.b.trans = 1;
       k_tc_kexp<<<(k + 7) / 8, 256, 0, ctx->stream>>>(g.b, k, kexp);
       QK_LAUNCHED();
       be->e = kexp;

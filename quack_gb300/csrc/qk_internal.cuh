@@ -166,9 +166,9 @@ int qk_gemm_tc_ex(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alp
                   const double* kscale, long long sK, double beta, double* C, long long ldc,
                   long long strideC, int batch, bool lower, bool always,
                   struct qk_basis_exp* be = nullptr);
-// k runs over basis functions and B holds their coefficients: independent of the functions' scales, by
-// an exponent per function from the largest elements of B's or, for several products over the same
-// functions, of c's n columns (found at the first of them that takes the tensor cores).
+// k runs over basis functions and B holds columns of their coefficients c: independent of the functions'
+// scales, by an exponent per function from the largest element of c's n columns, found at the first of
+// the products that takes the tensor cores.
 struct qk_basis_exp {
   const double* c;
   long long ld;
@@ -177,7 +177,7 @@ struct qk_basis_exp {
 };
 int qk_gemm_tc_basis(qk_ctx* ctx, char ta, char tb, int m, int n, int k, double alpha, const double* A,
                      long long lda, const double* B, long long ldb, double beta, double* C,
-                     long long ldc, qk_basis_exp* be = nullptr);
+                     long long ldc, qk_basis_exp* be);
 bool qk_gemm_tc_pays(const qk_ctx* ctx, int m, int n, int k, int batch);
 // The same contract with FP32 products and FP32 partial sums (split-K slices added in FP64);
 // the _lower form computes only the tiles touching the lower triangle of C and can scale the

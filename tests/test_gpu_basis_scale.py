@@ -72,3 +72,45 @@ def test_qsgw(ctx, width):
     for k in ("eGW", "Z"):
         assert np.array_equal(a[k], b[k])
     assert np.array_equal(a["c"], b["c"] * s[:, None])
+
+
+def test_qsgw_large():
+    """One cycle of 240 functions, where products of nBas^3 would be worth the tensor cores."""
+    import torch
+    n, nO, naux = 240, 2, 30
+    g = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *k: torch.randn(*k, generator=g, device="cuda", dtype=torch.float64)
+    B = r(n, n) * 0.02
+    S = torch.eye(n, device="cuda", dtype=torch.float64) + B @ B.T
+    w, U = torch.linalg.eigh(S)
+    X = U @ torch.diag(w.rsqrt()) @ U.T
+    T = torch.diag(torch.linspace(0.5, 4.0, n, device="cuda", dtype=torch.float64))
+    V = r(n, n) * 0.01
+    V = -(V + V.T) - torch.diag(torch.linspace(3.0, 0.1, n, device="cuda", dtype=torch.float64))
+    e, Cp = torch.linalg.eigh(X.T @ (T + V) @ X)
+    c = X @ Cp
+    P = 2.0 * c[:, :nO] @ c[:, :nO].T
+    L = r(naux, n, n) * 0.005
+    L = L + L.transpose(1, 2)
+    s = torch.from_numpy(_scales(n, np.random.default_rng(3), 20)).cuda()
+    f = lambda x: x.T.contiguous().reshape(-1)                   # Fortran order
+    Lf = L.reshape(naux, n * n)
+    E = (Lf.T @ Lf).reshape(n, n, n, n).permute(3, 1, 2, 0).contiguous()
+    ctx = api.Context(0)
+    res = []
+    try:
+        for k in (torch.ones_like(s), s):
+            kk = k[:, None] * k
+            E.mul_(k[:, None, None, None]).mul_(k[:, None, None]).mul_(k[:, None]).mul_(k)
+            ins = [e, f(c / k[:, None]), f(P / kk), f(S * kk), f(T * kk), f(V * kk), f((T + V) * kk),
+                   f(X / k[:, None]), E]
+            out = [torch.zeros(m, dtype=torch.float64, device="cuda") for m in (n, n * n, n * n, n)]
+            api.qsRGW_dev(api.GWOptions(eta=0.1, maxSCF=0), n, 0, nO, 0, *[t.data_ptr() for t in ins],
+                          *[t.data_ptr() for t in out], ctx=ctx, raise_on_fail=False)
+            res.append([out[0], out[1].reshape(n, n).T * k[:, None], out[3]])
+    finally:
+        ctx.close()
+    del E, ins, L, Lf
+    torch.cuda.empty_cache()
+    for a, b in zip(*res):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
